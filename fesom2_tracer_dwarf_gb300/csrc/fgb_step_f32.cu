@@ -111,9 +111,19 @@ int launch_stages_f32(const DMesh& m, const fgb_step_desc& d, int mask, cudaStre
   L.ns_ratio = (d.cfg[5] >= 1 && d.cfg[5] <= 4) ? d.cfg[5] : 0;
   L.ns_upd = ns(d.cfg[6], 1);
   L.vimpl_thomas = d.cfg[8] == 1;
-  // the tiled edge kernel stages rows with 16-byte asynchronous copies
+  // Edge fluxes: the tiled kernel unless cfg[0] or cfg[7] asks for a shape of
+  // the per-edge one. A block of the tiled kernel holds at most 32 edges, so a
+  // small mesh still fills the GPU, and a layer outside its triangles' window
+  // costs its own lane the element gradients around the nodes, not the whole
+  // warp. Edge stage, per-edge kernel against tiled: 48x40x30, 3 tracers, 103
+  // against 35 us; closed 513^2x64, 2 tracers, 930 / 477 us; pi refined to
+  // 188,661 nodes, 47 layers, 4 tracers, 670 / 438 us; 250x230x47, 2 tracers,
+  // 149 / 91 us; 256^2x64, 4 tracers, 162 / 125 us; no size was slower.
+  // The tiled kernel stages rows with 16-byte asynchronous copies; fields on
+  // other addresses take the per-edge kernel.
   auto al16 = [](const void* p) { return p == nullptr || reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-  L.hflux_tile = d.cfg[9] == 1 && al16(d.T) && al16(d.TA) && al16(d.workspace) && (d.strideT * 4) % 16 == 0 &&
+  const bool tile = d.cfg[9] == 1 || (d.cfg[0] == 0 && d.cfg[7] == 0);
+  L.hflux_tile = tile && al16(d.T) && al16(d.TA) && al16(d.workspace) && (d.strideT * 4) % 16 == 0 &&
                  (!d.TA || (d.strideTA * 4) % 16 == 0);
   L.hor = d.hor;
   L.ver = d.ver;

@@ -253,7 +253,8 @@ typedef struct {
   long long workspace_bytes;
   int tracer_vec; /* tracers per group of the FP32 layout: 0 or 1, 2, 4 */
   /* Launch configuration; 0 picks the default. Results do not depend on it.
-   * cfg[0]     warps (edges) per block of the edge-flux kernel: 2, 4, 8 (default 8)
+   * cfg[0]     warps (edges) per block of the edge-flux kernel: 2, 4, 8 (default 8;
+   *            FP32 form: of its per-edge kernel, see cfg[9])
    * cfg[1..3]  warps (node columns) per block of the LO, ratio and update
    *            kernels: 1, 2, 4 (default 4)
    * cfg[4..6]  FP64 form: tracers per chunk of the same three kernels: 1, 2,
@@ -263,12 +264,14 @@ typedef struct {
    *            memory (defaults: LO 2, update 1), or for the ratio kernel
    *            3 (its default) / 4 without shared memory, 4 with fewer
    *            registers (columns of at most 64 layers).
-   * cfg[7]     FP32 form: layers per lane per pass of the edge-flux kernel, 1 or 2
+   * cfg[7]     FP32 form: layers per lane per pass of the per-edge edge-flux
+   *            kernel, 1 or 2
    * cfg[8]     FP32 form, w_split: 0 parallel cyclic reduction, one warp per
    *            column (columns of at most 64 layers; deeper ones always use
    *            the other solver), 1 Thomas sweeps, one lane per column
    * cfg[9]     FP32 form: 1 edge fluxes by the tiled kernel (each tile's node
-   *            rows staged once in shared memory)
+   *            rows staged once in shared memory; the default when cfg[0] and
+   *            cfg[7] are 0 and the fields are 16-byte aligned)
    * cfg[10..11] unused, 0 */
   int cfg[12];
   /* w_split (dynamics%use_wsplit, lib/oce_adv_tra_driver.F90:221-231): NULL
