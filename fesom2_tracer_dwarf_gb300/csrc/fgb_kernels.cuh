@@ -16,7 +16,9 @@
 #pragma once
 #include <cstdint>
 
+#include "fgb_bits.cuh"
 #include "fgb_device.hpp"
+#include "fgb_intdiv.cuh"
 
 #ifndef FGB_FAST64
 #define FGB_FAST64 0
@@ -48,22 +50,26 @@ struct GeoSel<float> {
   __host__ __device__ static const GeoPtrs<float>& get(const DMesh& m) { return m.g32; }
 };
 
+// a < b ? a : b and a > b ? a : b, compared on the integer pipe.
 template <typename R>
-__device__ __forceinline__ R rmin(R a, R b) { return a < b ? a : b; }
+__device__ __forceinline__ R rmin(R a, R b) { return bits64::lesser(a, b); }
 template <typename R>
-__device__ __forceinline__ R rmax(R a, R b) { return a > b ? a : b; }
+__device__ __forceinline__ R rmax(R a, R b) { return bits64::greater(a, b); }
 template <typename R>
-__device__ __forceinline__ R rabs(R a) { return fabs(a); }
+__device__ __forceinline__ R rabs(R a) { return bits64::magnitude(a); }
 
-// Division: correctly rounded in the FP64 form (bit parity with the CPU
-// restatement), the fast single-precision reciprocal form (about 2 ulp) in
-// the FP32 form.
+// Division: correctly rounded (bit parity with the CPU restatement), on the
+// integer pipe.
 template <typename R>
-__device__ __forceinline__ R fdiv(R a, R b);
-template <>
-__device__ __forceinline__ double fdiv<double>(double a, double b) { return a / b; }
-template <>
-__device__ __forceinline__ float fdiv<float>(float a, float b) { return __fdividef(a, b); }
+__device__ __forceinline__ R fdiv(R a, R b) { return intdiv::divide(a, b); }
+// A divisor shared by several quotients: prepared once in the exact form (the
+// fast form multiplies with reciprocals instead).
+struct LayerDivisor {
+  intdiv::Divisor d;
+  __device__ __forceinline__ explicit LayerDivisor(double b) {
+    if constexpr (!FGB_FAST64) d = intdiv::prepare(b);
+  }
+};
 // a / c for a constant c: the reference's division, or (fast form) the product
 // with the reciprocal constant.
 template <typename R>
@@ -71,12 +77,12 @@ __device__ __forceinline__ R fdivc(R a, R c) {
   if constexpr (FGB_FAST64) return a * (R(1) / c);
   else return fdiv(a, c);
 }
-// (x dt) / areasvol: the reference's order, or (fast form) x times the
-// layer's dt / areasvol, formed once.
+// (x dt) / areasvol: the reference's order with the layer's prepared
+// areasvol, or (fast form) x times the layer's dt / areasvol, formed once.
 template <typename R>
-__device__ __forceinline__ R dt_per_vol(R x, R dt, R av, R rdt_av) {
+__device__ __forceinline__ R dt_per_vol(R x, R dt, const LayerDivisor& av, R rdt_av) {
   if constexpr (FGB_FAST64) return x * rdt_av;
-  else return fdiv(x * dt, av);
+  else return intdiv::divide(x * dt, av.d);
 }
 // a / g for a geometric g shared by the tracers of a column: the reference's
 // division, or (fast form) the product with 1 / g, which the compiler forms
@@ -822,6 +828,35 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_lo(DMesh 
   }
 }
 
+// The larger of lo and t joins the upper bound, the smaller the lower one (integer keys).
+__device__ __forceinline__ void join_bounds(double lo, double t, long long& mx, long long& mn) {
+  const long long a = bits64::key(lo), b = bits64::key(t);
+  const bool gt = a > b;
+  mx = max(mx, gt ? a : b);
+  mn = min(mn, gt ? b : a);
+}
+// The sums of the positive and of the negative terms: a term joins one of them
+// (the other would add an exact zero), so each costs one FP64 addition.
+__device__ __forceinline__ void add_part(double f, double& pos, double& neg) {
+  const bool p = bits64::sign_clear(f);
+  const double t = (p ? pos : neg) + f;
+  pos = p ? t : pos;
+  neg = p ? neg : t;
+}
+// Their first two terms x and -y: max(0, x) + max(0, -y) and min(0, x) + min(0, -y).
+__device__ __forceinline__ void first_parts(double x, double y, double& pos, double& neg) {
+  const bool px = bits64::sign_clear(x), py = !bits64::sign_clear(y);
+  const double t = x - y, u = bits64::negate_if(y, true);
+  pos = px ? (py ? t : x) : (py ? u : 0.0);
+  neg = px ? (py ? 0.0 : u) : (py ? x : t);
+}
+// A NaN term belongs to both sums.
+__device__ __forceinline__ void spread_nan(double& pos, double& neg) {
+  if (bits64::finite(pos, neg)) return;
+  if (isnan(pos)) neg = pos;
+  else if (isnan(neg)) pos = neg;
+}
+
 // ---------------------------------------------------------------------------
 // FCT stage 2: bounds a1-a3, antidiffusive sums b1 and the limiting factors
 // b2 (lib/oce_adv_tra_fct.F90:98-374). The cluster bound is the maximum over
@@ -861,13 +896,14 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_ratio(DMe
       const int k0 = 2 * p, z0 = k0 + 1, z1 = k0 + 2;
       // AUX = -/+1e3 of elements without the layer joins the bound (lib/oce_adv_tra_fct.F90:139-145)
       const R mx0i = z0 > minlev ? -big : -inf, mx1i = z1 > minlev ? -big : -inf;
-      R mx0[KC], mx1[KC], mn0[KC], mn1[KC];
+      // the bounds as integer keys (bits64::key), which order as the values do
+      long long mx0[KC], mx1[KC], mn0[KC], mn1[KC];
 #pragma unroll
       for (int i = 0; i < KC; ++i) {
-        mx0[i] = mx0i;
-        mx1[i] = mx1i;
-        mn0[i] = -mx0i;
-        mn1[i] = -mx1i;
+        mx0[i] = bits64::key(mx0i);
+        mx1[i] = bits64::key(mx1i);
+        mn0[i] = bits64::key(-mx0i);
+        mn1[i] = bits64::key(-mx1i);
       }
 #pragma unroll 2
       for (int j = 0; j < ncl; ++j) {
@@ -878,22 +914,46 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_ratio(DMe
         for (int i = 0; i < KC; ++i) {
           const size_t v = (size_t)node * LZ + k0;
           const vec2<R> lv = ld2(a.lo + (t0 + i) * a.sN + v), tv = ld2(a.T + (t0 + i) * a.sT + v);
-          if (a0) {
-            mx0[i] = rmax(mx0[i], rmax(lv.x, tv.x));
-            mn0[i] = rmin(mn0[i], rmin(lv.x, tv.x));
-          }
-          if (a1) {
-            mx1[i] = rmax(mx1[i], rmax(lv.y, tv.y));
-            mn1[i] = rmin(mn1[i], rmin(lv.y, tv.y));
-          }
+          if (a0) join_bounds(lv.x, tv.x, mx0[i], mn0[i]);
+          if (a1) join_bounds(lv.y, tv.y, mx1[i], mn1[i]);
         }
+      }
+      // A NaN is the largest or the smallest key of all, so it is still there:
+      // the column's bounds again with the floating-point comparisons, whose
+      // outcome with NaNs depends on the order.
+      bool nan = false;
+#pragma unroll
+      for (int i = 0; i < KC; ++i)
+        nan |= max(mx0[i], mx1[i]) > bits64::kKeyInf || min(mn0[i], mn1[i]) < -bits64::kKeyInf - 1;
+      if (nan) {
+        for (int i = 0; i < KC; ++i) {
+          R x0 = mx0i, x1 = mx1i, y0 = -mx0i, y1 = -mx1i;
+          for (int j = 0; j < ncl; ++j) {
+            const int lev = m.cl_lev[c0 + j];
+            const size_t v = (size_t)m.cl_node[c0 + j] * LZ + k0;
+            const vec2<R> lv = ld2(a.lo + (t0 + i) * a.sN + v), tv = ld2(a.T + (t0 + i) * a.sT + v);
+            if (z0 <= lev) {
+              x0 = rmax(x0, rmax(lv.x, tv.x));
+              y0 = rmin(y0, rmin(lv.x, tv.x));
+            }
+            if (z1 <= lev) {
+              x1 = rmax(x1, rmax(lv.y, tv.y));
+              y1 = rmin(y1, rmin(lv.y, tv.y));
+            }
+          }
+          smax[i * LW + k0] = x0;
+          smax[i * LW + k0 + 1] = x1;
+          smin[i * LW + k0] = y0;
+          smin[i * LW + k0 + 1] = y1;
+        }
+        continue;
       }
 #pragma unroll
       for (int i = 0; i < KC; ++i) {
-        smax[i * LW + k0] = mx0[i];
-        smax[i * LW + k0 + 1] = mx1[i];
-        smin[i * LW + k0] = mn0[i];
-        smin[i * LW + k0 + 1] = mn1[i];
+        smax[i * LW + k0] = bits64::unkey(mx0[i]);
+        smax[i * LW + k0 + 1] = bits64::unkey(mx1[i]);
+        smin[i * LW + k0] = bits64::unkey(mn0[i]);
+        smin[i * LW + k0 + 1] = bits64::unkey(mn1[i]);
       }
     }
     __syncwarp();
@@ -903,10 +963,8 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_ratio(DMe
 #pragma unroll
       for (int i = 0; i < KC; ++i) {
         const R* ad = sadv + i * LW;
-        pl0[i] = R(0) + (rmax(R(0), ad[k0]) + rmax(R(0), -ad[k0 + 1]));
-        mi0[i] = R(0) + (rmin(R(0), ad[k0]) + rmin(R(0), -ad[k0 + 1]));
-        pl1[i] = R(0) + (rmax(R(0), ad[k0 + 1]) + rmax(R(0), -ad[k0 + 2]));
-        mi1[i] = R(0) + (rmin(R(0), ad[k0 + 1]) + rmin(R(0), -ad[k0 + 2]));
+        first_parts(ad[k0], ad[k0 + 1], pl0[i], mi0[i]);
+        first_parts(ad[k0 + 1], ad[k0 + 2], pl1[i], mi1[i]);
       }
       const int z0 = k0 + 1, z1 = k0 + 2;
 #pragma unroll 2
@@ -915,22 +973,13 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_ratio(DMe
         const bool a0 = z0 >= q.lo && z0 <= q.hi, a1 = z1 >= q.lo && z1 <= q.hi;
 #pragma unroll
         for (int i = 0; i < KC; ++i) {
-          vec2<R> f = ld2(a.adfh + (t0 + i) * a.sE + (size_t)q.e * LZ + k0);
-          if (q.role) {
-            f.x = -f.x;
-            f.y = -f.y;
-          }
-          if (a0) {
-            pl0[i] = pl0[i] + rmax(R(0), f.x);
-            mi0[i] = mi0[i] + rmin(R(0), f.x);
-          }
-          if (a1) {
-            pl1[i] = pl1[i] + rmax(R(0), f.y);
-            mi1[i] = mi1[i] + rmin(R(0), f.y);
-          }
+          const vec2<R> f = ld2(a.adfh + (t0 + i) * a.sE + (size_t)q.e * LZ + k0);
+          if (a0) add_part(bits64::negate_if(f.x, q.role), pl0[i], mi0[i]);
+          if (a1) add_part(bits64::negate_if(f.y, q.role), pl1[i], mi1[i]);
         }
       }
       const vec2<R> av = ld2(g.areasvol + n * LZ + k0);
+      const LayerDivisor dv[2] = {LayerDivisor(av.x), LayerDivisor(av.y)};
 #pragma unroll
       for (int i = 0; i < KC; ++i) {
         const R* mxs = smax + i * LW;
@@ -952,9 +1001,11 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_ratio(DMe
           }
           const R avk = l ? av.y : av.x;
           const R rdk = rdt_vol(dt, avk);
-          R flux = dt_per_vol((l ? pl1[i] : pl0[i]), dt, avk, rdk) + R(1e-16);
+          R pl = l ? pl1[i] : pl0[i], mi = l ? mi1[i] : mi0[i];
+          spread_nan(pl, mi);
+          R flux = dt_per_vol(pl, dt, dv[l], rdk) + R(1e-16);
           out_p[l] = rmin(R(1), fdiv(bmax, flux));
-          flux = dt_per_vol((l ? mi1[i] : mi0[i]), dt, avk, rdk) - R(1e-16);
+          flux = dt_per_vol(mi, dt, dv[l], rdk) - R(1e-16);
           out_m[l] = rmin(R(1), fdiv(bmin, flux));
         }
         st4(a.rpm + 2 * ((t0 + i) * a.sN + n * LZ + k0), out_p[0], out_m[0], out_p[1], out_m[1]);
@@ -1005,21 +1056,10 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_update(DM
       for (int iz = lane; iz < nl; iz += kWarp) {
         const int z = iz + 1;
         R f = adfv[iz];
-        if (z == nzmin) {
-          R ae = R(1);
-          ae = (f >= R(0)) ? rmin(ae, Rp[iz]) : rmin(ae, Rm[iz]);
-          f = ae * f;
-        } else if (z > nzmin && z <= nzmax - 1) {
-          R ae = R(1);
-          if (f >= R(0)) {
-            ae = rmin(ae, Rm[iz - 1]);
-            ae = rmin(ae, Rp[iz]);
-          } else {
-            ae = rmin(ae, Rp[iz - 1]);
-            ae = rmin(ae, Rm[iz]);
-          }
-          f = ae * f;
-        }
+        const bool pos = bits64::sign_clear(f);
+        if (z == nzmin) f = (pos ? Rp[iz] : Rm[iz]) * f;
+        else if (z > nzmin && z <= nzmax - 1)
+          f = rmin(pos ? Rm[iz - 1] : Rp[iz - 1], pos ? Rp[iz] : Rm[iz]) * f;
         sLv[i * LW + iz] = f;
       }
     }
@@ -1028,6 +1068,7 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_update(DM
       const int k0 = 2 * p, z0 = k0 + 1, z1 = k0 + 2;
       const vec2<R> av = ld2(g.areasvol + n * LZ + k0);
       const vec2<R> rd{rdt_vol(dt, av.x), rdt_vol(dt, av.y)};  // fast form only
+      const LayerDivisor vd0(av.x), vd1(av.y);                   // exact form only
       R dh0[KC], dh1[KC];
 #pragma unroll
       for (int i = 0; i < KC; ++i) dh0[i] = dh1[i] = R(0);
@@ -1043,27 +1084,26 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_update(DM
           const vec2<R> rpo{ro.a, ro.c}, rmo{ro.b, ro.d};
           const R rpn0 = sRp[i * LW + k0], rpn1 = sRp[i * LW + k0 + 1];
           const R rmn0 = sRm[i * LW + k0], rmn1 = sRm[i * LW + k0 + 1];
-          R ae0 = R(1), ae1 = R(1);
-          if (q.role) {  // this node is the edge's second node
-            if (f.x >= R(0)) { ae0 = rmin(ae0, rpo.x); ae0 = rmin(ae0, rmn0); }
-            else { ae0 = rmin(ae0, rmo.x); ae0 = rmin(ae0, rpn0); }
-            if (f.y >= R(0)) { ae1 = rmin(ae1, rpo.y); ae1 = rmin(ae1, rmn1); }
-            else { ae1 = rmin(ae1, rmo.y); ae1 = rmin(ae1, rpn1); }
-            if (a0) dh0[i] = dh0[i] - dt_per_vol(ae0 * f.x, dt, av.x, rd.x);
-            if (a1) dh1[i] = dh1[i] - dt_per_vol(ae1 * f.y, dt, av.y, rd.y);
-          } else {
-            if (f.x >= R(0)) { ae0 = rmin(ae0, rpn0); ae0 = rmin(ae0, rmo.x); }
-            else { ae0 = rmin(ae0, rmn0); ae0 = rmin(ae0, rpo.x); }
-            if (f.y >= R(0)) { ae1 = rmin(ae1, rpn1); ae1 = rmin(ae1, rmo.y); }
-            else { ae1 = rmin(ae1, rmn1); ae1 = rmin(ae1, rpo.y); }
-            if (a0) dh0[i] = dh0[i] + dt_per_vol(ae0 * f.x, dt, av.x, rd.x);
-            if (a1) dh1[i] = dh1[i] + dt_per_vol(ae1 * f.y, dt, av.y, rd.y);
+          // this node's factor and the other one's, for the flux's sign; the reference takes the
+          // first node's against the second node's
+          if (a0) {
+            const bool up = bits64::sign_clear(f.x) != (bool)q.role;
+            const R own = up ? rpn0 : rmn0, oth = up ? rmo.x : rpo.x;
+            const R x = dt_per_vol((q.role ? rmin(oth, own) : rmin(own, oth)) * f.x, dt, vd0, rd.x);
+            dh0[i] = q.role ? dh0[i] - x : dh0[i] + x;
+          }
+          if (a1) {
+            const bool up = bits64::sign_clear(f.y) != (bool)q.role;
+            const R own = up ? rpn1 : rmn1, oth = up ? rmo.y : rpo.y;
+            const R x = dt_per_vol((q.role ? rmin(oth, own) : rmin(own, oth)) * f.y, dt, vd1, rd.y);
+            dh1[i] = q.role ? dh1[i] - x : dh1[i] + x;
           }
         }
       }
       const vec2<R> hn = ld2(g.hnode + n * LZ + k0), hnn = ld2(g.hnode_new + n * LZ + k0);
       const bool w0 = z0 >= nzmin && z0 <= nzmax - 1, w1 = z1 >= nzmin && z1 <= nzmax - 1;
       const vec2<R> rh{FGB_FAST64 ? R(1) / hnn.x : R(0), FGB_FAST64 ? R(1) / hnn.y : R(0)};
+      const LayerDivisor hd0(hnn.x), hd1(hnn.y);
 #pragma unroll
       for (int i = 0; i < KC; ++i) {
         R* __restrict__ T = a.T + (t0 + i) * a.sT + n * LZ + k0;
@@ -1072,18 +1112,18 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_update(DM
         const R* Lv = sLv + i * LW;
         R* del = a.del ? a.del + (t0 + i) * a.sN + n * LZ + k0 : nullptr;
         const vec2<R> d0 = del ? ld2(del) : vec2<R>{R(0), R(0)};
-        R dv0 = (R(0) - Tn.x * hn.x) + lo.x * hnn.x;
-        dv0 = dv0 + dt_per_vol(Lv[k0] - Lv[k0 + 1], dt, av.x, rd.x);
-        R dv1 = (R(0) - Tn.y * hn.y) + lo.y * hnn.y;
-        dv1 = dv1 + dt_per_vol(Lv[k0 + 1] - Lv[k0 + 2], dt, av.y, rd.y);
-        const R e0 = d0.x + dh0[i] + dv0, e1 = d0.y + dh1[i] + dv1;
+        R dv0 = lo.x * hnn.x - Tn.x * hn.x;  // the reference's (0 - T hnode) + LO hnode_new
+        dv0 = dv0 + dt_per_vol(Lv[k0] - Lv[k0 + 1], dt, vd0, rd.x);
+        R dv1 = lo.y * hnn.y - Tn.y * hn.y;
+        dv1 = dv1 + dt_per_vol(Lv[k0 + 1] - Lv[k0 + 2], dt, vd1, rd.y);
+        const R e0 = (del ? d0.x + dh0[i] : dh0[i]) + dv0, e1 = (del ? d0.y + dh1[i] : dh1[i]) + dv1;
         R n0 = Tn.x, n1v = Tn.y;
         if constexpr (FGB_FAST64) {
           if (w0) n0 = Tn.x + e0 * rh.x;
           if (w1) n1v = Tn.y + e1 * rh.y;
         } else {
-          if (w0) n0 = Tn.x + fdiv(e0, hnn.x);
-          if (w1) n1v = Tn.y + fdiv(e1, hnn.y);
+          if (w0) n0 = Tn.x + intdiv::divide(e0, hd0.d);
+          if (w1) n1v = Tn.y + intdiv::divide(e1, hd1.d);
         }
         st2(T, n0, n1v);
         if (del) st2(del, w0 ? e0 : d0.x, w1 ? e1 : d0.y);
@@ -1148,6 +1188,7 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_nofct_update(
       const int k0 = 2 * p, z0 = k0 + 1, z1 = k0 + 2;
       const vec2<R> av = ld2(g.areasvol + n * LZ + k0);
       const vec2<R> rd{rdt_vol(dt, av.x), rdt_vol(dt, av.y)};  // fast form only
+      const LayerDivisor vd0(av.x), vd1(av.y);                   // exact form only
       R dh0[KC], dh1[KC];
 #pragma unroll
       for (int i = 0; i < KC; ++i) dh0[i] = dh1[i] = R(0);
@@ -1159,17 +1200,18 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_nofct_update(
         for (int i = 0; i < KC; ++i) {
           const vec2<R> f = ld2(a.adfh + (t0 + i) * a.sE + (size_t)q.e * LZ + k0);
           if (q.role) {
-            if (a0) dh0[i] = dh0[i] - dt_per_vol(f.x, dt, av.x, rd.x);
-            if (a1) dh1[i] = dh1[i] - dt_per_vol(f.y, dt, av.y, rd.y);
+            if (a0) dh0[i] = dh0[i] - dt_per_vol(f.x, dt, vd0, rd.x);
+            if (a1) dh1[i] = dh1[i] - dt_per_vol(f.y, dt, vd1, rd.y);
           } else {
-            if (a0) dh0[i] = dh0[i] + dt_per_vol(f.x, dt, av.x, rd.x);
-            if (a1) dh1[i] = dh1[i] + dt_per_vol(f.y, dt, av.y, rd.y);
+            if (a0) dh0[i] = dh0[i] + dt_per_vol(f.x, dt, vd0, rd.x);
+            if (a1) dh1[i] = dh1[i] + dt_per_vol(f.y, dt, vd1, rd.y);
           }
         }
       }
       const vec2<R> hnn = ld2(g.hnode_new + n * LZ + k0);
       const bool w0 = z0 >= nzmin && z0 <= nzmax - 1, w1 = z1 >= nzmin && z1 <= nzmax - 1;
       const vec2<R> rh{FGB_FAST64 ? R(1) / hnn.x : R(0), FGB_FAST64 ? R(1) / hnn.y : R(0)};
+      const LayerDivisor hd0(hnn.x), hd1(hnn.y);
 #pragma unroll
       for (int i = 0; i < KC; ++i) {
         const R* F = sF + i * LW;
@@ -1177,16 +1219,16 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_nofct_update(
         const vec2<R> Tn = ld2(T);
         R* del = a.del ? a.del + (t0 + i) * a.sN + n * LZ + k0 : nullptr;
         const vec2<R> d0 = del ? ld2(del) : vec2<R>{R(0), R(0)};
-        const R dv0 = R(0) + dt_per_vol(F[k0] - F[k0 + 1], dt, av.x, rd.x);
-        const R dv1 = R(0) + dt_per_vol(F[k0 + 1] - F[k0 + 2], dt, av.y, rd.y);
-        const R e0 = d0.x + dh0[i] + dv0, e1 = d0.y + dh1[i] + dv1;
+        const R dv0 = dt_per_vol(F[k0] - F[k0 + 1], dt, vd0, rd.x);
+        const R dv1 = dt_per_vol(F[k0 + 1] - F[k0 + 2], dt, vd1, rd.y);
+        const R e0 = (del ? d0.x + dh0[i] : dh0[i]) + dv0, e1 = (del ? d0.y + dh1[i] : dh1[i]) + dv1;
         R n0 = Tn.x, n1v = Tn.y;
         if constexpr (FGB_FAST64) {
           if (w0) n0 = Tn.x + e0 * rh.x;
           if (w1) n1v = Tn.y + e1 * rh.y;
         } else {
-          if (w0) n0 = Tn.x + fdiv(e0, hnn.x);
-          if (w1) n1v = Tn.y + fdiv(e1, hnn.y);
+          if (w0) n0 = Tn.x + intdiv::divide(e0, hd0.d);
+          if (w1) n1v = Tn.y + intdiv::divide(e1, hd1.d);
         }
         st2(T, n0, n1v);
         if (del) st2(del, w0 ? e0 : d0.x, w1 ? e1 : d0.y);

@@ -11,7 +11,7 @@ torch = pytest.importorskip("torch")
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision,V", [("fp64", 1), ("fp32", 2), ("fp32", 4)])
-@pytest.mark.parametrize("nx,ny,nl", [(3, 3, 2), (17, 17, 2), (18, 17, 2), (129, 129, 17), (130, 129, 17)])
+@pytest.mark.parametrize("nx,ny,nl", [(3, 3, 3), (17, 9, 3), (18, 9, 3), (129, 129, 17), (130, 129, 17)])
 def test_stats_block_split(nx, ny, nl, precision, V):
     if not torch.cuda.is_available():
         pytest.skip("needs a CUDA GPU")
