@@ -33,14 +33,26 @@ __device__ __forceinline__ unsigned mag_hi(double x) { return (unsigned)(to_bits
 __device__ __forceinline__ bool finite(double x) { return mag_hi(x) < 0x7ff00000u; }
 __device__ __forceinline__ bool finite(double x, double y) { return max(mag_hi(x), mag_hi(y)) < 0x7ff00000u; }
 
+// The floating-point expressions behind the integer ones: out of line, because
+// the compiler would otherwise predicate these few instructions into the common
+// path, where they occupy the FP64 pipe all the same.
+static __device__ __noinline__ double hw_lesser(double a, double b) { return a < b ? a : b; }
+static __device__ __noinline__ double hw_greater(double a, double b) { return a > b ? a : b; }
+static __device__ __noinline__ bool hw_exceeds(double a, double b) { return a > b; }
+static __device__ __noinline__ double hw_scale(double x, double s) { return x * s; }
+static __device__ __noinline__ double hw_upwind(double v, double t1, double t2) {
+  return 0.5 * (t1 * (v + fabs(v)) + t2 * (v - fabs(v)));
+}
+static __device__ __noinline__ bool hw_product_positive(double a, double b) { return a * b > 0.0; }
+
 // a < b ? a : b
 __device__ __forceinline__ double lesser(double a, double b) {
-  if (!finite(a, b)) return a < b ? a : b;
+  if (!finite(a, b)) return hw_lesser(a, b);
   return key(a) < key(b) ? a : b;
 }
 // a > b ? a : b
 __device__ __forceinline__ double greater(double a, double b) {
-  if (!finite(a, b)) return a > b ? a : b;
+  if (!finite(a, b)) return hw_greater(a, b);
   return key(a) > key(b) ? a : b;
 }
 // x >= 0 by the sign bit: -0 and NaN may go either way.
@@ -55,15 +67,38 @@ __device__ __forceinline__ double magnitude(double x) { return from_bits(to_bits
 __device__ __forceinline__ double twice(double x) {
   const uint64_t b = to_bits(x);
   const unsigned e = (unsigned)(b >> 32) & 0x7ff00000u;
-  if (e - 0x00100000u >= 0x7fd00000u) return x + x;
+  if ((b << 1) == 0) return x;
+  if (e - 0x00100000u >= 0x7fd00000u) return hw_scale(x, 2.0);
   return from_bits(b + (1ull << 52));
 }
 __device__ __forceinline__ double half(double x) {
   const uint64_t b = to_bits(x);
   const unsigned e = (unsigned)(b >> 32) & 0x7ff00000u;
-  if (e - 0x00200000u >= 0x7fd00000u) return x * 0.5;
+  if ((b << 1) == 0) return x;
+  if (e - 0x00200000u >= 0x7fd00000u) return hw_scale(x, 0.5);
   return from_bits(b - (1ull << 52));
 }
+
+// (t1 (v + |v|) + t2 (v - |v|)) / 2, the upwind product of a first-order flux:
+// one factor in brackets is zero and the other 2 v, so it is v times the
+// upwind value, one FP64 instruction (the same bits unless the product is
+// subnormal). Infinities, NaNs and numbers whose double overflows by the
+// expression as written.
+__device__ __forceinline__ double upwind(double v, double t1, double t2) {
+  if (max(mag_hi(v), max(mag_hi(t1), mag_hi(t2))) >= 0x7fe00000u)
+    return hw_upwind(v, t1, t2);
+  return (sign_clear(v) ? t1 : t2) * v;
+}
+// a * b > 0, from the signs; factors small enough for the product to vanish by multiplication.
+__device__ __forceinline__ bool product_positive(double a, double b) {
+  const uint64_t ua = to_bits(a), ub = to_bits(b);
+  if ((ua << 1) == 0 || (ub << 1) == 0) return false;
+  const unsigned ea = mag_hi(a) >> 20, eb = mag_hi(b) >> 20;  // biased exponents
+  if (min(ea, eb) < 550u || max(ea, eb) == 0x7ffu) return hw_product_positive(a, b);
+  return (long long)(ua ^ ub) >= 0;
+}
+// a > b (of finite zeros: +0 > -0).
+__device__ __forceinline__ bool exceeds(double a, double b) { return finite(a, b) ? key(a) > key(b) : hw_exceeds(a, b); }
 
 }  // namespace bits64
 }  // namespace fgb

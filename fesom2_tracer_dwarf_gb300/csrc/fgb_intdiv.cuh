@@ -110,6 +110,10 @@ FGB_HD Divisor prepare(double b) {
   return d;
 }
 
+// The divisors 3 and 6: x = floor(2^64 / 1.5).
+FGB_HD Divisor three() { return Divisor{0xaaaaaaaaaaaaaaaaull, 3.0, 1024}; }
+FGB_HD Divisor six() { return Divisor{0xaaaaaaaaaaaaaaaaull, 6.0, 1025}; }
+
 // a / d.b, rounded to nearest even.
 FGB_HD double divide(double a, const Divisor& d) {
   const uint64_t bits = to_bits(a), A = significand(bits);

@@ -70,12 +70,15 @@ struct LayerDivisor {
     if constexpr (!FGB_FAST64) d = intdiv::prepare(b);
   }
 };
-// a / c for a constant c: the reference's division, or (fast form) the product
-// with the reciprocal constant.
-template <typename R>
-__device__ __forceinline__ R fdivc(R a, R c) {
-  if constexpr (FGB_FAST64) return a * (R(1) / c);
-  else return fdiv(a, c);
+// a / 3 and a / 6: the reference's division, or (fast form) the product with
+// the reciprocal constant.
+__device__ __forceinline__ double third(double a) {
+  if constexpr (FGB_FAST64) return a * (1.0 / 3.0);
+  else return intdiv::divide(a, intdiv::three());
+}
+__device__ __forceinline__ double sixth(double a) {
+  if constexpr (FGB_FAST64) return a * (1.0 / 6.0);
+  else return intdiv::divide(a, intdiv::six());
 }
 // (x dt) / areasvol: the reference's order with the layer's prepared
 // areasvol, or (fast form) x times the layer's dt / areasvol, formed once.
@@ -84,17 +87,9 @@ __device__ __forceinline__ R dt_per_vol(R x, R dt, const LayerDivisor& av, R rdt
   if constexpr (FGB_FAST64) return x * rdt_av;
   else return intdiv::divide(x * dt, av.d);
 }
-// a / g for a geometric g shared by the tracers of a column: the reference's
-// division, or (fast form) the product with 1 / g, which the compiler forms
-// once for all tracers.
-template <typename R>
-__device__ __forceinline__ R fdivg(R a, R g) {
-  if constexpr (FGB_FAST64) return a * (R(1) / g);
-  else return fdiv(a, g);
-}
 template <typename R>
 __device__ __forceinline__ R rdt_vol(R dt, R av) {
-  if constexpr (FGB_FAST64) return dt / av;
+  if constexpr (FGB_FAST64) return fdiv(dt, av);
   else return R(0);  // unused by the exact form
 }
 
@@ -261,11 +256,11 @@ __device__ __forceinline__ R ho_flux(R v, R vp, R vm, R ta1, R ta2, R g1, R g2, 
   if (HOR == 0) return -(R(0.5) * (ta1 * vp + ta2 * vm));
   R Tm2, Tm1;
   if (HOR == 1) {
-    Tm2 = ta2 - fdivc(R(2) * (ta2 - ta1) + ex * g2 + ey * g4, R(6)) * c2;
-    Tm1 = ta1 + fdivc(R(2) * (ta2 - ta1) + ex * g1 + ey * g3, R(6)) * c1;
+    Tm2 = ta2 - sixth(R(2) * (ta2 - ta1) + ex * g2 + ey * g4) * c2;
+    Tm1 = ta1 + sixth(R(2) * (ta2 - ta1) + ex * g1 + ey * g3) * c1;
   } else {
-    Tm2 = ta2 - fdivc(R(2) * (ta2 - ta1) + ex * g2 + ey * g4, R(6));
-    Tm1 = ta1 + fdivc(R(2) * (ta2 - ta1) + ex * g1 + ey * g3, R(6));
+    Tm2 = ta2 - sixth(R(2) * (ta2 - ta1) + ex * g2 + ey * g4);
+    Tm1 = ta1 + sixth(R(2) * (ta2 - ta1) + ex * g1 + ey * g3);
   }
   const R cHO = vp * Tm1 + vm * Tm2;
   return -((R(0.5) * (R(1) - ph)) * cHO) - ((v * ph) * R(0.5)) * (Tm1 + Tm2);
@@ -404,31 +399,46 @@ template <typename R>
 __device__ __forceinline__ R ver_upw1(const Col<R>& c, int z, int nzmin, int nzmax, R fold) {
   if (z == nzmin) return -((c.W[z - 1] * c.T[z - 1]) * c.area[z - 1]) - fold;
   if (z == nzmax) return R(0) - fold;
-  const R W = c.W[z - 1];
-  return -((R(0.5) * (c.T[z - 1] * (W + rabs(W)) + c.T[z - 2] * (W - rabs(W)))) * c.area[z - 1]) - fold;
+  return -(bits64::upwind(c.W[z - 1], c.T[z - 1], c.T[z - 2]) * c.area[z - 1]) - fold;
 }
 
+// QR4C: the layer-to-layer slopes (T(z-1) - T(z)) / (Z(z-1) - Z(z)) are staged in c.tv by
+// interface (qr4c_slopes): an interface uses its own and both neighbours'.
 template <typename R>
 __device__ __forceinline__ R ver_qr4c(const Col<R>& c, int z, int nzmin, int nzmax, R num_ord, R fold) {
   const R W = c.W[z - 1];
   if (z == nzmin) return -((c.T[z - 1] * W) * c.area[z - 1]) - fold;
   if (z == nzmax) return R(0) - fold;
   if (z == nzmin + 1 || z == nzmax - 1) {
-    const R x = -(((R(0.5) * (c.T[z - 2] + c.T[z - 1])) * W) * c.area[z - 1]);
+    const R x = -((bits64::half(c.T[z - 2] + c.T[z - 1]) * W) * c.area[z - 1]);
     R f = x - fold;
     if (nzmin + 1 == nzmax - 1) f = x - f;  // written twice (lib/oce_adv_tra_ver.F90:405-411)
     return f;
   }
-  const R T0 = c.T[z - 1], Tm1 = c.T[z - 2], Tm2 = c.T[z - 3], Tp1 = c.T[z];
-  const R Z0 = c.Z[z - 1], Zm1 = c.Z[z - 2], Zm2 = c.Z[z - 3], Zp1 = c.Z[z];
-  const R qc = fdivg(Tm1 - T0, Zm1 - Z0);
-  const R qu = fdivg(T0 - Tp1, Z0 - Zp1);
-  const R qd = fdivg(Tm2 - Tm1, Zm2 - Zm1);
+  const R T0 = c.T[z - 1], Tm1 = c.T[z - 2];
+  const R q2 = bits64::twice(c.tv[z - 1]), qu = c.tv[z], qd = c.tv[z - 2];
   const R zb = c.zb[z - 1];
-  const R tm1 = T0 + fdivc((R(2) * qc + qu) * (zb - Z0), R(3));
-  const R tm2 = Tm1 + fdivc((R(2) * qc + qd) * (zb - Zm1), R(3));
+  const R tm1 = T0 + third((q2 + qu) * (zb - c.Z[z - 1]));
+  const R tm2 = Tm1 + third((q2 + qd) * (zb - c.Z[z - 2]));
+  const R mean = (num_ord * bits64::half(tm1 + tm2)) * W;
+  // num_ord = 1: the upwind part is an exact zero (of finite values)
+  if (num_ord == R(1) && bits64::finite(tm1, tm2) && bits64::finite(W)) return -mean * c.area[z - 1] - fold;
   const R tm = (W + rabs(W)) * tm1 + (W - rabs(W)) * tm2;
-  return (-((R(0.5) * (R(1) - num_ord)) * tm) - (num_ord * (R(0.5) * (tm1 + tm2))) * W) * c.area[z - 1] - fold;
+  return (-((R(0.5) * (R(1) - num_ord)) * tm) - mean) * c.area[z - 1] - fold;
+}
+
+// The slopes of KC tracer columns (T, q: LW apart), the divisor of an interface prepared once.
+template <typename R, int KC>
+__device__ __forceinline__ void qr4c_slopes(const R* T, const R* Z, R* q, int LW, int nzmin, int nzmax, int lane) {
+  for (int iz = nzmin + lane; iz < nzmax - 1; iz += kWarp) {
+    const intdiv::Divisor dz = intdiv::prepare(Z[iz - 1] - Z[iz]);
+    const R rz = FGB_FAST64 ? intdiv::divide(R(1), dz) : R(0);
+#pragma unroll
+    for (int i = 0; i < KC; ++i) {
+      const R d = T[i * LW + iz - 1] - T[i * LW + iz];
+      q[i * LW + iz] = FGB_FAST64 ? d * rz : intdiv::divide(d, dz);
+    }
+  }
 }
 
 template <typename R>
@@ -436,63 +446,58 @@ __device__ __forceinline__ R ver_cdiff(const Col<R>& c, int z, int nzmin, int nl
   const int nzmax = nlev - 1;  // lib/oce_adv_tra_ver.F90:689
   if (z == nzmin) return -((c.W[z - 1] * c.T[z - 1]) * c.area[z - 1]) - fold;
   if (z <= nzmax) {
-    const R tv = R(0.5) * (c.T[z - 2] + c.T[z - 1]);
+    const R tv = bits64::half(c.T[z - 2] + c.T[z - 1]);
     return -((tv * c.W[z - 1]) * c.area[z - 1]) - fold;
   }
   return fold;  // the bottom interface is left untouched
 }
 
-// PPM edge value tv(z) of lib/oce_adv_tra_ver.F90:510-594; the later
-// assignment wins where the special cases coincide.
+// PPM edge value tv(z) of lib/oce_adv_tra_ver.F90:510-594 outside its
+// four-point range (column_ppm has that); the later assignment wins where the
+// special cases coincide.
 template <typename R>
-__device__ __forceinline__ R ppm_tv(const Col<R>& c, int z, int nzmin, int nzmax) {
-  const R* T = c.T;
-  if (z >= nzmin + 2 && z <= nzmax - 2) {
-    const int nz = z - 1;  // layer whose upper neighbour interface is z
-    const R dzjm1 = c.hnn[nz - 2], dzj = c.hnn[nz - 1], dzjp1 = c.hnn[nz], dzjp2 = c.hnn[nz + 1];
-    const R Tm = T[nz - 2], T0 = T[nz - 1], Tp = T[nz], Tpp = T[nz + 1];
-    R deltaj = fdiv(dzj, dzjm1 + dzj + dzjp1) *
-               (fdiv(R(2) * dzjm1 + dzj, dzjp1 + dzj) * (Tp - T0) + fdiv(dzj + R(2) * dzjp1, dzjm1 + dzj) * (T0 - Tm));
-    R deltajp1 = fdiv(dzjp1, dzj + dzjp1 + dzjp2) *
-                 (fdiv(R(2) * dzj + dzjp1, dzjp2 + dzjp1) * (Tpp - Tp) + fdiv(dzjp1 + R(2) * dzjp2, dzj + dzjp1) * (Tp - T0));
-    if ((Tp - T0) * (T0 - Tm) > R(0))
-      deltaj = rmin(rmin(rabs(deltaj), R(2) * rabs(Tp - T0)), R(2) * rabs(T0 - Tm)) * copysign(R(1), deltaj);
-    else
-      deltaj = R(0);
-    if ((Tpp - Tp) * (Tp - T0) > R(0))
-      deltajp1 = rmin(rmin(rabs(deltajp1), R(2) * rabs(Tpp - Tp)), R(2) * rabs(Tp - T0)) * copysign(R(1), deltajp1);
-    else
-      deltajp1 = R(0);
-    const R inner1 = fdiv((R(2) * dzjp1) * dzj, dzj + dzjp1) *
-                     (fdiv(dzjm1 + dzj, R(2) * dzj + dzjp1) - fdiv(dzjp2 + dzjp1, R(2) * dzjp1 + dzj)) * (Tp - T0);
-    const R inner2 = fdiv(dzj * (dzjm1 + dzj), R(2) * dzj + dzjp1) * deltajp1;
-    const R inner3 = fdiv(dzjp1 * (dzjp1 + dzjp2), dzj + R(2) * dzjp1) * deltaj;
-    return (T0 + fdiv(dzj, dzj + dzjp1) * (Tp - T0)) + fdiv(R(1), dzjm1 + dzj + dzjp1 + dzjp2) * (inner1 - inner2 + inner3);
-  }
+__device__ __forceinline__ R ppm_tv_end(const R* T, const R* W, int z, int nzmin, int nzmax) {
   if (z == nzmax) return T[nzmax - 2];
   if (z == nzmax - 1) {
-    const R s = copysign(R(1), c.W[nzmax - 2]);
-    return -(T[nzmax - 3] * rmin(s, R(0))) + T[nzmax - 2] * rmax(s, R(0));
+    const R Tu = T[nzmax - 3], Tl = T[nzmax - 2];
+    if (bits64::finite(Tu, Tl)) return bits64::sign_clear(W[nzmax - 2]) ? Tl : Tu;
+    const R s = copysign(R(1), W[nzmax - 2]);
+    return -(Tu * rmin(s, R(0))) + Tl * rmax(s, R(0));
   }
-  if (z == nzmin + 1) return R(0.5) * (T[nzmin - 1] + T[nzmin]);
+  if (z == nzmin + 1) return bits64::half(T[nzmin - 1] + T[nzmin]);
   return T[nzmin - 1];
 }
 
-// The tracer part of ppm_layer for a given x = min(|W| dt / h, 1) of the layer.
+// The flux of a layer's parabola through one of its interfaces
+// (lib/oce_adv_tra_ver.F90:598-632) for x = min(|W| dt / h, 1), hx = x / 2 and
+// cx = 1 - 2/3 x of the layer.
 template <typename R>
-__device__ __forceinline__ R ppm_layer_x(R aL, R aR, R T0, R x, bool upper, R area, R W) {
-  if ((aR - T0) * (T0 - aL) <= R(0)) {
-    aL = T0;
-    aR = T0;
+__device__ __forceinline__ R ppm_layer_x(R aL, R aR, R T0, R hx, R cx, bool upper, R area, R W) {
+  if (!bits64::product_positive(aR - T0, T0 - aL)) {
+    // (a NaN product is not <= 0)
+    if (bits64::finite(aR, aL) && bits64::finite(T0)) {
+      aL = T0;
+      aR = T0;
+    } else if ((aR - T0) * (T0 - aL) <= R(0)) {
+      aL = T0;
+      aR = T0;
+    }
   }
-  if ((aR - aL) * (T0 - R(0.5) * (aL + aR)) > fdivc((aR - aL) * (aR - aL), R(6))) aL = R(3) * T0 - R(2) * aR;
-  if ((aR - aL) * (T0 - R(0.5) * (aR + aL)) < -fdivc((aR - aL) * (aR - aL), R(6))) aR = R(3) * T0 - R(2) * aL;
-  const R aj = R(6) * (T0 - R(0.5) * (aL + aR));
-  if (upper) {
-    R tv = -aL - (R(0.5) * x) * ((aR - aL) + (R(1) - fdivc(R(2), R(3)) * x) * aj);
-    return (tv * area) * W;
+  R d = aR - aL, c = T0 - bits64::half(aL + aR), dc = d * c, dd = sixth(d * d);
+  if (bits64::exceeds(dc, dd)) {
+    aL = R(3) * T0 - bits64::twice(aR);
+    d = aR - aL;
+    c = T0 - bits64::half(aR + aL);
+    dc = d * c;
+    dd = sixth(d * d);
   }
-  R tv = -aR + (R(0.5) * x) * ((aR - aL) - (R(1) - fdivc(R(2), R(3)) * x) * aj);
+  if (bits64::exceeds(-dd, dc)) {
+    aR = R(3) * T0 - bits64::twice(aL);
+    d = aR - aL;
+    c = T0 - bits64::half(aL + aR);
+  }
+  const R aj = R(6) * c;
+  const R tv = upper ? -aL - hx * (d + cx * aj) : -aR + hx * (d - cx * aj);
   return (tv * area) * W;
 }
 
@@ -502,37 +507,10 @@ __device__ __forceinline__ R ppm_x(R W, R dt, R dzj, bool upper) {
   return upper ? rmin(fdiv(W * dt, dzj), R(1)) : rmin(-fdiv(W * dt, dzj), R(1));
 }
 
-// PPM flux contribution of layer nz to its interface (upper: W(nz) > 0 side,
-// lower: W(nz+1) < 0 side), lib/oce_adv_tra_ver.F90:598-632.
-template <typename R>
-__device__ __forceinline__ R ppm_layer(const Col<R>& c, int nz, bool upper, R dt) {
-  const R dzj = c.hn[nz - 1];
-  if (upper) {
-    const R W = c.W[nz - 1];
-    return ppm_layer_x(c.tv[nz - 1], c.tv[nz], c.T[nz - 1], ppm_x(W, dt, dzj, true), true, c.area[nz - 1], W);
-  }
-  const R W = c.W[nz];
-  return ppm_layer_x(c.tv[nz - 1], c.tv[nz], c.T[nz - 1], ppm_x(W, dt, dzj, false), false, c.area[nz], W);
-}
-
-template <typename R>
-__device__ __forceinline__ R ver_ppm(const Col<R>& c, int z, int nzmin, int nzmax, R dt, R fold) {
-  R tvert = R(0);
-  if (z == nzmin) {
-    tvert = -((c.tv[nzmin - 1] * c.W[nzmin - 1]) * c.area[nzmin - 1]);
-  } else if (z < nzmax) {
-    const R W = c.W[z - 1];
-    if (W > R(0)) tvert = ppm_layer(c, z, true, dt);
-    else if (W < R(0)) tvert = ppm_layer(c, z - 1, false, dt);
-  }
-  return tvert - fold;
-}
-
-template <typename R, int VER>
+template <typename R, int VER>  // not PPM: column_ppm
 __device__ __forceinline__ R ver_flux(const Col<R>& c, int z, int nzmin, int nzmax, R num_ord, R dt, R fold) {
   if (VER == 1) return ver_qr4c(c, z, nzmin, nzmax, num_ord, fold);
   if (VER == 2) return ver_cdiff(c, z, nzmin, nzmax, fold);
-  if (VER == 3) return ver_ppm(c, z, nzmin, nzmax, dt, fold);
   return ver_upw1(c, z, nzmin, nzmax, fold);
 }
 
@@ -549,19 +527,11 @@ __device__ __forceinline__ void stage(R* dst, const R* __restrict__ src, int n, 
   for (int k = lane; k < n; k += kWarp) dst[k] = src[k];
 }
 
-// Vertical HO flux of the column into out[iz] (interfaces), PPM edge values
-// computed first when needed. fold[iz] holds the value subtracted.
+// Vertical flux of the column into out[iz] (interfaces) by a scheme other
+// than PPM; QR4C needs its slopes in c.tv. fold[iz] holds the value subtracted.
 template <typename R, int VER>
-__device__ __forceinline__ void column_ver_flux(Col<R>& c, R* tvbuf, const R* fold, R* out, int nl, int nzmin,
-                                                int nzmax, R num_ord, R dt, int lane) {
-  if (VER == 3) {
-    for (int iz = lane; iz < nl; iz += kWarp) {
-      const int z = iz + 1;
-      tvbuf[iz] = (z >= nzmin && z <= nzmax) ? ppm_tv(c, z, nzmin, nzmax) : R(0);
-    }
-    __syncwarp();
-    c.tv = tvbuf;
-  }
+__device__ __forceinline__ void column_ver_flux(const Col<R>& c, const R* fold, R* out, int nl, int nzmin, int nzmax,
+                                                R num_ord, R dt, int lane) {
   for (int iz = lane; iz < nl; iz += kWarp) {
     const int z = iz + 1;
     const R f0 = fold ? fold[iz] : R(0);
@@ -570,59 +540,59 @@ __device__ __forceinline__ void column_ver_flux(Col<R>& c, R* tvbuf, const R* fo
   __syncwarp();
 }
 
-// PPM vertical HO fluxes of KC tracer columns of one node (column_ver_flux
-// with VER = 3 for each tracer), with the geometry-only divisions of the edge
-// values and of x done once per interface instead of once per tracer: the
-// same operations on the same operands, so the results are bit-identical.
-// T, tv, fold and out hold KC columns LW apart; fold == out is allowed.
+// PPM vertical fluxes of KC tracer columns of one node (adv_tra_vert_ppm,
+// lib/oce_adv_tra_ver.F90:448-644). What the reference forms per interface is
+// formed once: the limited slope of a layer (its deltaj at one interface and
+// deltajp1 at the next are the same expression of the same operands) and, for
+// all tracers, the quotients of layer thicknesses, whose divisors repeat. T,
+// tv, fold and out hold KC columns LW apart; fold == out is allowed. tv holds
+// the slopes by layer first and is overwritten with the edge values from the
+// bottom up, each pass after the slopes it reads.
 template <typename R, int KC>
 __device__ __forceinline__ void column_ppm_multi(const Col<R>& g, const R* T, R* tv, const R* fold, R* out, int LW,
                                                  int nl, int nzmin, int nzmax, R dt, int lane) {
   const R* hnn = g.hnn;
-  for (int iz = lane; iz < nl; iz += kWarp) {
-    const int z = iz + 1;
-    if (z < nzmin || z > nzmax) {
+  for (int j = nzmin + lane; j <= nzmax - 3; j += kWarp) {  // layers (0-based) with both neighbours
+    const R dzm = hnn[j - 1], dz = hnn[j], dzp = hnn[j + 1];
+    const R sm = dzm + dz;
+    const R ga = fdiv(dz, sm + dzp);
+    const R gb = fdiv(bits64::twice(dzm) + dz, dzp + dz), gc = fdiv(dz + bits64::twice(dzp), sm);
 #pragma unroll
-      for (int i = 0; i < KC; ++i) tv[i * LW + iz] = R(0);
-      continue;
+    for (int i = 0; i < KC; ++i) {
+      const R* Ti = T + i * LW;
+      const R d1 = Ti[j + 1] - Ti[j], d0 = Ti[j] - Ti[j - 1];
+      const R del = ga * (gb * d1 + gc * d0);
+      R r = R(0);
+      if (bits64::product_positive(d1, d0))
+        r = copysign(rmin(rmin(rabs(del), rabs(bits64::twice(d1))), rabs(bits64::twice(d0))), del);
+      tv[i * LW + j] = r;
     }
+  }
+  __syncwarp();
+  for (int base = (nl - 1) / kWarp * kWarp; base >= 0; base -= kWarp) {
+    const int iz = base + lane, z = iz + 1;
+    R e[KC];
     if (z >= nzmin + 2 && z <= nzmax - 2) {
-      const int nz = z - 1;
-      const R dzjm1 = hnn[nz - 2], dzj = hnn[nz - 1], dzjp1 = hnn[nz], dzjp2 = hnn[nz + 1];
-      const R ga = fdiv(dzj, dzjm1 + dzj + dzjp1);
-      const R gb = fdiv(R(2) * dzjm1 + dzj, dzjp1 + dzj), gc = fdiv(dzj + R(2) * dzjp1, dzjm1 + dzj);
-      const R gd = fdiv(dzjp1, dzj + dzjp1 + dzjp2);
-      const R ge = fdiv(R(2) * dzj + dzjp1, dzjp2 + dzjp1), gf = fdiv(dzjp1 + R(2) * dzjp2, dzj + dzjp1);
-      const R gh = fdiv((R(2) * dzjp1) * dzj, dzj + dzjp1) *
-                   (fdiv(dzjm1 + dzj, R(2) * dzj + dzjp1) - fdiv(dzjp2 + dzjp1, R(2) * dzjp1 + dzj));
-      const R gi = fdiv(dzj * (dzjm1 + dzj), R(2) * dzj + dzjp1);
-      const R gj = fdiv(dzjp1 * (dzjp1 + dzjp2), dzj + R(2) * dzjp1);
-      const R gk = fdiv(dzj, dzj + dzjp1), gl = fdiv(R(1), dzjm1 + dzj + dzjp1 + dzjp2);
+      const R dzjm1 = hnn[iz - 2], dzj = hnn[iz - 1], dzjp1 = hnn[iz], dzjp2 = hnn[iz + 1];
+      const R su = dzjm1 + dzj, sl = dzjp2 + dzjp1;
+      const intdiv::Divisor ds = intdiv::prepare(dzj + dzjp1), du = intdiv::prepare(bits64::twice(dzj) + dzjp1),
+                            dl = intdiv::prepare(bits64::twice(dzjp1) + dzj);
+      const R gh = intdiv::divide(bits64::twice(dzjp1) * dzj, ds) * (intdiv::divide(su, du) - intdiv::divide(sl, dl));
+      const R gi = intdiv::divide(dzj * su, du), gj = intdiv::divide(dzjp1 * sl, dl);
+      const R gk = intdiv::divide(dzj, ds), gl = fdiv(R(1), su + dzjp1 + dzjp2);
 #pragma unroll
       for (int i = 0; i < KC; ++i) {
-        const R* Ti = T + i * LW;
-        const R Tm = Ti[nz - 2], T0 = Ti[nz - 1], Tp = Ti[nz], Tpp = Ti[nz + 1];
-        R deltaj = ga * (gb * (Tp - T0) + gc * (T0 - Tm));
-        R deltajp1 = gd * (ge * (Tpp - Tp) + gf * (Tp - T0));
-        if ((Tp - T0) * (T0 - Tm) > R(0))
-          deltaj = rmin(rmin(rabs(deltaj), R(2) * rabs(Tp - T0)), R(2) * rabs(T0 - Tm)) * copysign(R(1), deltaj);
-        else
-          deltaj = R(0);
-        if ((Tpp - Tp) * (Tp - T0) > R(0))
-          deltajp1 = rmin(rmin(rabs(deltajp1), R(2) * rabs(Tpp - Tp)), R(2) * rabs(Tp - T0)) * copysign(R(1), deltajp1);
-        else
-          deltajp1 = R(0);
-        const R inner1 = gh * (Tp - T0);
-        const R inner2 = gi * deltajp1;
-        const R inner3 = gj * deltaj;
-        tv[i * LW + iz] = (T0 + gk * (Tp - T0)) + gl * (inner1 - inner2 + inner3);
+        const R T0 = T[i * LW + iz - 1], d = T[i * LW + iz] - T0;
+        e[i] = (T0 + gk * d) + gl * (gh * d - gi * tv[i * LW + iz] + gj * tv[i * LW + iz - 1]);
       }
     } else {
 #pragma unroll
-      for (int i = 0; i < KC; ++i) {
-        const Col<R> ci{T + i * LW, g.W, g.area, g.hn, g.hnn, g.Z, g.zb, nullptr};
-        tv[i * LW + iz] = ppm_tv(ci, z, nzmin, nzmax);
-      }
+      for (int i = 0; i < KC; ++i) e[i] = (z < nzmin || z > nzmax) ? R(0) : ppm_tv_end(T + i * LW, g.W, z, nzmin, nzmax);
+    }
+    __syncwarp();
+    if (iz < nl) {
+#pragma unroll
+      for (int i = 0; i < KC; ++i) tv[i * LW + iz] = e[i];
     }
   }
   __syncwarp();
@@ -647,10 +617,11 @@ __device__ __forceinline__ void column_ppm_multi(const Col<R>& g, const R* T, R*
       const bool up = W > R(0);
       const int L = up ? z : z - 1;  // the layer whose parabola crosses the interface
       const R x = ppm_x(W, dt, g.hn[L - 1], up);
+      const R hx = bits64::half(x), cx = R(1) - R(2.0 / 3.0) * x;
 #pragma unroll
       for (int i = 0; i < KC; ++i)
         out[i * LW + iz] =
-            ppm_layer_x(tv[i * LW + L - 1], tv[i * LW + L], T[i * LW + L - 1], x, up, g.area[z - 1], W) - f0[i];
+            ppm_layer_x(tv[i * LW + L - 1], tv[i * LW + L], T[i * LW + L - 1], hx, cx, up, g.area[z - 1], W) - f0[i];
     } else {
 #pragma unroll
       for (int i = 0; i < KC; ++i) out[i * LW + iz] = R(0) - f0[i];
@@ -754,7 +725,7 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_lo(DMesh 
     // LO vertical flux: adv_tra_ver_upw1(we, ttf) with init zero.
     for (int i = 0; i < KC; ++i) {
       Col<R> clo{sT + i * LW, sWE, sA, sHn, sHnn, sZ, sX, nullptr};
-      column_ver_flux<R, 0>(clo, nullptr, nullptr, sFv + i * LW, nl, nzmin, nzmax, R(1), dt, lane);
+      column_ver_flux<R, 0>(clo, nullptr, sFv + i * LW, nl, nzmin, nzmax, R(1), dt, lane);
     }
     for (int p = lane; 2 * p < m.LZ; p += kWarp) {
       const int k0 = 2 * p, z0 = k0 + 1, z1 = k0 + 2;
@@ -766,18 +737,16 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_lo(DMesh 
         const Nbr q = nb.get(m, j);
         const bool a0 = z0 >= q.lo && z0 <= q.hi, a1 = z1 >= q.lo && z1 <= q.hi;
         const vec2<R> vv = ld2(a.vf + (size_t)q.e * LZ + k0);
-        const R vp0 = vv.x + rabs(vv.x), vm0 = vv.x - rabs(vv.x);
-        const R vp1 = vv.y + rabs(vv.y), vm1 = vv.y - rabs(vv.y);
 #pragma unroll
         for (int i = 0; i < KC; ++i) {
           const vec2<R> to = ld2(a.T + (t0 + i) * a.sT + (size_t)q.other * LZ + k0);
           const R tn0 = sT[i * LW + k0], tn1 = sT[i * LW + k0 + 1];
           if (q.role) {  // this node is the edge's second node
-            if (a0) acc0[i] = acc0[i] - (-(R(0.5) * (to.x * vp0 + tn0 * vm0)));
-            if (a1) acc1[i] = acc1[i] - (-(R(0.5) * (to.y * vp1 + tn1 * vm1)));
+            if (a0) acc0[i] = acc0[i] + bits64::upwind(vv.x, to.x, tn0);
+            if (a1) acc1[i] = acc1[i] + bits64::upwind(vv.y, to.y, tn1);
           } else {
-            if (a0) acc0[i] = acc0[i] + (-(R(0.5) * (tn0 * vp0 + to.x * vm0)));
-            if (a1) acc1[i] = acc1[i] + (-(R(0.5) * (tn1 * vp1 + to.y * vm1)));
+            if (a0) acc0[i] = acc0[i] - bits64::upwind(vv.x, tn0, to.x);
+            if (a1) acc1[i] = acc1[i] - bits64::upwind(vv.y, tn1, to.y);
           }
         }
       }
@@ -786,7 +755,8 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_lo(DMesh 
       const bool w0 = z0 >= nzmin && z0 <= nzmax - 1, w1 = z1 >= nzmin && z1 <= nzmax - 1;
       // fast form: dt / areasvol and 1 / hnode_new of the two layers, once
       const vec2<R> rd{rdt_vol(dt, av.x), rdt_vol(dt, av.y)};
-      const vec2<R> rh{FGB_FAST64 ? R(1) / hnn.x : R(0), FGB_FAST64 ? R(1) / hnn.y : R(0)};
+      const vec2<R> rh{FGB_FAST64 ? fdiv(R(1), hnn.x) : R(0), FGB_FAST64 ? fdiv(R(1), hnn.y) : R(0)};
+      const LayerDivisor vd0(av.x), vd1(av.y), hd0(hnn.x), hd1(hnn.y);  // exact form only
 #pragma unroll
       for (int i = 0; i < KC; ++i) {
         const R* Ti = sT + i * LW;
@@ -796,8 +766,14 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_lo(DMesh 
           if (w0) l0 = (Ti[k0] * hn.x + (acc0[i] + (Fi[k0] - Fi[k0 + 1])) * rd.x) * rh.x;
           if (w1) l1 = (Ti[k0 + 1] * hn.y + (acc1[i] + (Fi[k0 + 1] - Fi[k0 + 2])) * rd.y) * rh.y;
         } else {
-          if (w0) l0 = fdiv(Ti[k0] * hn.x + fdiv((acc0[i] + (Fi[k0] - Fi[k0 + 1])) * dt, av.x), hnn.x);
-          if (w1) l1 = fdiv(Ti[k0 + 1] * hn.y + fdiv((acc1[i] + (Fi[k0 + 1] - Fi[k0 + 2])) * dt, av.y), hnn.y);
+          if (w0) {
+            const R x = dt_per_vol(acc0[i] + (Fi[k0] - Fi[k0 + 1]), dt, vd0, R(0));
+            l0 = intdiv::divide(Ti[k0] * hn.x + x, hd0.d);
+          }
+          if (w1) {
+            const R x = dt_per_vol(acc1[i] + (Fi[k0 + 1] - Fi[k0 + 2]), dt, vd1, R(0));
+            l1 = intdiv::divide(Ti[k0 + 1] * hn.y + x, hd1.d);
+          }
         }
         st2(a.lo + (t0 + i) * a.sN + n * LZ + k0, l0, l1);
       }
@@ -808,7 +784,7 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_lo(DMesh 
       // (lib/oce_adv_tra_driver.F90:221-231)
       for (int i = 0; i < KC; ++i) {
         Col<R> clw{sT + i * LW, sW, sA, sHn, sHnn, sZ, sX, nullptr};
-        column_ver_flux<R, 0>(clw, nullptr, nullptr, sFv + i * LW, nl, nzmin, nzmax, R(1), dt, lane);
+        column_ver_flux<R, 0>(clw, nullptr, sFv + i * LW, nl, nzmin, nzmax, R(1), dt, lane);
       }
     }
     // HO vertical flux on T_AB with w; adf_v = HO - LO ("X - flux").
@@ -816,10 +792,14 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_lo(DMesh 
       const Col<R> g{nullptr, sW, sA, sHn, sHnn, sZ, sX, nullptr};
       column_ppm_multi<R, KC>(g, ta_sep ? sTA : sT, sTv, sFv, sFv, (int)LW, nl, nzmin, nzmax, dt, lane);
     }
+    if constexpr (VER == 1) {
+      qr4c_slopes<R, KC>(ta_sep ? sTA : sT, sZ, sTv, (int)LW, nzmin, nzmax, lane);
+      __syncwarp();
+    }
     for (int i = 0; i < KC; ++i) {
       if constexpr (VER != 3) {
-        Col<R> cho{(ta_sep ? sTA : sT) + i * LW, sW, sA, sHn, sHnn, sZ, sX, nullptr};
-        column_ver_flux<R, VER>(cho, sTv + i * LW, sFv + i * LW, sFv + i * LW, nl, nzmin, nzmax, a.pv, dt, lane);
+        const Col<R> cho{(ta_sep ? sTA : sT) + i * LW, sW, sA, sHn, sHnn, sZ, sX, sTv + i * LW};
+        column_ver_flux<R, VER>(cho, sFv + i * LW, sFv + i * LW, nl, nzmin, nzmax, a.pv, dt, lane);
       }
       R* __restrict__ adfv = a.adfv + (t0 + i) * a.sW + n * LW;
       for (int iz = lane; iz < (int)LW; iz += kWarp) adfv[iz] = iz < nl ? sFv[i * LW + iz] : R(0);
@@ -1102,7 +1082,7 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_update(DM
       }
       const vec2<R> hn = ld2(g.hnode + n * LZ + k0), hnn = ld2(g.hnode_new + n * LZ + k0);
       const bool w0 = z0 >= nzmin && z0 <= nzmax - 1, w1 = z1 >= nzmin && z1 <= nzmax - 1;
-      const vec2<R> rh{FGB_FAST64 ? R(1) / hnn.x : R(0), FGB_FAST64 ? R(1) / hnn.y : R(0)};
+      const vec2<R> rh{FGB_FAST64 ? fdiv(R(1), hnn.x) : R(0), FGB_FAST64 ? fdiv(R(1), hnn.y) : R(0)};
       const LayerDivisor hd0(hnn.x), hd1(hnn.y);
 #pragma unroll
       for (int i = 0; i < KC; ++i) {
@@ -1179,9 +1159,13 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_nofct_update(
       const Col<R> gc{nullptr, sW, sA, sHn, sHnn, sZ, sX, nullptr};
       column_ppm_multi<R, KC>(gc, sTA, sTv, nullptr, sF, (int)LW, nl, nzmin, nzmax, dt, lane);
     } else {
+      if constexpr (VER == 1) {
+        qr4c_slopes<R, KC>(sTA, sZ, sTv, (int)LW, nzmin, nzmax, lane);
+        __syncwarp();
+      }
       for (int i = 0; i < KC; ++i) {
-        Col<R> c{sTA + i * LW, sW, sA, sHn, sHnn, sZ, sX, nullptr};
-        column_ver_flux<R, VER>(c, sTv + i * LW, nullptr, sF + i * LW, nl, nzmin, nzmax, a.pv, dt, lane);
+        const Col<R> c{sTA + i * LW, sW, sA, sHn, sHnn, sZ, sX, sTv + i * LW};
+        column_ver_flux<R, VER>(c, nullptr, sF + i * LW, nl, nzmin, nzmax, a.pv, dt, lane);
       }
     }
     for (int p = lane; 2 * p < m.LZ; p += kWarp) {
@@ -1210,7 +1194,7 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_nofct_update(
       }
       const vec2<R> hnn = ld2(g.hnode_new + n * LZ + k0);
       const bool w0 = z0 >= nzmin && z0 <= nzmax - 1, w1 = z1 >= nzmin && z1 <= nzmax - 1;
-      const vec2<R> rh{FGB_FAST64 ? R(1) / hnn.x : R(0), FGB_FAST64 ? R(1) / hnn.y : R(0)};
+      const vec2<R> rh{FGB_FAST64 ? fdiv(R(1), hnn.x) : R(0), FGB_FAST64 ? fdiv(R(1), hnn.y) : R(0)};
       const LayerDivisor hd0(hnn.x), hd1(hnn.y);
 #pragma unroll
       for (int i = 0; i < KC; ++i) {
