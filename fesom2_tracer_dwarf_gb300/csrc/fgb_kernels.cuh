@@ -93,51 +93,85 @@ __device__ __forceinline__ R rdt_vol(R dt, R av) {
   else return R(0);  // unused by the exact form
 }
 
-// Layer membership of the horizontal-flux segments A-E of
-// lib/oce_adv_tra_hor.F90:171-252 (1-based layer z): which elements' volume
-// fluxes contribute at z. Returns 0 (inactive), 1, 2 or 3 (both).
-__device__ __forceinline__ int edge_seg(int z, int nu1, int nl1, int nu2, int nl2) {
-  const int nl12 = min(nl1, nl2), nu12 = max(nu1, nu2);
-  const bool inA = z >= nu1 && z <= nu12 - 1;
-  const bool inB = nu2 > 0 && z >= nu2 && z <= nu12 - 1;
-  const bool inC = z >= nu12 && z <= nl12;
-  const bool inD = z >= nl12 + 1 && z <= nl1;
-  const bool inE = z >= nl12 + 1 && z <= nl2;
-  return ((inA || inC || inD) ? 1 : 0) | ((inB || inC || inE) ? 2 : 0);
+// ---------------------------------------------------------------------------
+// Edges. A block of the edge kernels takes kEdgeTile edges of the visit order
+// (the three edge families interleaved by node, for cache locality); their
+// tables are staged once, then each thread takes one (edge, layer) pair at a
+// time, so that warps are full whatever the number of layers: these kernels
+// are bound by the FP64 pipe, which a warp instruction with idle lanes
+// occupies as long as a full one (one edge per warp, two layers per lane,
+// left a quarter of the lanes idle at 48 layers).
+// ---------------------------------------------------------------------------
+constexpr int kEdgeTile = 16;
+constexpr int kEdgeThreads = 256;
+
+struct EdgeTab {
+  int e, n1, n2, el1, el2, nl1, nl2;  // ulevels = 1: element 1 contributes at layers 1..nl1, element 2 at 1..nl2
+  int up, dn, gm0, gm1, nb1, nb2;
+  double dX1, dY1, dX2, dY2, ex, ey;
+};
+
+template <int HOR>
+__device__ __forceinline__ EdgeTab load_edge(const DMesh& m, int w) {
+  EdgeTab q{};
+  const int e = m.edge_order ? m.edge_order[w] : w;
+  q.e = e;
+  q.n1 = m.edge_nodes[2 * e];
+  q.n2 = m.edge_nodes[2 * e + 1];
+  q.el1 = m.edge_tri[2 * e];
+  q.el2 = m.edge_tri[2 * e + 1];
+  q.nl1 = m.edge_lev[4 * e + 1];
+  q.nl2 = q.el2 >= 0 ? m.edge_lev[4 * e + 3] : 0;
+  const double* cr = m.g64.edge_cross + 4 * (size_t)e;
+  q.dX1 = cr[0];
+  q.dY1 = cr[1];
+  q.dX2 = cr[2];
+  q.dY2 = cr[3];
+  q.gm0 = -1;
+  if (HOR != 0) {
+    q.gm0 = m.edge_gm[2 * e];
+    q.gm1 = m.edge_gm[2 * e + 1];
+    q.up = m.edge_updn[2 * e];
+    q.dn = m.edge_updn[2 * e + 1];
+    q.ex = m.g64.edge_dxa[2 * e];
+    q.ey = m.g64.edge_dxa[2 * e + 1];
+    q.nb1 = m.nbl[q.n1];
+    q.nb2 = m.nbl[q.n2];
+  }
+  return q;
+}
+
+// Volume flux through the edge's segments at layer k (vflux of
+// lib/oce_adv_tra_hor.F90:174,194,215-216).
+__device__ __forceinline__ double edge_vflux(const DMesh& m, const EdgeTab& q, const double* __restrict__ vel, int k) {
+  const bool s1 = k < q.nl1, s2 = k < q.nl2;
+  double v1 = 0.0, v2 = 0.0;
+  if (s1) {
+    const size_t i = (size_t)q.el1 * m.LZ + k;
+    const double u = vel[2 * i], w = vel[2 * i + 1];
+    v1 = (-(w * q.dX1) + u * q.dY1) * m.g64.helem[i];
+  }
+  if (s2) {
+    const size_t i = (size_t)q.el2 * m.LZ + k;
+    const double u = vel[2 * i], w = vel[2 * i + 1];
+    v2 = (w * q.dX2 - u * q.dY2) * m.g64.helem[i];
+  }
+  return s1 && s2 ? v1 + v2 : (s1 ? v1 : v2);
 }
 
 // ---------------------------------------------------------------------------
-// Volume flux through each edge segment (shared by all tracers of a step):
-// vflux of lib/oce_adv_tra_hor.F90:174,194,215-216.
+// Volume flux through each edge segment (shared by all tracers of a step),
+// for calls of single stages; a whole step forms it in the edge-flux kernel.
 // ---------------------------------------------------------------------------
 template <typename R>
-__global__ void __launch_bounds__(256) k_vflux(DMesh m, const R* __restrict__ vel, R* __restrict__ vf) {
-  const int lane = threadIdx.x & (kWarp - 1);
-  const int e = blockIdx.x * (blockDim.x / kWarp) + (threadIdx.x / kWarp);
-  if (e >= m.E) return;
-  const GeoPtrs<R>& g = GeoSel<R>::get(m);
-  const int nu1 = m.edge_lev[4 * e], nl1 = m.edge_lev[4 * e + 1];
-  const int nu2 = m.edge_lev[4 * e + 2], nl2 = m.edge_lev[4 * e + 3];
-  const int el1 = m.edge_tri[2 * e], el2 = m.edge_tri[2 * e + 1];
-  const R dX1 = g.edge_cross[4 * e], dY1 = g.edge_cross[4 * e + 1];
-  const R dX2 = g.edge_cross[4 * e + 2], dY2 = g.edge_cross[4 * e + 3];
-  const size_t LZ = m.LZ;
-  for (int k = lane; k < m.LZ; k += kWarp) {
-    R v = R(0);
-    if (k < m.nz) {
-      const int seg = edge_seg(k + 1, nu1, nl1, nu2, nl2);
-      R v1 = R(0), v2 = R(0);
-      if (seg & 1) {
-        const R u = vel[2 * (el1 * LZ + k)], vv = vel[2 * (el1 * LZ + k) + 1];
-        v1 = (-(vv * dX1) + u * dY1) * g.helem[el1 * LZ + k];
-      }
-      if (seg & 2) {
-        const R u = vel[2 * (el2 * LZ + k)], vv = vel[2 * (el2 * LZ + k) + 1];
-        v2 = (vv * dX2 - u * dY2) * g.helem[el2 * LZ + k];
-      }
-      v = (seg == 3) ? v1 + v2 : (seg == 1 ? v1 : v2);
-    }
-    vf[e * LZ + k] = v;
+__global__ void __launch_bounds__(kEdgeThreads) k_vflux(DMesh m, const R* __restrict__ vel, R* __restrict__ vf) {
+  __shared__ EdgeTab tab[kEdgeTile];
+  const int w0 = blockIdx.x * kEdgeTile, ne = min(kEdgeTile, m.E - w0);
+  if ((int)threadIdx.x < ne) tab[threadIdx.x] = load_edge<0>(m, w0 + threadIdx.x);
+  __syncthreads();
+  for (unsigned i = threadIdx.x; i < (unsigned)(ne * m.LZ); i += kEdgeThreads) {
+    const unsigned j = i / (unsigned)m.LZ, k = i - j * (unsigned)m.LZ;
+    vf[(size_t)tab[j].e * m.LZ + k] = edge_vflux(m, tab[j], vel, (int)k);
   }
 }
 
@@ -154,51 +188,62 @@ __device__ __forceinline__ void elem_grad(const DMesh& m, const GeoPtrs<R>& g, c
   gy = gs[3] * ta + gs[4] * tb + gs[5] * tc;
 }
 
-// A triangle's nodes and gradient coefficients held in registers.
+// The elemental gradients of every wet layer and tracer, (K, M, LZ) pairs: each
+// triangle is the up- or downwind one of three edges on average, which would
+// form its gradient again (ten FP64 instructions of each edge's 25 per side).
+constexpr int kElemTile = 16;
 template <typename R>
-struct Tri {
-  int a, b, c;
-  R x0, x1, x2, y0, y1, y2;
-};
-
-template <typename R>
-__device__ __forceinline__ Tri<R> load_tri(const DMesh& m, const GeoPtrs<R>& g, int el) {
-  Tri<R> q;
-  q.a = m.elem_nodes[3 * el];
-  q.b = m.elem_nodes[3 * el + 1];
-  q.c = m.elem_nodes[3 * el + 2];
-  const R* gs = g.grad_sca + 6 * (size_t)el;
-  q.x0 = gs[0]; q.x1 = gs[1]; q.x2 = gs[2];
-  q.y0 = gs[3]; q.y1 = gs[4]; q.y2 = gs[5];
-  return q;
+__global__ void __launch_bounds__(kEdgeThreads) k_elem_grad(DMesh m, StepPtrs<R> a, double2* __restrict__ out) {
+  const int w0 = blockIdx.x * kElemTile, ne = min(kElemTile, m.M - w0);
+  const size_t LZ = m.LZ;
+  for (unsigned i = threadIdx.x; i < (unsigned)(ne * m.LZ); i += kEdgeThreads) {
+    const unsigned j = i / (unsigned)m.LZ, k = i - j * (unsigned)m.LZ;
+    const int el = w0 + (int)j;
+    if ((int)k >= m.elem_nlev[el] - 1) continue;
+    const int na = m.elem_nodes[3 * el], nb = m.elem_nodes[3 * el + 1], nc = m.elem_nodes[3 * el + 2];
+    const R* gs = m.g64.grad_sca + 6 * (size_t)el;
+    const R x0 = gs[0], x1 = gs[1], x2 = gs[2], y0 = gs[3], y1 = gs[4], y2 = gs[5];
+    for (int t = 0; t < a.K; ++t) {
+      const R* __restrict__ T = a.TA + t * a.sTA + k;
+      const R ta = T[na * LZ], tb = T[nb * LZ], tc = T[nc * LZ];
+      out[((size_t)t * m.M + el) * LZ + k] = make_double2(x0 * ta + x1 * tb + x2 * tc, y0 * ta + y1 * tb + y2 * tc);
+    }
+  }
 }
 
-template <typename R>
-__device__ __forceinline__ void tri_grad(const Tri<R>& q, const R* __restrict__ T, size_t LZ, int k, R& gx, R& gy) {
-  const R ta = T[q.a * LZ + k], tb = T[q.b * LZ + k], tc = T[q.c * LZ + k];
-  gx = q.x0 * ta + q.x1 * tb + q.x2 * tc;
-  gy = q.y0 * ta + q.y1 * tb + q.y2 * tc;
+// Element gradients of one tracer: from k_elem_grad's array, or formed here.
+template <bool GRAD>
+__device__ __forceinline__ void grad_at(const DMesh& m, const double* __restrict__ T, const double2* __restrict__ G,
+                                        int el, int k, double& gx, double& gy) {
+  if constexpr (GRAD) {
+    const double2 v = G[(size_t)el * m.LZ + k];
+    gx = v.x;
+    gy = v.y;
+  } else {
+    elem_grad(m, m.g64, T, el, (size_t)k, gx, gy);
+  }
 }
 
 // Area-weighted mean of the element gradients around a node at layer z
 // (lib/oce_muscl_adv.F90:393-410).
-template <typename R>
-__device__ __forceinline__ void node_mean_grad(const DMesh& m, const GeoPtrs<R>& g, const R* __restrict__ T,
-                                               int n, int k, R& gx, R& gy) {
-  R tvol = R(0), tx = R(0), ty = R(0);
+template <bool GRAD>
+__device__ __forceinline__ void node_mean_grad(const DMesh& m, const double* __restrict__ T,
+                                               const double2* __restrict__ G, int n, int k, double& gx, double& gy) {
+  double tvol = 0.0, tx = 0.0, ty = 0.0;
   const int z = k + 1;
   for (int j = m.nie_ptr[n]; j < m.nie_ptr[n + 1]; ++j) {
     const int el = m.nie_idx[j];
     if (m.elem_nlev[el] - 1 < z) continue;
-    R ex, ey;
-    elem_grad(m, g, T, el, k, ex, ey);
-    const R ar = g.elem_area[el];
+    double ex, ey;
+    grad_at<GRAD>(m, T, G, el, k, ex, ey);
+    const double ar = m.g64.elem_area[el];
     tvol = tvol + ar;
     tx = tx + ex * ar;
     ty = ty + ey * ar;
   }
-  gx = fdiv(tx, tvol);
-  gy = fdiv(ty, tvol);
+  const intdiv::Divisor d = intdiv::prepare(tvol);
+  gx = intdiv::divide(tx, d);
+  gy = intdiv::divide(ty, d);
 }
 
 // Two consecutive layers per lane: vector loads and stores of R pairs.
@@ -247,132 +292,91 @@ __device__ __forceinline__ void st4(double* p, double a, double b, double c, dou
   *reinterpret_cast<double2*>(p + 2) = make_double2(c, d);
 }
 
-// High-order horizontal flux of one layer: upwind (adv_tra_hor_upw1,
-// lib/oce_adv_tra_hor.F90:218-220) or the MUSCL/MFCT edge reconstruction
-// (lib/oce_adv_tra_hor.F90:454-497, :748-790); c1, c2 are the c_lo masks.
-template <typename R, int HOR>
-__device__ __forceinline__ R ho_flux(R v, R vp, R vm, R ta1, R ta2, R g1, R g2, R g3, R g4, R ex, R ey, R c1, R c2,
-                                     R ph) {
-  if (HOR == 0) return -(R(0.5) * (ta1 * vp + ta2 * vm));
-  R Tm2, Tm1;
-  if (HOR == 1) {
-    Tm2 = ta2 - sixth(R(2) * (ta2 - ta1) + ex * g2 + ey * g4) * c2;
-    Tm1 = ta1 + sixth(R(2) * (ta2 - ta1) + ex * g1 + ey * g3) * c1;
-  } else {
-    Tm2 = ta2 - sixth(R(2) * (ta2 - ta1) + ex * g2 + ey * g4);
-    Tm1 = ta1 + sixth(R(2) * (ta2 - ta1) + ex * g1 + ey * g3);
-  }
-  const R cHO = vp * Tm1 + vm * Tm2;
-  return -((R(0.5) * (R(1) - ph)) * cHO) - ((v * ph) * R(0.5)) * (Tm1 + Tm2);
-}
-
 // ---------------------------------------------------------------------------
 // Horizontal edge fluxes of all K tracers. FCT: the antidiffusive flux
 // HO(T_AB) - LO(T) (adv_tra_hor_* with o_init_zero=.false. after
 // adv_tra_hor_upw1, lib/oce_adv_tra_driver.F90:95,244-255); otherwise the HO
-// flux. HOR: 0 UPW1, 1 MUSCL (with the nboundary_lay mask c_lo), 2 MFCT.
-// One warp per edge, two layers per lane. Edges are visited in edge_order
-// (the three edge families interleaved by node) for cache locality; results
-// are stored at the edge's own index.
+// flux. HOR: 0 UPW1 (lib/oce_adv_tra_hor.F90:218-220), 1 MUSCL (:454-497, with
+// the nboundary_lay mask c_lo), 2 MFCT (:748-790). VF: the volume fluxes are
+// formed and stored here (else read). GRAD: element gradients from
+// k_elem_grad's array. Results are stored at the edge's own index.
+// Bound by the FP64 pipe: 15 FP64 instructions per layer and tracer (MUSCL,
+// ph = 1; 87 in the form it replaced) and two divisions by six on the integer
+// pipe. 512^2 x 48, 2 tracers: volume fluxes, gradients and edge fluxes 4.4 ms
+// together against 10.9.
 // ---------------------------------------------------------------------------
-template <typename R, int HOR, bool FCT>
-__global__ void __launch_bounds__(256, (sizeof(R) == 4 ? 3 : 2)) k_hflux(DMesh m, StepPtrs<R> a) {
-  const int lane = threadIdx.x & (kWarp - 1);
-  const int w = blockIdx.x * (blockDim.x / kWarp) + (threadIdx.x / kWarp);
-  if (w >= m.E) return;
-  const int e = m.edge_order ? m.edge_order[w] : w;
-  const GeoPtrs<R>& g = GeoSel<R>::get(m);
+// The slow forms behind it, out of line (see bits64): the reconstruction's mask as a
+// product where a value is infinite or NaN, and the flux for any ph.
+static __device__ __noinline__ double hw_product(double a, double b) { return a * b; }
+static __device__ __noinline__ double hor_flux_any(double v, double Tm1, double Tm2, double ph) {
+  const double cHO = (v + fabs(v)) * Tm1 + (v - fabs(v)) * Tm2;
+  return -((0.5 * (1.0 - ph)) * cHO) - ((v * ph) * 0.5) * (Tm1 + Tm2);
+}
+
+template <typename R, int HOR, bool FCT, bool VF, bool GRAD>
+__global__ void __launch_bounds__(kEdgeThreads, 3) k_hflux(DMesh m, StepPtrs<R> a, const double2* __restrict__ grad) {
+  __shared__ EdgeTab tab[kEdgeTile];
+  const int w0 = blockIdx.x * kEdgeTile, ne = min(kEdgeTile, m.E - w0);
+  if ((int)threadIdx.x < ne) tab[threadIdx.x] = load_edge<HOR>(m, w0 + threadIdx.x);
+  __syncthreads();
   const size_t LZ = m.LZ;
-  const int n1 = m.edge_nodes[2 * e], n2 = m.edge_nodes[2 * e + 1];
-  const int nu1 = m.edge_lev[4 * e], nl1 = m.edge_lev[4 * e + 1];
-  const int nu2 = m.edge_lev[4 * e + 2], nl2 = m.edge_lev[4 * e + 3];
-  int gm0 = -1, gm1 = -1, nb1 = 0, nb2 = 0;
-  R ex = R(0), ey = R(0);
-  Tri<R> tu{}, td{};
-  if (HOR != 0) {
-    gm0 = m.edge_gm[2 * e];
-    gm1 = m.edge_gm[2 * e + 1];
-    ex = g.edge_dxa[2 * e];
-    ey = g.edge_dxa[2 * e + 1];
-    nb1 = m.nbl[n1];
-    nb2 = m.nbl[n2];
-    if (gm0 >= 0) {
-      tu = load_tri(m, g, m.edge_updn[2 * e]);
-      td = load_tri(m, g, m.edge_updn[2 * e + 1]);
-    }
-  }
-  const R ph = a.ph;
   const bool ta_sep = a.TA != a.T;
-  for (int p = lane; 2 * p < m.LZ; p += kWarp) {
-    const int k0 = 2 * p;
-    const int z0 = k0 + 1, z1 = k0 + 2;
-    const size_t ek = (size_t)e * LZ + k0;
-    const bool a0 = k0 < m.nz && edge_seg(z0, nu1, nl1, nu2, nl2) != 0;
-    const bool a1 = k0 + 1 < m.nz && edge_seg(z1, nu1, nl1, nu2, nl2) != 0;
-    if (!a0 && !a1) {
-      for (int t = 0; t < a.K; ++t) st2(a.adfh + t * a.sE + ek, R(0), R(0));
+  const bool ph1 = a.ph == R(1);
+  for (unsigned i = threadIdx.x; i < (unsigned)(ne * m.LZ); i += kEdgeThreads) {
+    const unsigned j = i / (unsigned)m.LZ;
+    const int k = (int)(i - j * (unsigned)m.LZ), z = k + 1;
+    const EdgeTab& q = tab[j];
+    const size_t ek = (size_t)q.e * LZ + k;
+    R v;
+    if (VF) {
+      v = edge_vflux(m, q, a.vel, k);
+      a.vf[ek] = v;
+    }
+    if (z > max(q.nl1, q.nl2)) {
+      for (int t = 0; t < a.K; ++t) a.adfh[t * a.sE + ek] = R(0);
       continue;
     }
-    const vec2<R> vv = ld2(a.vf + ek);
-    const R v0 = vv.x, v1 = vv.y;
-    const R vp0 = v0 + rabs(v0), vm0 = v0 - rabs(v0), vp1 = v1 + rabs(v1), vm1 = v1 - rabs(v1);
-    const bool tri0 = gm0 >= 0 && z0 >= gm0 && z0 <= gm1 - 1;
-    const bool tri1 = gm0 >= 0 && z1 >= gm0 && z1 <= gm1 - 1;
-    const R c10 = (nb1 - z0 >= 0) ? R(1) : R(0), c11 = (nb1 - z1 >= 0) ? R(1) : R(0);
-    const R c20 = (nb2 - z0 >= 0) ? R(1) : R(0), c21 = (nb2 - z1 >= 0) ? R(1) : R(0);
+    if (!VF) v = a.vf[ek];
+    const R B = bits64::half(ph1 ? v : v * a.ph);
+    const bool tri = q.gm0 >= 0 && z >= q.gm0 && z <= q.gm1 - 1;
+    const bool c1 = HOR == 2 || q.nb1 - z >= 0, c2 = HOR == 2 || q.nb2 - z >= 0;
+    const size_t i1 = q.n1 * LZ + k, i2 = q.n2 * LZ + k;
     for (int t = 0; t < a.K; ++t) {
       const R* __restrict__ T = a.T + t * a.sT;
       const R* __restrict__ TA = ta_sep ? a.TA + t * a.sTA : T;
-      const vec2<R> s1 = ld2(TA + n1 * LZ + k0), s2 = ld2(TA + n2 * LZ + k0);
-      R lo0 = R(0), lo1 = R(0);
-      if (FCT) {
-        const vec2<R> r1 = ta_sep ? ld2(T + n1 * LZ + k0) : s1;
-        const vec2<R> r2 = ta_sep ? ld2(T + n2 * LZ + k0) : s2;
-        lo0 = -(R(0.5) * (r1.x * vp0 + r2.x * vm0));
-        lo1 = -(R(0.5) * (r1.y * vp1 + r2.y * vm1));
-      }
-      R g10 = R(0), g20 = R(0), g30 = R(0), g40 = R(0), g11 = R(0), g21 = R(0), g31 = R(0), g41 = R(0);
-      if (HOR != 0) {
-        if (tri0 && tri1) {
-          // the upwind triangle holds node 1 and the downwind one node 2: reuse those columns
-          const vec2<R> ua = tu.a == n1 ? s1 : ld2(TA + tu.a * LZ + k0);
-          const vec2<R> ub = tu.b == n1 ? s1 : ld2(TA + tu.b * LZ + k0);
-          const vec2<R> uc = tu.c == n1 ? s1 : ld2(TA + tu.c * LZ + k0);
-          const vec2<R> da = td.a == n2 ? s2 : ld2(TA + td.a * LZ + k0);
-          const vec2<R> db = td.b == n2 ? s2 : ld2(TA + td.b * LZ + k0);
-          const vec2<R> dc = td.c == n2 ? s2 : ld2(TA + td.c * LZ + k0);
-          g10 = tu.x0 * ua.x + tu.x1 * ub.x + tu.x2 * uc.x;
-          g30 = tu.y0 * ua.x + tu.y1 * ub.x + tu.y2 * uc.x;
-          g11 = tu.x0 * ua.y + tu.x1 * ub.y + tu.x2 * uc.y;
-          g31 = tu.y0 * ua.y + tu.y1 * ub.y + tu.y2 * uc.y;
-          g20 = td.x0 * da.x + td.x1 * db.x + td.x2 * dc.x;
-          g40 = td.y0 * da.x + td.y1 * db.x + td.y2 * dc.x;
-          g21 = td.x0 * da.y + td.x1 * db.y + td.x2 * dc.y;
-          g41 = td.y0 * da.y + td.y1 * db.y + td.y2 * dc.y;
+      const R s1 = TA[i1], s2 = TA[i2];
+      R lo = R(0);  // minus the low-order flux
+      if (FCT) lo = ta_sep ? bits64::upwind(v, T[i1], T[i2]) : bits64::upwind(v, s1, s2);
+      R h;
+      if (HOR == 0) {
+        h = -(FCT && !ta_sep ? lo : bits64::upwind(v, s1, s2));
+      } else {
+        const double2* __restrict__ G = GRAD ? grad + (size_t)t * m.M * LZ : nullptr;
+        R g1, g2, g3, g4;
+        if (tri) {
+          grad_at<GRAD>(m, TA, G, q.up, k, g1, g3);
+          grad_at<GRAD>(m, TA, G, q.dn, k, g2, g4);
         } else {
-          if (a0) {
-            if (tri0) {
-              tri_grad(tu, TA, LZ, k0, g10, g30);
-              tri_grad(td, TA, LZ, k0, g20, g40);
-            } else {
-              node_mean_grad(m, g, TA, n1, k0, g10, g30);
-              node_mean_grad(m, g, TA, n2, k0, g20, g40);
-            }
-          }
-          if (a1) {
-            if (tri1) {
-              tri_grad(tu, TA, LZ, k0 + 1, g11, g31);
-              tri_grad(td, TA, LZ, k0 + 1, g21, g41);
-            } else {
-              node_mean_grad(m, g, TA, n1, k0 + 1, g11, g31);
-              node_mean_grad(m, g, TA, n2, k0 + 1, g21, g41);
-            }
+          node_mean_grad<GRAD>(m, TA, G, q.n1, k, g1, g3);
+          node_mean_grad<GRAD>(m, TA, G, q.n2, k, g2, g4);
+        }
+        const R d2 = bits64::twice(s2 - s1);
+        R r1 = sixth(d2 + q.ex * g1 + q.ey * g3), r2 = sixth(d2 + q.ex * g2 + q.ey * g4);
+        if (HOR == 1 && !(c1 && c2)) {
+          if (bits64::finite(r1, r2)) {
+            r1 = c1 ? r1 : R(0);
+            r2 = c2 ? r2 : R(0);
+          } else {
+            r1 = hw_product(r1, c1 ? R(1) : R(0));
+            r2 = hw_product(r2, c2 ? R(1) : R(0));
           }
         }
+        const R Tm1 = s1 + r1, Tm2 = s2 - r2;
+        // ph = 1: the upwind part is an exact zero (of finite values)
+        if (ph1 && bits64::finite(Tm1, Tm2) && bits64::finite(v)) h = -(B * (Tm1 + Tm2));
+        else h = hor_flux_any(v, Tm1, Tm2, a.ph);
       }
-      const R h0 = ho_flux<R, HOR>(v0, vp0, vm0, s1.x, s2.x, g10, g20, g30, g40, ex, ey, c10, c20, ph);
-      const R h1 = ho_flux<R, HOR>(v1, vp1, vm1, s1.y, s2.y, g11, g21, g31, g41, ex, ey, c11, c21, ph);
-      st2(a.adfh + t * a.sE + ek, a0 ? (FCT ? h0 - lo0 : h0) : R(0), a1 ? (FCT ? h1 - lo1 : h1) : R(0));
+      a.adfh[t * a.sE + ek] = FCT ? h + lo : h;
     }
   }
 }

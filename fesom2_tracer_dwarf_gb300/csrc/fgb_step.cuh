@@ -18,15 +18,24 @@ inline namespace fast64 {
 inline namespace exact64 {
 #endif
 
-constexpr int kEdgeWarps = 8;  // default edges per block
 constexpr int kNodeWarps = 4;  // default node columns per block (the kernels' launch bound)
 
 
+template <typename R, int HOR, bool FCT>
+void launch_hflux_as(const DMesh& m, const StepPtrs<R>& a, bool vf, const double2* grad, cudaStream_t s) {
+  const int grid = (m.E + kEdgeTile - 1) / kEdgeTile;
+  if (HOR != 0 && grad) {
+    if (vf) k_hflux<R, HOR, FCT, true, HOR != 0><<<grid, kEdgeThreads, 0, s>>>(m, a, grad);
+    else k_hflux<R, HOR, FCT, false, HOR != 0><<<grid, kEdgeThreads, 0, s>>>(m, a, grad);
+  } else {
+    if (vf) k_hflux<R, HOR, FCT, true, false><<<grid, kEdgeThreads, 0, s>>>(m, a, nullptr);
+    else k_hflux<R, HOR, FCT, false, false><<<grid, kEdgeThreads, 0, s>>>(m, a, nullptr);
+  }
+}
 template <typename R, int HOR>
-void launch_hflux(const DMesh& m, const StepPtrs<R>& a, bool fct, int ew, cudaStream_t s) {
-  dim3 grid((m.E + ew - 1) / ew), block(ew * kWarp);
-  if (fct) k_hflux<R, HOR, true><<<grid, block, 0, s>>>(m, a);
-  else k_hflux<R, HOR, false><<<grid, block, 0, s>>>(m, a);
+void launch_hflux(const DMesh& m, const StepPtrs<R>& a, bool fct, bool vf, const double2* grad, cudaStream_t s) {
+  if (fct) launch_hflux_as<R, HOR, true>(m, a, vf, grad, s);
+  else launch_hflux_as<R, HOR, false>(m, a, vf, grad, s);
 }
 
 // Dynamic shared memory above the 48 KB default needs an opt-in per kernel.
@@ -147,21 +156,32 @@ int launch_stages(const DMesh& m, const fgb_step_desc& d, int mask, cudaStream_t
   auto pick_w = [](int want, int a, int b, int c, int def) {
     return (want == a || want == b || want == c) ? want : def;
   };
-  const int ew = pick_w(d.cfg[0], 2, 4, 8, kEdgeWarps);
   const int nw_lo = pick_w(d.cfg[1], 1, 2, 4, kNodeWarps);
   const int nw_ratio = pick_w(d.cfg[2], 1, 2, 4, kNodeWarps);
   const int nw_upd = pick_w(d.cfg[3], 1, 2, 4, kNodeWarps);
   const int kc_lo = pick_kc(K, d.cfg[4]), kc_ratio = pick_kc(K, d.cfg[5]), kc_upd = pick_kc(K, d.cfg[6]);
   int launches = 0;
-  if (mask & FGB_STAGE_VFLUX) {
-    dim3 grid((m.E + kEdgeWarps - 1) / kEdgeWarps), block(kEdgeWarps * kWarp);
-    k_vflux<R><<<grid, block, 0, s>>>(m, a.vel, a.vf);
+  const bool hflux = mask & FGB_STAGE_HFLUX, vflux = mask & FGB_STAGE_VFLUX;
+  if (vflux && !hflux) {
+    k_vflux<R><<<(m.E + kEdgeTile - 1) / kEdgeTile, kEdgeThreads, 0, s>>>(m, a.vel, a.vf);
     ++launches;
   }
-  if (mask & FGB_STAGE_HFLUX) {
-    if (d.hor == FGB_HOR_UPW1) launch_hflux<R, 0>(m, a, fct, ew, s);
-    else if (d.hor == FGB_HOR_MUSCL) launch_hflux<R, 1>(m, a, fct, ew, s);
-    else launch_hflux<R, 2>(m, a, fct, ew, s);
+  if (hflux) {
+    // The element gradients of MUSCL and MFCT use the space of the LO, vertical
+    // flux and limiting-factor arrays (consecutive in the workspace), when this
+    // call writes those afterwards or no stage reads them, and they fit (two
+    // elements per node at most, as in any triangulation of the plane or torus).
+    const long long room = wl.total - wl.off[3], need = (long long)K * m.M * m.LZ * 2 * (long long)sizeof(R);
+    const int later = FGB_STAGE_LO | FGB_STAGE_RATIO;
+    double2* grad = nullptr;
+    if (d.hor != FGB_HOR_UPW1 && need <= room && (!fct || (mask & later) == later)) {
+      grad = reinterpret_cast<double2*>(ws + wl.off[3]);
+      k_elem_grad<R><<<(m.M + kElemTile - 1) / kElemTile, kEdgeThreads, 0, s>>>(m, a, grad);
+      ++launches;
+    }
+    if (d.hor == FGB_HOR_UPW1) launch_hflux<R, 0>(m, a, fct, vflux, grad, s);
+    else if (d.hor == FGB_HOR_MUSCL) launch_hflux<R, 1>(m, a, fct, vflux, grad, s);
+    else launch_hflux<R, 2>(m, a, fct, vflux, grad, s);
     ++launches;
   }
   if (fct) {

@@ -253,8 +253,8 @@ typedef struct {
   long long workspace_bytes;
   int tracer_vec; /* tracers per group of the FP32 layout: 0 or 1, 2, 4 */
   /* Launch configuration; 0 picks the default. Results do not depend on it.
-   * cfg[0]     warps (edges) per block of the edge-flux kernel: 2, 4, 8 (default 8;
-   *            FP32 form: of its per-edge kernel, see cfg[9])
+   * cfg[0]     FP32 form: warps (edges) per block of the per-edge edge-flux
+   *            kernel: 2, 4, 8 (default 8; see cfg[9])
    * cfg[1..3]  warps (node columns) per block of the LO, ratio and update
    *            kernels: 1, 2, 4 (default 4)
    * cfg[4..6]  FP64 form: tracers per chunk of the same three kernels: 1, 2,
