@@ -84,13 +84,16 @@ struct Divisor {
   int e;       // biased exponent; far out of range for divisors the integer path leaves to the hardware
 };
 
+// The divisor b with its x from an earlier prepare(b).
+FGB_HD Divisor prepared(double b, uint64_t x) {
+  const int e = (int)(to_bits(b) >> 52) & 0x7ff;
+  return Divisor{x, b, (unsigned)(e - 1) >= 2046u ? -100000 : e};
+}
+
 FGB_HD Divisor prepare(double b) {
-  Divisor d;
-  d.b = b;
-  const uint64_t bits = to_bits(b), B = significand(bits);
+  Divisor d = prepared(b, 0);
+  const uint64_t B = significand(to_bits(b));
   const uint32_t Bhi = (uint32_t)(B >> 32), Blo = (uint32_t)B;
-  d.e = (int)(bits >> 52) & 0x7ff;
-  if ((unsigned)(d.e - 1) >= 2046u) d.e = -100000;
   // x0 / 2^32 below 2^63 / B by a factor of 1 - 2^-20 .. 1 - 2^-23: the estimate of the
   // truncated significand's reciprocal (relative error 2^-23, truncation 2^-23) times 1 - 2^-21
   const uint32_t fb = 0x3f800000u | ((Bhi >> 8) & 0x7fffffu);

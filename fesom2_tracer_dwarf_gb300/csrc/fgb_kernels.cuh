@@ -1,14 +1,12 @@
-// Device kernels of the FESOM2 tracer-advection step (do_oce_adv_tra,
-// lib/oce_adv_tra_driver.F90:23-294) for GB300 (sm_103a).
+// Device kernels of the FP64 forms of the FESOM2 tracer-advection step
+// (do_oce_adv_tra, lib/oce_adv_tra_driver.F90:23-294) for GB300 (sm_103a).
 //
 // Layout: level index fastest, columns padded to LZ layers / LW interfaces.
-// Node-column kernels run one warp per node with the column staged in shared
-// memory; edge kernels run one warp per edge, lanes over layers (coalesced
-// rows) with two consecutive layers per lane. Node kernels loop over the
-// tracers of a launch KC at a time, so the mesh tables, geometry and edge
-// volume fluxes they load serve all tracers. The reference's edge scatters (atomics / OpenMP locks) are
-// replaced by gathers over each node's incident edges in ascending edge order,
-// which reproduces the reference's per-node summation order exactly.
+// Node kernels run one warp per column and deal its (tracer, layer) pairs to
+// the lanes; edge kernels deal the (edge, layer) pairs of a tile of edges to a
+// block. The reference's edge scatters (atomics / OpenMP locks) are replaced by
+// gathers over each node's incident edges in ascending edge order, which
+// reproduces the reference's per-node summation order exactly.
 //
 // R is the storage and arithmetic type. Every expression keeps the
 // reference's evaluation order; the FP64 translation unit is compiled without
@@ -246,52 +244,6 @@ __device__ __forceinline__ void node_mean_grad(const DMesh& m, const double* __r
   gy = intdiv::divide(ty, d);
 }
 
-// Two consecutive layers per lane: vector loads and stores of R pairs.
-template <typename R>
-struct V2T;
-template <>
-struct V2T<float> {
-  using T = float2;
-};
-template <>
-struct V2T<double> {
-  using T = double2;
-};
-template <typename R>
-using vec2 = typename V2T<R>::T;
-template <typename R>
-__device__ __forceinline__ vec2<R> ld2(const R* p) {
-  return *reinterpret_cast<const vec2<R>*>(p);
-}
-template <typename R>
-__device__ __forceinline__ void st2(R* p, R a, R b) {
-  vec2<R> v;
-  v.x = a;
-  v.y = b;
-  *reinterpret_cast<vec2<R>*>(p) = v;
-}
-
-// Four values per lane (two layers of an interleaved pair array).
-template <typename R>
-struct Q4 {
-  R a, b, c, d;
-};
-__device__ __forceinline__ Q4<float> ld4(const float* p) {
-  const float4 v = *reinterpret_cast<const float4*>(p);
-  return Q4<float>{v.x, v.y, v.z, v.w};
-}
-__device__ __forceinline__ Q4<double> ld4(const double* p) {
-  const double2 u = *reinterpret_cast<const double2*>(p), v = *reinterpret_cast<const double2*>(p + 2);
-  return Q4<double>{u.x, u.y, v.x, v.y};
-}
-__device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
-  *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
-}
-__device__ __forceinline__ void st4(double* p, double a, double b, double c, double d) {
-  *reinterpret_cast<double2*>(p) = make_double2(a, b);
-  *reinterpret_cast<double2*>(p + 2) = make_double2(c, d);
-}
-
 // ---------------------------------------------------------------------------
 // Horizontal edge fluxes of all K tracers. FCT: the antidiffusive flux
 // HO(T_AB) - LO(T) (adv_tra_hor_* with o_init_zero=.false. after
@@ -382,265 +334,18 @@ __global__ void __launch_bounds__(kEdgeThreads, 3) k_hflux(DMesh m, StepPtrs<R> 
 }
 
 // ---------------------------------------------------------------------------
-// Vertical fluxes of one column at interface z (1-based), given the staged
-// column. flux_old is the value the reference subtracts ("X - flux").
-// VER: 0 UPW1, 1 QR4C, 2 CDIFF, 3 PPM (lib/oce_adv_tra_ver.F90:248-712).
-// Staged arrays are 0-based by layer/interface.
-// ---------------------------------------------------------------------------
-template <typename R>
-struct Col {
-  const R* T;     // tracer at layers
-  const R* W;     // vertical velocity at interfaces
-  const R* area;  // at interfaces
-  const R* hn;    // hnode at layers (PPM)
-  const R* hnn;   // hnode_new at layers (PPM)
-  const R* Z;     // Z_3d_n at layers (QR4C)
-  const R* zb;    // zbar_3d_n at interfaces (QR4C)
-  const R* tv;    // PPM edge values at interfaces
-};
-
-template <typename R>
-__device__ __forceinline__ R ver_upw1(const Col<R>& c, int z, int nzmin, int nzmax, R fold) {
-  if (z == nzmin) return -((c.W[z - 1] * c.T[z - 1]) * c.area[z - 1]) - fold;
-  if (z == nzmax) return R(0) - fold;
-  return -(bits64::upwind(c.W[z - 1], c.T[z - 1], c.T[z - 2]) * c.area[z - 1]) - fold;
-}
-
-// QR4C: the layer-to-layer slopes (T(z-1) - T(z)) / (Z(z-1) - Z(z)) are staged in c.tv by
-// interface (qr4c_slopes): an interface uses its own and both neighbours'.
-template <typename R>
-__device__ __forceinline__ R ver_qr4c(const Col<R>& c, int z, int nzmin, int nzmax, R num_ord, R fold) {
-  const R W = c.W[z - 1];
-  if (z == nzmin) return -((c.T[z - 1] * W) * c.area[z - 1]) - fold;
-  if (z == nzmax) return R(0) - fold;
-  if (z == nzmin + 1 || z == nzmax - 1) {
-    const R x = -((bits64::half(c.T[z - 2] + c.T[z - 1]) * W) * c.area[z - 1]);
-    R f = x - fold;
-    if (nzmin + 1 == nzmax - 1) f = x - f;  // written twice (lib/oce_adv_tra_ver.F90:405-411)
-    return f;
-  }
-  const R T0 = c.T[z - 1], Tm1 = c.T[z - 2];
-  const R q2 = bits64::twice(c.tv[z - 1]), qu = c.tv[z], qd = c.tv[z - 2];
-  const R zb = c.zb[z - 1];
-  const R tm1 = T0 + third((q2 + qu) * (zb - c.Z[z - 1]));
-  const R tm2 = Tm1 + third((q2 + qd) * (zb - c.Z[z - 2]));
-  const R mean = (num_ord * bits64::half(tm1 + tm2)) * W;
-  // num_ord = 1: the upwind part is an exact zero (of finite values)
-  if (num_ord == R(1) && bits64::finite(tm1, tm2) && bits64::finite(W)) return -mean * c.area[z - 1] - fold;
-  const R tm = (W + rabs(W)) * tm1 + (W - rabs(W)) * tm2;
-  return (-((R(0.5) * (R(1) - num_ord)) * tm) - mean) * c.area[z - 1] - fold;
-}
-
-// The slopes of KC tracer columns (T, q: LW apart), the divisor of an interface prepared once.
-template <typename R, int KC>
-__device__ __forceinline__ void qr4c_slopes(const R* T, const R* Z, R* q, int LW, int nzmin, int nzmax, int lane) {
-  for (int iz = nzmin + lane; iz < nzmax - 1; iz += kWarp) {
-    const intdiv::Divisor dz = intdiv::prepare(Z[iz - 1] - Z[iz]);
-    const R rz = FGB_FAST64 ? intdiv::divide(R(1), dz) : R(0);
-#pragma unroll
-    for (int i = 0; i < KC; ++i) {
-      const R d = T[i * LW + iz - 1] - T[i * LW + iz];
-      q[i * LW + iz] = FGB_FAST64 ? d * rz : intdiv::divide(d, dz);
-    }
-  }
-}
-
-template <typename R>
-__device__ __forceinline__ R ver_cdiff(const Col<R>& c, int z, int nzmin, int nlev, R fold) {
-  const int nzmax = nlev - 1;  // lib/oce_adv_tra_ver.F90:689
-  if (z == nzmin) return -((c.W[z - 1] * c.T[z - 1]) * c.area[z - 1]) - fold;
-  if (z <= nzmax) {
-    const R tv = bits64::half(c.T[z - 2] + c.T[z - 1]);
-    return -((tv * c.W[z - 1]) * c.area[z - 1]) - fold;
-  }
-  return fold;  // the bottom interface is left untouched
-}
-
-// PPM edge value tv(z) of lib/oce_adv_tra_ver.F90:510-594 outside its
-// four-point range (column_ppm has that); the later assignment wins where the
-// special cases coincide.
-template <typename R>
-__device__ __forceinline__ R ppm_tv_end(const R* T, const R* W, int z, int nzmin, int nzmax) {
-  if (z == nzmax) return T[nzmax - 2];
-  if (z == nzmax - 1) {
-    const R Tu = T[nzmax - 3], Tl = T[nzmax - 2];
-    if (bits64::finite(Tu, Tl)) return bits64::sign_clear(W[nzmax - 2]) ? Tl : Tu;
-    const R s = copysign(R(1), W[nzmax - 2]);
-    return -(Tu * rmin(s, R(0))) + Tl * rmax(s, R(0));
-  }
-  if (z == nzmin + 1) return bits64::half(T[nzmin - 1] + T[nzmin]);
-  return T[nzmin - 1];
-}
-
-// The flux of a layer's parabola through one of its interfaces
-// (lib/oce_adv_tra_ver.F90:598-632) for x = min(|W| dt / h, 1), hx = x / 2 and
-// cx = 1 - 2/3 x of the layer.
-template <typename R>
-__device__ __forceinline__ R ppm_layer_x(R aL, R aR, R T0, R hx, R cx, bool upper, R area, R W) {
-  if (!bits64::product_positive(aR - T0, T0 - aL)) {
-    // (a NaN product is not <= 0)
-    if (bits64::finite(aR, aL) && bits64::finite(T0)) {
-      aL = T0;
-      aR = T0;
-    } else if ((aR - T0) * (T0 - aL) <= R(0)) {
-      aL = T0;
-      aR = T0;
-    }
-  }
-  R d = aR - aL, c = T0 - bits64::half(aL + aR), dc = d * c, dd = sixth(d * d);
-  if (bits64::exceeds(dc, dd)) {
-    aL = R(3) * T0 - bits64::twice(aR);
-    d = aR - aL;
-    c = T0 - bits64::half(aR + aL);
-    dc = d * c;
-    dd = sixth(d * d);
-  }
-  if (bits64::exceeds(-dd, dc)) {
-    aR = R(3) * T0 - bits64::twice(aL);
-    d = aR - aL;
-    c = T0 - bits64::half(aL + aR);
-  }
-  const R aj = R(6) * c;
-  const R tv = upper ? -aL - hx * (d + cx * aj) : -aR + hx * (d - cx * aj);
-  return (tv * area) * W;
-}
-
-// x of ppm_layer: upper side min(W dt / h, 1), lower side min(-(W dt / h), 1).
-template <typename R>
-__device__ __forceinline__ R ppm_x(R W, R dt, R dzj, bool upper) {
-  return upper ? rmin(fdiv(W * dt, dzj), R(1)) : rmin(-fdiv(W * dt, dzj), R(1));
-}
-
-template <typename R, int VER>  // not PPM: column_ppm
-__device__ __forceinline__ R ver_flux(const Col<R>& c, int z, int nzmin, int nzmax, R num_ord, R dt, R fold) {
-  if (VER == 1) return ver_qr4c(c, z, nzmin, nzmax, num_ord, fold);
-  if (VER == 2) return ver_cdiff(c, z, nzmin, nzmax, fold);
-  return ver_upw1(c, z, nzmin, nzmax, fold);
-}
-
-// Shared-memory slices of one warp's column.
-template <typename R>
-struct ColSmem {
-  R* s;
-  int LW;
-  __device__ R* slice(int i) const { return s + (size_t)i * LW; }
-};
-
-template <typename R>
-__device__ __forceinline__ void stage(R* dst, const R* __restrict__ src, int n, int lane) {
-  for (int k = lane; k < n; k += kWarp) dst[k] = src[k];
-}
-
-// Vertical flux of the column into out[iz] (interfaces) by a scheme other
-// than PPM; QR4C needs its slopes in c.tv. fold[iz] holds the value subtracted.
-template <typename R, int VER>
-__device__ __forceinline__ void column_ver_flux(const Col<R>& c, const R* fold, R* out, int nl, int nzmin, int nzmax,
-                                                R num_ord, R dt, int lane) {
-  for (int iz = lane; iz < nl; iz += kWarp) {
-    const int z = iz + 1;
-    const R f0 = fold ? fold[iz] : R(0);
-    out[iz] = (z >= nzmin && z <= nzmax) ? ver_flux<R, VER>(c, z, nzmin, nzmax, num_ord, dt, f0) : f0;
-  }
-  __syncwarp();
-}
-
-// PPM vertical fluxes of KC tracer columns of one node (adv_tra_vert_ppm,
-// lib/oce_adv_tra_ver.F90:448-644). What the reference forms per interface is
-// formed once: the limited slope of a layer (its deltaj at one interface and
-// deltajp1 at the next are the same expression of the same operands) and, for
-// all tracers, the quotients of layer thicknesses, whose divisors repeat. T,
-// tv, fold and out hold KC columns LW apart; fold == out is allowed. tv holds
-// the slopes by layer first and is overwritten with the edge values from the
-// bottom up, each pass after the slopes it reads.
-template <typename R, int KC>
-__device__ __forceinline__ void column_ppm_multi(const Col<R>& g, const R* T, R* tv, const R* fold, R* out, int LW,
-                                                 int nl, int nzmin, int nzmax, R dt, int lane) {
-  const R* hnn = g.hnn;
-  for (int j = nzmin + lane; j <= nzmax - 3; j += kWarp) {  // layers (0-based) with both neighbours
-    const R dzm = hnn[j - 1], dz = hnn[j], dzp = hnn[j + 1];
-    const R sm = dzm + dz;
-    const R ga = fdiv(dz, sm + dzp);
-    const R gb = fdiv(bits64::twice(dzm) + dz, dzp + dz), gc = fdiv(dz + bits64::twice(dzp), sm);
-#pragma unroll
-    for (int i = 0; i < KC; ++i) {
-      const R* Ti = T + i * LW;
-      const R d1 = Ti[j + 1] - Ti[j], d0 = Ti[j] - Ti[j - 1];
-      const R del = ga * (gb * d1 + gc * d0);
-      R r = R(0);
-      if (bits64::product_positive(d1, d0))
-        r = copysign(rmin(rmin(rabs(del), rabs(bits64::twice(d1))), rabs(bits64::twice(d0))), del);
-      tv[i * LW + j] = r;
-    }
-  }
-  __syncwarp();
-  for (int base = (nl - 1) / kWarp * kWarp; base >= 0; base -= kWarp) {
-    const int iz = base + lane, z = iz + 1;
-    R e[KC];
-    if (z >= nzmin + 2 && z <= nzmax - 2) {
-      const R dzjm1 = hnn[iz - 2], dzj = hnn[iz - 1], dzjp1 = hnn[iz], dzjp2 = hnn[iz + 1];
-      const R su = dzjm1 + dzj, sl = dzjp2 + dzjp1;
-      const intdiv::Divisor ds = intdiv::prepare(dzj + dzjp1), du = intdiv::prepare(bits64::twice(dzj) + dzjp1),
-                            dl = intdiv::prepare(bits64::twice(dzjp1) + dzj);
-      const R gh = intdiv::divide(bits64::twice(dzjp1) * dzj, ds) * (intdiv::divide(su, du) - intdiv::divide(sl, dl));
-      const R gi = intdiv::divide(dzj * su, du), gj = intdiv::divide(dzjp1 * sl, dl);
-      const R gk = intdiv::divide(dzj, ds), gl = fdiv(R(1), su + dzjp1 + dzjp2);
-#pragma unroll
-      for (int i = 0; i < KC; ++i) {
-        const R T0 = T[i * LW + iz - 1], d = T[i * LW + iz] - T0;
-        e[i] = (T0 + gk * d) + gl * (gh * d - gi * tv[i * LW + iz] + gj * tv[i * LW + iz - 1]);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < KC; ++i) e[i] = (z < nzmin || z > nzmax) ? R(0) : ppm_tv_end(T + i * LW, g.W, z, nzmin, nzmax);
-    }
-    __syncwarp();
-    if (iz < nl) {
-#pragma unroll
-      for (int i = 0; i < KC; ++i) tv[i * LW + iz] = e[i];
-    }
-  }
-  __syncwarp();
-  for (int iz = lane; iz < nl; iz += kWarp) {
-    const int z = iz + 1;
-    R f0[KC];
-#pragma unroll
-    for (int i = 0; i < KC; ++i) f0[i] = fold ? fold[i * LW + iz] : R(0);
-    if (z < nzmin || z > nzmax) {
-#pragma unroll
-      for (int i = 0; i < KC; ++i) out[i * LW + iz] = f0[i];
-      continue;
-    }
-    if (z == nzmin) {
-#pragma unroll
-      for (int i = 0; i < KC; ++i)
-        out[i * LW + iz] = -((tv[i * LW + nzmin - 1] * g.W[nzmin - 1]) * g.area[nzmin - 1]) - f0[i];
-      continue;
-    }
-    const R W = g.W[z - 1];
-    if (z < nzmax && W != R(0)) {
-      const bool up = W > R(0);
-      const int L = up ? z : z - 1;  // the layer whose parabola crosses the interface
-      const R x = ppm_x(W, dt, g.hn[L - 1], up);
-      const R hx = bits64::half(x), cx = R(1) - R(2.0 / 3.0) * x;
-#pragma unroll
-      for (int i = 0; i < KC; ++i)
-        out[i * LW + iz] =
-            ppm_layer_x(tv[i * LW + L - 1], tv[i * LW + L], T[i * LW + L - 1], hx, cx, up, g.area[z - 1], W) - f0[i];
-    } else {
-#pragma unroll
-      for (int i = 0; i < KC; ++i) out[i * LW + iz] = R(0) - f0[i];
-    }
-  }
-  __syncwarp();
-}
-
-// ---------------------------------------------------------------------------
-// Node-column kernels. One warp per node, two layers per lane; tracers are
-// processed KC at a time. The node's incident edges (ascending edge index,
-// the reference's scatter order) and its FCT cluster are staged once in
-// shared memory; gathers run edge-outer, tracer-inner, so every edge's
-// metadata is read once and the loads of all KC tracers are in flight
-// together. Per-(tracer, layer) summation order is the reference's.
+// Node-column kernels. One warp per node. The node's incident edges (ascending
+// edge index, the reference's scatter order) and its FCT cluster are staged
+// once in shared memory. The column's (tracer, layer) pairs of a chunk of up to
+// kc tracers are dealt to the lanes one at a time, down to the column's bottom:
+// warps are full whatever the number of layers (the kernels are bound by the
+// FP64 pipe, which a warp instruction with idle lanes occupies as long as a
+// full one), a lane holds one layer of one tracer (few registers, more warps),
+// and its chain of dependent operations is short. Per (tracer, layer) the
+// summation order is the reference's. 512^2 x 48, 2 tracers, against two layers
+// per lane and a compile-time tracer chunk: LO 1.95 / 3.34 ms, ratio 1.50 /
+// 2.07, update 1.62 / 2.64; closed 321^2 x 64, fast form: 2.17 / 2.43, 0.68 /
+// 0.76, 0.65 / 1.11; 361 columns of 9 layers, no limiter: 10 / 18 us.
 // ---------------------------------------------------------------------------
 struct Nbr {
   int e, role, other, lo, hi;
@@ -674,141 +379,330 @@ template <typename R>
 __host__ __device__ constexpr size_t warp_smem(int slices, int LW, int extra_bytes) {
   return ((size_t)slices * LW * sizeof(R) + kMaxDeg * sizeof(Nbr) + extra_bytes + 15) / 16 * 16;
 }
-__host__ __device__ constexpr int lo_slices(int KC) { return 7 + 4 * KC; }
-__host__ __device__ constexpr int ratio_slices(int KC) { return 3 * KC; }
-__host__ __device__ constexpr int upd_slices(int KC) { return 3 * KC; }
-__host__ __device__ constexpr int nofct_slices(int KC) { return 7 + 3 * KC; }
+// Columns of the vertical schemes' geometry and of one tracer's work (QR4C
+// slopes; PPM slopes and edge values).
+__host__ __device__ constexpr int ver_geo_slices(int ver) { return ver == 3 ? 10 : (ver == 1 ? 4 : 0); }
+__host__ __device__ constexpr int ver_work_slices(int ver) { return ver == 3 ? 2 : (ver == 1 ? 1 : 0); }
+__host__ __device__ constexpr int lo_slices(int ver, int kc, bool ta_sep) {
+  return ver_geo_slices(ver) + kc * (2 + (ta_sep ? 1 : 0) + ver_work_slices(ver));
+}
+__host__ __device__ constexpr int ratio_slices(int kc) { return 2 * kc; }
+__host__ __device__ constexpr int upd_slices(int kc) { return kc; }
+__host__ __device__ constexpr int nofct_slices(int ver, int kc) {
+  return ver_geo_slices(ver) + kc * (2 + ver_work_slices(ver));
+}
 constexpr int kClBytes = kMaxCl * 2 * (int)sizeof(int);
+
+// The column of one node: interfaces nzmin..nzmax (1-based), layers k0..k0+nlay-1 (0-based).
+struct Column {
+  int n, nzmin, nzmax, k0;
+  unsigned nlay;
+  size_t iz, iw;  // first layer / interface of the node in (N,LZ) / (N,LW) arrays
+  __device__ __forceinline__ Column(const DMesh& m, int n_)
+      : n(n_), nzmin(m.ulev[n_]), nzmax(m.nlev[n_]), k0(nzmin - 1), nlay((unsigned)(nzmax - nzmin)),
+        iz((size_t)n_ * m.LZ), iw((size_t)n_ * m.LW) {}
+};
+
+// ---------------------------------------------------------------------------
+// Vertical high-order fluxes (lib/oce_adv_tra_ver.F90:248-712).
+// VER: 0 UPW1, 1 QR4C, 2 CDIFF, 3 PPM.
+// ---------------------------------------------------------------------------
+// The expressions of infinite and NaN values and of any num_ord, out of line.
+static __device__ __noinline__ double qr4c_any(double W, double tm1, double tm2, double num_ord, double A) {
+  const double tm = (W + fabs(W)) * tm1 + (W - fabs(W)) * tm2;
+  return (-((0.5 * (1.0 - num_ord)) * tm) - (num_ord * (0.5 * (tm1 + tm2))) * W) * A;
+}
+static __device__ __noinline__ double hw_ppm_bottom(double Tu, double Tl, double W) {
+  const double s = copysign(1.0, W);
+  return -(Tu * (s < 0.0 ? s : 0.0)) + Tl * (s > 0.0 ? s : 0.0);
+}
+
+// What a vertical scheme needs of a column's geometry, for all its tracers.
+// PPM: the quotients of layer thicknesses, which the reference forms per tracer
+// and twice per layer (a layer's deltaj at one interface and deltajp1 at the
+// next are the same expression of the same operands), by layer (ga, gb, gc)
+// and by interface (gh..gl), and x / 2 and 1 - 2/3 x of the upwind layer.
+// QR4C: zbar - Z of both layers and the prepared divisor Z(z-1) - Z(z) (fast
+// form: its reciprocal).
+template <int VER>
+struct VerGeo {
+  double* s;
+  int LW;
+  __device__ __forceinline__ double& at(int slice, int k) const { return s[slice * LW + k]; }
+  enum { GA, GB, GC, GH, GI, GJ, GK, GL, HX, CX };  // PPM
+  enum { A1, A2, DZ, DX };                             // QR4C
+
+  __device__ __forceinline__ void form(const DMesh& m, const Column& c, const double* __restrict__ w, double dt,
+                                       int lane) const {
+    using bits64::twice;
+    const GeoPtrs<double>& g = m.g64;
+    if constexpr (VER == 1) {
+      const double* Z = g.Z3 + c.iz;
+      for (int i = c.nzmin + lane; i <= c.nzmax - 2; i += kWarp) {
+        const double zb = g.zbar3[c.iw + i], Z0 = Z[i], Zu = Z[i - 1];
+        at(A1, i) = zb - Z0;
+        at(A2, i) = zb - Zu;
+        const intdiv::Divisor d = intdiv::prepare(Zu - Z0);
+        at(DZ, i) = FGB_FAST64 ? intdiv::divide(1.0, d) : d.b;
+        at(DX, i) = bits64::from_bits(d.x);
+      }
+    }
+    if constexpr (VER == 3) {
+      const double* h = g.hnode_new + c.iz;
+      for (int j = c.nzmin + lane; j <= c.nzmax - 3; j += kWarp) {  // layers (0-based) with both neighbours
+        const double hm = h[j - 1], h0 = h[j], hp = h[j + 1], sm = hm + h0;
+        at(GA, j) = fdiv(h0, sm + hp);
+        at(GB, j) = fdiv(twice(hm) + h0, hp + h0);
+        at(GC, j) = fdiv(h0 + twice(hp), sm);
+      }
+      for (int i = c.nzmin + 1 + lane; i <= c.nzmax - 3; i += kWarp) {  // interfaces (0-based) of the four-point formula
+        const double hm = h[i - 2], h0 = h[i - 1], hp = h[i], hpp = h[i + 1], su = hm + h0, sl = hpp + hp;
+        const intdiv::Divisor ds = intdiv::prepare(h0 + hp), du = intdiv::prepare(twice(h0) + hp),
+                              dl = intdiv::prepare(twice(hp) + h0);
+        at(GH, i) = intdiv::divide(twice(hp) * h0, ds) * (intdiv::divide(su, du) - intdiv::divide(sl, dl));
+        at(GI, i) = intdiv::divide(h0 * su, du);
+        at(GJ, i) = intdiv::divide(hp * sl, dl);
+        at(GK, i) = intdiv::divide(h0, ds);
+        at(GL, i) = fdiv(1.0, su + hp + hpp);
+      }
+      for (int i = c.nzmin + lane; i <= c.nzmax - 2; i += kWarp) {
+        const double W = w[c.iw + i];  // x = min(W dt / h, 1) of the layer below (W > 0) or min(-(W dt / h), 1) above
+        const bool up = bits64::sign_clear(W);
+        const double q = fdiv(W * dt, g.hnode[c.iz + (up ? i : i - 1)]);
+        const double x = rmin(up ? q : -q, 1.0);
+        at(HX, i) = bits64::half(x);
+        at(CX, i) = 1.0 - (2.0 / 3.0) * x;
+      }
+    }
+  }
+};
+
+// Tracer work of a scheme before its fluxes: T, and the scheme's columns S
+// (and, for PPM, TV) of kc tracers, LW apart. Ends synchronised.
+template <int VER>
+__device__ __forceinline__ void ver_prepare(const VerGeo<VER>& g, const Column& c, const double* T, double* S,
+                                            double* TV, const double* __restrict__ w, unsigned kc, int lane) {
+  const int LW = g.LW;
+  if constexpr (VER == 1) {
+    // slopes (T(z-1) - T(z)) / (Z(z-1) - Z(z)) by interface: an interface uses its own and both neighbours'
+    const unsigned cnt = c.nlay - 1;
+    for (unsigned it = lane; it < kc * cnt; it += kWarp) {
+      const unsigned t = it / cnt;
+      const int i = c.nzmin + (int)(it - t * cnt);
+      const double* Ti = T + t * LW;
+      const double d = Ti[i - 1] - Ti[i];
+      if constexpr (FGB_FAST64) {
+        S[t * LW + i] = d * g.at(g.DZ, i);
+      } else {
+        S[t * LW + i] = intdiv::divide(d, intdiv::prepared(g.at(g.DZ, i), bits64::to_bits(g.at(g.DX, i))));
+      }
+    }
+    __syncwarp();
+  }
+  if constexpr (VER == 3) {
+    const int cnt = c.nzmax - 2 - c.nzmin;  // layers (0-based) nzmin..nzmax-3
+    for (int it = lane; cnt > 0 && it < (int)kc * cnt; it += kWarp) {
+      const int t = it / cnt, j = c.nzmin + it - t * cnt;
+      const double* Ti = T + t * LW;
+      const double d1 = Ti[j + 1] - Ti[j], d0 = Ti[j] - Ti[j - 1];
+      const double del = g.at(g.GA, j) * (g.at(g.GB, j) * d1 + g.at(g.GC, j) * d0);
+      double r = 0.0;
+      if (bits64::product_positive(d1, d0))
+        r = copysign(rmin(rmin(rabs(del), rabs(bits64::twice(d1))), rabs(bits64::twice(d0))), del);
+      S[t * LW + j] = r;
+    }
+    __syncwarp();
+    // edge values tv (:510-594); the later assignment wins where the special cases coincide
+    const unsigned ni = c.nlay + 1;
+    for (unsigned it = lane; it < kc * ni; it += kWarp) {
+      const unsigned t = it / ni;
+      const int i = c.k0 + (int)(it - t * ni), z = i + 1;
+      const double* Ti = T + t * LW;
+      double e;
+      if (z >= c.nzmin + 2 && z <= c.nzmax - 2) {
+        const double T0 = Ti[i - 1], d = Ti[i] - T0;
+        e = (T0 + g.at(g.GK, i) * d) +
+            g.at(g.GL, i) * (g.at(g.GH, i) * d - g.at(g.GI, i) * S[t * LW + i] + g.at(g.GJ, i) * S[t * LW + i - 1]);
+      } else if (z == c.nzmax) {
+        e = Ti[c.nzmax - 2];
+      } else if (z == c.nzmax - 1) {
+        const double Tu = Ti[c.nzmax - 3], Tl = Ti[c.nzmax - 2], W = w[c.iw + c.nzmax - 2];
+        e = bits64::finite(Tu, Tl) ? (bits64::sign_clear(W) ? Tl : Tu) : hw_ppm_bottom(Tu, Tl, W);
+      } else if (z == c.nzmin + 1) {
+        e = bits64::half(Ti[i - 1] + Ti[i]);
+      } else {
+        e = Ti[i];
+      }
+      TV[t * LW + i] = e;
+    }
+    __syncwarp();
+  }
+}
+
+// First-order upwind flux through interface i (0-based, above layer i).
+__device__ __forceinline__ double ver_upw1(const double* T, int i, int k0, double W, double A) {
+  const double T0 = T[i], Tu = i == k0 ? T0 : T[i - 1];
+  double x = bits64::upwind(W, T0, Tu);
+  if (i == k0 && !bits64::finite(T0, W)) x = hw_product(W, T0);  // the surface: W T as written
+  return -(x * A);
+}
+
+// The flux of a layer's parabola through one of its interfaces (:598-632) for
+// hx = x / 2 and cx = 1 - 2/3 x, x = min(|W| dt / h, 1).
+__device__ __forceinline__ double ppm_layer(double aL, double aR, double T0, double hx, double cx, bool upper, double A,
+                                            double W) {
+  if (!bits64::product_positive(aR - T0, T0 - aL) &&
+      ((bits64::finite(aR, aL) && bits64::finite(T0)) || hw_product(aR - T0, T0 - aL) <= 0.0)) {
+    aL = T0;
+    aR = T0;
+  }
+  double d = aR - aL, c = T0 - bits64::half(aL + aR), dc = d * c, dd = sixth(d * d);
+  if (bits64::exceeds(dc, dd)) {
+    aL = 3.0 * T0 - bits64::twice(aR);
+    d = aR - aL;
+    c = T0 - bits64::half(aR + aL);
+    dc = d * c;
+    dd = sixth(d * d);
+  }
+  if (bits64::exceeds(-dd, dc)) {
+    aR = 3.0 * T0 - bits64::twice(aL);
+    d = aR - aL;
+    c = T0 - bits64::half(aL + aR);
+  }
+  const double aj = 6.0 * c;
+  const double tv = upper ? -aL - hx * (d + cx * aj) : -aR + hx * (d - cx * aj);
+  return (tv * A) * W;
+}
+
+// High-order flux through interface i (0-based, above layer i of the column)
+// minus f0 ("X - flux"). The boundary interfaces differ in their operands only,
+// so that the lanes holding them do not make the warp run each case in turn.
+template <int VER>
+__device__ __forceinline__ double ver_flux(const VerGeo<VER>& g, const Column& c, const double* T, const double* S,
+                                           const double* TV, int i, double W, double A, double num_ord, double f0) {
+  const int z = i + 1;
+  if constexpr (VER == 0) return ver_upw1(T, i, c.k0, W, A) - f0;
+  if constexpr (VER == 1) {
+    const double T0 = T[i], Tu = i == c.k0 ? T0 : T[i - 1];
+    const bool mid = z >= c.nzmin + 2 && z <= c.nzmax - 2;
+    double x = Tu, y = T0;
+    if (mid) {
+      const double q2 = bits64::twice(S[i]);
+      y = T0 + third((q2 + S[i + 1]) * g.at(g.A1, i));
+      x = Tu + third((q2 + S[i - 1]) * g.at(g.A2, i));
+    }
+    const double mean = i == c.k0 ? T0 : bits64::half(x + y);
+    double ho = -((mean * W) * A);
+    // num_ord = 1: the upwind part is an exact zero (of finite values)
+    if (mid && !(num_ord == 1.0 && bits64::finite(x, y) && bits64::finite(W))) ho = qr4c_any(W, y, x, num_ord, A);
+    const double f = ho - f0;
+    return z == c.nzmin + 1 && z == c.nzmax - 1 ? ho - f : f;  // written twice (:405-411)
+  }
+  if constexpr (VER == 2) {
+    const double T0 = T[i];
+    return -(((i == c.k0 ? T0 : bits64::half(T[i == c.k0 ? i : i - 1] + T0)) * W) * A) - f0;
+  }
+  // PPM
+  if (i == c.k0) return -((TV[i] * W) * A) - f0;
+  if ((bits64::to_bits(W) << 1) == 0) return 0.0 - f0;
+  const bool up = bits64::sign_clear(W);
+  const int L = up ? i : i - 1;  // the layer whose parabola crosses the interface
+  return ppm_layer(TV[L], TV[L + 1], T[L], g.at(g.HX, i), g.at(g.CX, i), up, A, W) - f0;
+}
 
 // ---------------------------------------------------------------------------
 // FCT stage 1: low-order solution fct_LO (lib/oce_adv_tra_driver.F90:91-235)
 // and the vertical antidiffusive flux HO(T_AB, w) - LO(T, w_e). The low-order
 // horizontal edge fluxes are formed here from T and the edge volume fluxes,
 // with the expression adv_tra_hor_upw1 uses (lib/oce_adv_tra_hor.F90:218-220).
+// kc: tracers per chunk.
 // ---------------------------------------------------------------------------
-template <typename R, int VER, int KC>
-__global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_lo(DMesh m, StepPtrs<R> a) {
+template <typename R, int VER>
+__global__ void __launch_bounds__(128, 6) k_fct_lo(DMesh m, StepPtrs<R> a, int kc_max) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kWarp - 1), wib = threadIdx.x / kWarp;
   const int vi = blockIdx.x * (blockDim.x / kWarp) + wib;
   if (vi >= m.N) return;
-  const int n = visit_node(m, vi);
-  const GeoPtrs<R>& g = GeoSel<R>::get(m);
+  const Column c(m, visit_node(m, vi));
+  const GeoPtrs<R>& g = m.g64;
   const size_t LZ = m.LZ, LW = m.LW;
-  const int nl = m.nl, nz = m.nz;
-  unsigned char* base = smem_raw + (size_t)wib * warp_smem<R>(lo_slices(KC), m.LW, 0);
-  R* sl = reinterpret_cast<R*>(base);
-  R *sW = sl, *sWE = sl + LW, *sA = sl + 2 * LW, *sHn = sl + 3 * LW, *sHnn = sl + 4 * LW, *sX = sl + 5 * LW;
-  R* sZ = sl + 6 * LW;
-  R* sT = sl + 7 * LW;                 // KC columns
-  R* sTA = sT + (size_t)KC * LW;       // KC columns (T_AB when it is a separate field)
-  R* sFv = sTA + (size_t)KC * LW;      // KC columns of vertical fluxes
-  R* sTv = sFv + (size_t)KC * LW;      // KC columns of PPM edge values
-  const NbrList nb = stage_nbrs(m, n, reinterpret_cast<Nbr*>(base + lo_slices(KC) * LW * sizeof(R)), lane);
-  stage(sW, a.w + n * LW, nl, lane);
-  stage(sWE, a.we + n * LW, nl, lane);
-  stage(sA, g.area + n * LW, nl, lane);
-  if (VER == 3) {
-    stage(sHn, g.hnode + n * LZ, nz, lane);
-    stage(sHnn, g.hnode_new + n * LZ, nz, lane);
-  }
-  if (VER == 1) {
-    stage(sZ, g.Z3 + n * LZ, nz, lane);
-    stage(sX, g.zbar3 + n * LW, nl, lane);
-  }
-  const int nzmin = m.ulev[n], nzmax = m.nlev[n];
   const bool ta_sep = a.TA != a.T;
+  const int slices = lo_slices(VER, kc_max, ta_sep);
+  unsigned char* base = smem_raw + (size_t)wib * warp_smem<R>(slices, m.LW, 0);
+  const VerGeo<VER> geo{reinterpret_cast<R*>(base), m.LW};
+  R* sT = geo.s + ver_geo_slices(VER) * LW;
+  R* sF = sT + kc_max * LW;  // low-order vertical fluxes
+  R* sTA = ta_sep ? sF + kc_max * LW : sT;
+  R* sS = (ta_sep ? sTA : sF) + kc_max * LW;
+  R* sTV = sS + kc_max * LW;
+  const NbrList nb = stage_nbrs(m, c.n, reinterpret_cast<Nbr*>(base + slices * LW * sizeof(R)), lane);
+  geo.form(m, c, a.w, a.dt, lane);
   const R dt = a.dt;
-  for (int t0 = 0; t0 < a.K; t0 += KC) {
-#pragma unroll
-    for (int i = 0; i < KC; ++i) {
-      stage(sT + i * LW, a.T + (t0 + i) * a.sT + n * LZ, nz, lane);
-      if (ta_sep) stage(sTA + i * LW, a.TA + (t0 + i) * a.sTA + n * LZ, nz, lane);
+  for (int t0 = 0; t0 < a.K; t0 += kc_max) {
+    const unsigned kc = min(kc_max, a.K - t0), items = kc * c.nlay;
+    __syncwarp();
+    for (unsigned it = lane; it < items; it += kWarp) {
+      const unsigned t = it / c.nlay;
+      const int k = c.k0 + (int)(it - t * c.nlay);
+      sT[t * LW + k] = a.T[(t0 + t) * a.sT + c.iz + k];
+      if (ta_sep) sTA[t * LW + k] = a.TA[(t0 + t) * a.sTA + c.iz + k];
     }
     __syncwarp();
-    // LO vertical flux: adv_tra_ver_upw1(we, ttf) with init zero.
-    for (int i = 0; i < KC; ++i) {
-      Col<R> clo{sT + i * LW, sWE, sA, sHn, sHnn, sZ, sX, nullptr};
-      column_ver_flux<R, 0>(clo, nullptr, sFv + i * LW, nl, nzmin, nzmax, R(1), dt, lane);
+    // LO vertical flux: adv_tra_ver_upw1(we, ttf) with init zero
+    for (unsigned it = lane; it < items; it += kWarp) {
+      const unsigned t = it / c.nlay;
+      const int i = c.k0 + (int)(it - t * c.nlay);
+      sF[t * LW + i] = ver_upw1(sT + t * LW, i, c.k0, a.we[c.iw + i], g.area[c.iw + i]);
     }
-    for (int p = lane; 2 * p < m.LZ; p += kWarp) {
-      const int k0 = 2 * p, z0 = k0 + 1, z1 = k0 + 2;
-      R acc0[KC], acc1[KC];
-#pragma unroll
-      for (int i = 0; i < KC; ++i) acc0[i] = acc1[i] = R(0);
+    if (lane < (int)kc) sF[lane * LW + c.nzmax - 1] = R(0);
+    __syncwarp();
+    for (unsigned it = lane; it < items; it += kWarp) {
+      const unsigned t = it / c.nlay;
+      const int k = c.k0 + (int)(it - t * c.nlay), z = k + 1;
+      const R* __restrict__ T = a.T + (t0 + t) * a.sT + k;
+      const R tn = sT[t * LW + k];
+      const R hn = g.hnode[c.iz + k], hnn = g.hnode_new[c.iz + k], av = g.areasvol[c.iz + k];
+      R acc = R(0);
 #pragma unroll 2
       for (int j = 0; j < nb.deg; ++j) {
         const Nbr q = nb.get(m, j);
-        const bool a0 = z0 >= q.lo && z0 <= q.hi, a1 = z1 >= q.lo && z1 <= q.hi;
-        const vec2<R> vv = ld2(a.vf + (size_t)q.e * LZ + k0);
-#pragma unroll
-        for (int i = 0; i < KC; ++i) {
-          const vec2<R> to = ld2(a.T + (t0 + i) * a.sT + (size_t)q.other * LZ + k0);
-          const R tn0 = sT[i * LW + k0], tn1 = sT[i * LW + k0 + 1];
-          if (q.role) {  // this node is the edge's second node
-            if (a0) acc0[i] = acc0[i] + bits64::upwind(vv.x, to.x, tn0);
-            if (a1) acc1[i] = acc1[i] + bits64::upwind(vv.y, to.y, tn1);
-          } else {
-            if (a0) acc0[i] = acc0[i] - bits64::upwind(vv.x, tn0, to.x);
-            if (a1) acc1[i] = acc1[i] - bits64::upwind(vv.y, tn1, to.y);
-          }
-        }
+        if (z < q.lo || z > q.hi) continue;
+        const R v = a.vf[(size_t)q.e * LZ + k], to = T[(size_t)q.other * LZ];
+        // the second node gains what the first one loses
+        const R x = bits64::upwind(v, q.role ? to : tn, q.role ? tn : to);
+        acc = acc + bits64::negate_if(x, !q.role);
       }
-      const vec2<R> hn = ld2(g.hnode + n * LZ + k0), hnn = ld2(g.hnode_new + n * LZ + k0);
-      const vec2<R> av = ld2(g.areasvol + n * LZ + k0);
-      const bool w0 = z0 >= nzmin && z0 <= nzmax - 1, w1 = z1 >= nzmin && z1 <= nzmax - 1;
-      // fast form: dt / areasvol and 1 / hnode_new of the two layers, once
-      const vec2<R> rd{rdt_vol(dt, av.x), rdt_vol(dt, av.y)};
-      const vec2<R> rh{FGB_FAST64 ? fdiv(R(1), hnn.x) : R(0), FGB_FAST64 ? fdiv(R(1), hnn.y) : R(0)};
-      const LayerDivisor vd0(av.x), vd1(av.y), hd0(hnn.x), hd1(hnn.y);  // exact form only
-#pragma unroll
-      for (int i = 0; i < KC; ++i) {
-        const R* Ti = sT + i * LW;
-        const R* Fi = sFv + i * LW;
-        R l0 = acc0[i], l1 = acc1[i];
-        if constexpr (FGB_FAST64) {
-          if (w0) l0 = (Ti[k0] * hn.x + (acc0[i] + (Fi[k0] - Fi[k0 + 1])) * rd.x) * rh.x;
-          if (w1) l1 = (Ti[k0 + 1] * hn.y + (acc1[i] + (Fi[k0 + 1] - Fi[k0 + 2])) * rd.y) * rh.y;
-        } else {
-          if (w0) {
-            const R x = dt_per_vol(acc0[i] + (Fi[k0] - Fi[k0 + 1]), dt, vd0, R(0));
-            l0 = intdiv::divide(Ti[k0] * hn.x + x, hd0.d);
-          }
-          if (w1) {
-            const R x = dt_per_vol(acc1[i] + (Fi[k0 + 1] - Fi[k0 + 2]), dt, vd1, R(0));
-            l1 = intdiv::divide(Ti[k0 + 1] * hn.y + x, hd1.d);
-          }
-        }
-        st2(a.lo + (t0 + i) * a.sN + n * LZ + k0, l0, l1);
+      const R dF = sF[t * LW + k] - sF[t * LW + k + 1];
+      R l;
+      if constexpr (FGB_FAST64) {
+        l = (tn * hn + (acc + dF) * rdt_vol(dt, av)) * fdiv(R(1), hnn);
+      } else {
+        l = fdiv(tn * hn + fdiv((acc + dF) * dt, av), hnn);
       }
+      a.lo[(t0 + t) * a.sN + c.iz + k] = l;
     }
-    __syncwarp();  // every lane has read the LO fluxes before they are overwritten
+    for (unsigned t = 0; t < kc; ++t)  // below the bottom
+      for (int k = c.nzmax - 1 + lane; k < (int)LZ; k += kWarp) a.lo[(t0 + t) * a.sN + c.iz + k] = R(0);
     if (a.wi) {
       // w_split: the antidiffusive flux takes the upwind flux of the full w
       // (lib/oce_adv_tra_driver.F90:221-231)
-      for (int i = 0; i < KC; ++i) {
-        Col<R> clw{sT + i * LW, sW, sA, sHn, sHnn, sZ, sX, nullptr};
-        column_ver_flux<R, 0>(clw, nullptr, sFv + i * LW, nl, nzmin, nzmax, R(1), dt, lane);
+      __syncwarp();  // every lane has read the LO fluxes before they are overwritten
+      for (unsigned it = lane; it < items; it += kWarp) {
+        const unsigned t = it / c.nlay;
+        const int i = c.k0 + (int)(it - t * c.nlay);
+        sF[t * LW + i] = ver_upw1(sT + t * LW, i, c.k0, a.w[c.iw + i], g.area[c.iw + i]);
       }
     }
-    // HO vertical flux on T_AB with w; adf_v = HO - LO ("X - flux").
-    if constexpr (VER == 3) {
-      const Col<R> g{nullptr, sW, sA, sHn, sHnn, sZ, sX, nullptr};
-      column_ppm_multi<R, KC>(g, ta_sep ? sTA : sT, sTv, sFv, sFv, (int)LW, nl, nzmin, nzmax, dt, lane);
+    // HO vertical flux on T_AB with w; adf_v = HO - LO ("X - flux")
+    ver_prepare<VER>(geo, c, sTA, sS, sTV, a.w, kc, lane);
+    for (unsigned it = lane; it < items; it += kWarp) {
+      const unsigned t = it / c.nlay;
+      const int i = c.k0 + (int)(it - t * c.nlay);
+      a.adfv[(t0 + t) * a.sW + c.iw + i] = ver_flux<VER>(geo, c, sTA + t * LW, sS + t * LW, sTV + t * LW, i, a.w[c.iw + i],
+                                                         g.area[c.iw + i], a.pv, sF[t * LW + i]);
     }
-    if constexpr (VER == 1) {
-      qr4c_slopes<R, KC>(ta_sep ? sTA : sT, sZ, sTv, (int)LW, nzmin, nzmax, lane);
-      __syncwarp();
-    }
-    for (int i = 0; i < KC; ++i) {
-      if constexpr (VER != 3) {
-        const Col<R> cho{(ta_sep ? sTA : sT) + i * LW, sW, sA, sHn, sHnn, sZ, sX, sTv + i * LW};
-        column_ver_flux<R, VER>(cho, sFv + i * LW, sFv + i * LW, nl, nzmin, nzmax, a.pv, dt, lane);
-      }
-      R* __restrict__ adfv = a.adfv + (t0 + i) * a.sW + n * LW;
-      for (int iz = lane; iz < (int)LW; iz += kWarp) adfv[iz] = iz < nl ? sFv[i * LW + iz] : R(0);
-    }
-    __syncwarp();
+    for (unsigned t = 0; t < kc; ++t)  // from the bottom interface on
+      for (int i = c.nzmax - 1 + lane; i < (int)LW; i += kWarp) a.adfv[(t0 + t) * a.sW + c.iw + i] = R(0);
   }
 }
 
@@ -847,388 +741,251 @@ __device__ __forceinline__ void spread_nan(double& pos, double& neg) {
 // the cluster's elements of the maximum over their nodes; max is exact, so
 // the distinct nodes with the deepest layer reaching them give the same value.
 // ---------------------------------------------------------------------------
-template <typename R, int KC>
-__global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_ratio(DMesh m, StepPtrs<R> a) {
+template <typename R>
+__global__ void __launch_bounds__(128, 6) k_fct_ratio(DMesh m, StepPtrs<R> a, int kc_max) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kWarp - 1), wib = threadIdx.x / kWarp;
   const int vi = blockIdx.x * (blockDim.x / kWarp) + wib;
   if (vi >= m.N) return;
-  const int n = visit_node(m, vi);
-  const GeoPtrs<R>& g = GeoSel<R>::get(m);
+  const Column c(m, visit_node(m, vi));
+  const GeoPtrs<R>& g = m.g64;
   const size_t LZ = m.LZ, LW = m.LW;
-  unsigned char* base = smem_raw + (size_t)wib * warp_smem<R>(ratio_slices(KC), m.LW, kClBytes);
+  unsigned char* base = smem_raw + (size_t)wib * warp_smem<R>(ratio_slices(kc_max), m.LW, kClBytes);
   R* smax = reinterpret_cast<R*>(base);
-  R* smin = smax + (size_t)KC * LW;
-  R* sadv = smin + (size_t)KC * LW;
-  const NbrList nb = stage_nbrs(m, n, reinterpret_cast<Nbr*>(base + ratio_slices(KC) * LW * sizeof(R)), lane);
-  int* scl = reinterpret_cast<int*>(base + ratio_slices(KC) * LW * sizeof(R) + kMaxDeg * sizeof(Nbr));
-  const int c0 = m.cl_ptr[n], ncl = m.cl_ptr[n + 1] - c0, minlev = m.cl_minlev[n];
+  R* smin = smax + kc_max * LW;
+  const NbrList nb = stage_nbrs(m, c.n, reinterpret_cast<Nbr*>(base + ratio_slices(kc_max) * LW * sizeof(R)), lane);
+  int* scl = reinterpret_cast<int*>(base + ratio_slices(kc_max) * LW * sizeof(R) + kMaxDeg * sizeof(Nbr));
+  const int c0 = m.cl_ptr[c.n], ncl = m.cl_ptr[c.n + 1] - c0, minlev = m.cl_minlev[c.n];
   const bool cl_staged = ncl <= kMaxCl;
   if (cl_staged)
     for (int j = lane; j < ncl; j += kWarp) {
       scl[2 * j] = m.cl_node[c0 + j];
       scl[2 * j + 1] = m.cl_lev[c0 + j];
     }
-  const int nzmin = m.ulev[n], nzmax = m.nlev[n];
-  const R big = R(1e3), dt = a.dt;
-  const R inf = R(INFINITY);
-  for (int t0 = 0; t0 < a.K; t0 += KC) {
-#pragma unroll
-    for (int i = 0; i < KC; ++i) stage(sadv + i * LW, a.adfv + (t0 + i) * a.sW + n * LW, m.nl, lane);
+  const R dt = a.dt;
+  for (int t0 = 0; t0 < a.K; t0 += kc_max) {
+    const unsigned kc = min(kc_max, a.K - t0), items = kc * c.nlay;
     __syncwarp();
-    for (int p = lane; 2 * p < m.LZ; p += kWarp) {
-      const int k0 = 2 * p, z0 = k0 + 1, z1 = k0 + 2;
+    for (unsigned it = lane; it < items; it += kWarp) {
+      const unsigned t = it / c.nlay;
+      const int k = c.k0 + (int)(it - t * c.nlay), z = k + 1;
+      const R* __restrict__ lo = a.lo + (t0 + t) * a.sN + k;
+      const R* __restrict__ T = a.T + (t0 + t) * a.sT + k;
       // AUX = -/+1e3 of elements without the layer joins the bound (lib/oce_adv_tra_fct.F90:139-145)
-      const R mx0i = z0 > minlev ? -big : -inf, mx1i = z1 > minlev ? -big : -inf;
+      const R first = z > minlev ? R(-1e3) : R(-INFINITY);
       // the bounds as integer keys (bits64::key), which order as the values do
-      long long mx0[KC], mx1[KC], mn0[KC], mn1[KC];
-#pragma unroll
-      for (int i = 0; i < KC; ++i) {
-        mx0[i] = bits64::key(mx0i);
-        mx1[i] = bits64::key(mx1i);
-        mn0[i] = bits64::key(-mx0i);
-        mn1[i] = bits64::key(-mx1i);
-      }
+      long long mx = bits64::key(first), mn = bits64::key(-first);
 #pragma unroll 2
       for (int j = 0; j < ncl; ++j) {
         const int node = cl_staged ? scl[2 * j] : m.cl_node[c0 + j];
         const int lev = cl_staged ? scl[2 * j + 1] : m.cl_lev[c0 + j];
-        const bool a0 = z0 <= lev, a1 = z1 <= lev;
-#pragma unroll
-        for (int i = 0; i < KC; ++i) {
-          const size_t v = (size_t)node * LZ + k0;
-          const vec2<R> lv = ld2(a.lo + (t0 + i) * a.sN + v), tv = ld2(a.T + (t0 + i) * a.sT + v);
-          if (a0) join_bounds(lv.x, tv.x, mx0[i], mn0[i]);
-          if (a1) join_bounds(lv.y, tv.y, mx1[i], mn1[i]);
-        }
+        if (z <= lev) join_bounds(lo[(size_t)node * LZ], T[(size_t)node * LZ], mx, mn);
       }
+      R x = bits64::unkey(mx), y = bits64::unkey(mn);
       // A NaN is the largest or the smallest key of all, so it is still there:
-      // the column's bounds again with the floating-point comparisons, whose
-      // outcome with NaNs depends on the order.
-      bool nan = false;
-#pragma unroll
-      for (int i = 0; i < KC; ++i)
-        nan |= max(mx0[i], mx1[i]) > bits64::kKeyInf || min(mn0[i], mn1[i]) < -bits64::kKeyInf - 1;
-      if (nan) {
-        for (int i = 0; i < KC; ++i) {
-          R x0 = mx0i, x1 = mx1i, y0 = -mx0i, y1 = -mx1i;
-          for (int j = 0; j < ncl; ++j) {
-            const int lev = m.cl_lev[c0 + j];
-            const size_t v = (size_t)m.cl_node[c0 + j] * LZ + k0;
-            const vec2<R> lv = ld2(a.lo + (t0 + i) * a.sN + v), tv = ld2(a.T + (t0 + i) * a.sT + v);
-            if (z0 <= lev) {
-              x0 = rmax(x0, rmax(lv.x, tv.x));
-              y0 = rmin(y0, rmin(lv.x, tv.x));
-            }
-            if (z1 <= lev) {
-              x1 = rmax(x1, rmax(lv.y, tv.y));
-              y1 = rmin(y1, rmin(lv.y, tv.y));
-            }
-          }
-          smax[i * LW + k0] = x0;
-          smax[i * LW + k0 + 1] = x1;
-          smin[i * LW + k0] = y0;
-          smin[i * LW + k0 + 1] = y1;
+      // the bounds again with the floating-point comparisons, whose outcome
+      // with NaNs depends on the order.
+      if (mx > bits64::kKeyInf || mn < -bits64::kKeyInf - 1) {
+        x = first;
+        y = -first;
+        for (int j = 0; j < ncl; ++j) {
+          if (z > m.cl_lev[c0 + j]) continue;
+          const size_t v = (size_t)m.cl_node[c0 + j] * LZ;
+          x = rmax(x, rmax(lo[v], T[v]));
+          y = rmin(y, rmin(lo[v], T[v]));
         }
-        continue;
       }
-#pragma unroll
-      for (int i = 0; i < KC; ++i) {
-        smax[i * LW + k0] = bits64::unkey(mx0[i]);
-        smax[i * LW + k0 + 1] = bits64::unkey(mx1[i]);
-        smin[i * LW + k0] = bits64::unkey(mn0[i]);
-        smin[i * LW + k0 + 1] = bits64::unkey(mn1[i]);
-      }
+      smax[t * LW + k] = x;
+      smin[t * LW + k] = y;
     }
     __syncwarp();
-    for (int p = lane; 2 * p < m.LZ; p += kWarp) {
-      const int k0 = 2 * p;
-      R pl0[KC], pl1[KC], mi0[KC], mi1[KC];
-#pragma unroll
-      for (int i = 0; i < KC; ++i) {
-        const R* ad = sadv + i * LW;
-        first_parts(ad[k0], ad[k0 + 1], pl0[i], mi0[i]);
-        first_parts(ad[k0 + 1], ad[k0 + 2], pl1[i], mi1[i]);
-      }
-      const int z0 = k0 + 1, z1 = k0 + 2;
+    for (unsigned it = lane; it < items; it += kWarp) {
+      const unsigned t = it / c.nlay;
+      const int k = c.k0 + (int)(it - t * c.nlay), z = k + 1;
+      const R* __restrict__ adfv = a.adfv + (t0 + t) * a.sW + c.iw + k;
+      const R* __restrict__ adfh = a.adfh + (t0 + t) * a.sE + k;
+      R pl, mi;
+      first_parts(adfv[0], adfv[1], pl, mi);
 #pragma unroll 2
       for (int j = 0; j < nb.deg; ++j) {
         const Nbr q = nb.get(m, j);
-        const bool a0 = z0 >= q.lo && z0 <= q.hi, a1 = z1 >= q.lo && z1 <= q.hi;
-#pragma unroll
-        for (int i = 0; i < KC; ++i) {
-          const vec2<R> f = ld2(a.adfh + (t0 + i) * a.sE + (size_t)q.e * LZ + k0);
-          if (a0) add_part(bits64::negate_if(f.x, q.role), pl0[i], mi0[i]);
-          if (a1) add_part(bits64::negate_if(f.y, q.role), pl1[i], mi1[i]);
-        }
+        if (z >= q.lo && z <= q.hi) add_part(bits64::negate_if(adfh[(size_t)q.e * LZ], q.role), pl, mi);
       }
-      const vec2<R> av = ld2(g.areasvol + n * LZ + k0);
-      const LayerDivisor dv[2] = {LayerDivisor(av.x), LayerDivisor(av.y)};
-#pragma unroll
-      for (int i = 0; i < KC; ++i) {
-        const R* mxs = smax + i * LW;
-        const R* mns = smin + i * LW;
-        const vec2<R> lo = ld2(a.lo + (t0 + i) * a.sN + n * LZ + k0);
-        R out_p[2] = {R(0), R(0)}, out_m[2] = {R(0), R(0)};
-#pragma unroll
-        for (int l = 0; l < 2; ++l) {
-          const int k = k0 + l, z = k + 1;
-          if (z < nzmin || z > nzmax - 1) continue;
-          const R lov = l ? lo.y : lo.x;
-          R bmax, bmin;
-          if (z == nzmax - 1 || z == nzmin) {
-            bmax = mxs[k] - lov;
-            bmin = mns[k] - lov;
-          } else {
-            bmax = rmax(rmax(mxs[k - 1], mxs[k]), mxs[k + 1]) - lov;
-            bmin = rmin(rmin(mns[k - 1], mns[k]), mns[k + 1]) - lov;
-          }
-          const R avk = l ? av.y : av.x;
-          const R rdk = rdt_vol(dt, avk);
-          R pl = l ? pl1[i] : pl0[i], mi = l ? mi1[i] : mi0[i];
-          spread_nan(pl, mi);
-          R flux = dt_per_vol(pl, dt, dv[l], rdk) + R(1e-16);
-          out_p[l] = rmin(R(1), fdiv(bmax, flux));
-          flux = dt_per_vol(mi, dt, dv[l], rdk) - R(1e-16);
-          out_m[l] = rmin(R(1), fdiv(bmin, flux));
-        }
-        st4(a.rpm + 2 * ((t0 + i) * a.sN + n * LZ + k0), out_p[0], out_m[0], out_p[1], out_m[1]);
+      spread_nan(pl, mi);
+      const R lo = a.lo[(t0 + t) * a.sN + c.iz + k];
+      const R* mxs = smax + t * LW + k;
+      const R* mns = smin + t * LW + k;
+      R x = mxs[0], y = mns[0];
+      if (z != c.nzmax - 1 && z != c.nzmin) {
+        x = rmax(rmax(mxs[-1], x), mxs[1]);
+        y = rmin(rmin(mns[-1], y), mns[1]);
       }
+      const R av = g.areasvol[c.iz + k];
+      const LayerDivisor dv(av);
+      const R rd = rdt_vol(dt, av);
+      const R rp = rmin(R(1), fdiv(x - lo, dt_per_vol(pl, dt, dv, rd) + R(1e-16)));
+      const R rm = rmin(R(1), fdiv(y - lo, dt_per_vol(mi, dt, dv, rd) - R(1e-16)));
+      reinterpret_cast<double2*>(a.rpm)[(t0 + t) * a.sN + c.iz + k] = make_double2(rp, rm);
     }
-    __syncwarp();
+    for (unsigned t = 0; t < kc; ++t)  // below the bottom
+      for (int k = c.nzmax - 1 + lane; k < (int)LZ; k += kWarp)
+        reinterpret_cast<double2*>(a.rpm)[(t0 + t) * a.sN + c.iz + k] = make_double2(0.0, 0.0);
   }
+}
+
+// New value and its AB level of one layer, from the layer's tendency e.
+template <typename R>
+__device__ __forceinline__ void store_new(const StepPtrs<R>& a, int t, size_t i, R Tn, R e, R hnn) {
+  const R nv = FGB_FAST64 ? Tn + e * fdiv(R(1), hnn) : Tn + fdiv(e, hnn);
+  a.T[t * a.sT + i] = nv;
+  if (a.del) a.del[t * a.sN + i] = e;
+  if (a.TAout) a.TAout[t * a.sTA + i] = a.ab2 ? a.ab_old * Tn + a.ab_new * nv : nv;
+}
+// The AB level of the layers below a column's bottom, whose values stay.
+template <typename R>
+__device__ __forceinline__ void store_ab_below(const DMesh& m, const StepPtrs<R>& a, const Column& c, int lane) {
+  if (!a.TAout) return;
+  for (int t = 0; t < a.K; ++t)
+    for (int k = c.nzmax - 1 + lane; k < m.LZ; k += kWarp) {
+      const R Tn = a.T[t * a.sT + c.iz + k];
+      a.TAout[t * a.sTA + c.iz + k] = a.ab2 ? a.ab_old * Tn + a.ab_new * Tn : Tn;
+    }
 }
 
 // ---------------------------------------------------------------------------
 // FCT stage 3: limiting b3 (lib/oce_adv_tra_fct.F90:396-471), flux divergence
 // (oce_tra_adv_flux2dtracer with use_lo, lib/oce_adv_tra_driver.F90:298-450)
 // and the caller's tendency update (src/fesom_analytic.F90:419-437 or, with a
-// persistent del_ttf, lib/tracer_c_interface.F90:194-214).
+// persistent del_ttf, lib/tracer_c_interface.F90:194-214). The limiting
+// factors are at most 1 (or NaN), so the reference's min(1, a, b) is min(a, b).
 // ---------------------------------------------------------------------------
-template <typename R, int KC>
-__global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_fct_update(DMesh m, StepPtrs<R> a) {
+template <typename R>
+__global__ void __launch_bounds__(128, 6) k_fct_update(DMesh m, StepPtrs<R> a, int kc_max) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kWarp - 1), wib = threadIdx.x / kWarp;
   const int vi = blockIdx.x * (blockDim.x / kWarp) + wib;
   if (vi >= m.N) return;
-  const int n = visit_node(m, vi);
-  const GeoPtrs<R>& g = GeoSel<R>::get(m);
+  const Column c(m, visit_node(m, vi));
+  const GeoPtrs<R>& g = m.g64;
   const size_t LZ = m.LZ, LW = m.LW;
-  const int nz = m.nz, nl = m.nl;
-  unsigned char* base = smem_raw + (size_t)wib * warp_smem<R>(upd_slices(KC), m.LW, 0);
-  R* sLv = reinterpret_cast<R*>(base);
-  R* sRp = sLv + (size_t)KC * LW;
-  R* sRm = sRp + (size_t)KC * LW;
-  const NbrList nb = stage_nbrs(m, n, reinterpret_cast<Nbr*>(base + upd_slices(KC) * LW * sizeof(R)), lane);
-  const int nzmin = m.ulev[n], nzmax = m.nlev[n];
+  unsigned char* base = smem_raw + (size_t)wib * warp_smem<R>(upd_slices(kc_max), m.LW, 0);
+  R* sF = reinterpret_cast<R*>(base);  // limited vertical fluxes
+  const NbrList nb = stage_nbrs(m, c.n, reinterpret_cast<Nbr*>(base + upd_slices(kc_max) * LW * sizeof(R)), lane);
   const R dt = a.dt;
-  for (int t0 = 0; t0 < a.K; t0 += KC) {
-#pragma unroll
-    for (int i = 0; i < KC; ++i) {
-      const R* src = a.rpm + 2 * ((t0 + i) * a.sN + n * LZ);
-      for (int k = lane; k < nz; k += kWarp) {
-        sRp[i * LW + k] = src[2 * k];
-        sRm[i * LW + k] = src[2 * k + 1];
-      }
-    }
+  for (int t0 = 0; t0 < a.K; t0 += kc_max) {
+    const unsigned kc = min(kc_max, a.K - t0), items = kc * c.nlay;
     __syncwarp();
-#pragma unroll
-    for (int i = 0; i < KC; ++i) {
-      const R* __restrict__ adfv = a.adfv + (t0 + i) * a.sW + n * LW;
-      const R* Rp = sRp + i * LW;
-      const R* Rm = sRm + i * LW;
-      for (int iz = lane; iz < nl; iz += kWarp) {
-        const int z = iz + 1;
-        R f = adfv[iz];
-        const bool pos = bits64::sign_clear(f);
-        if (z == nzmin) f = (pos ? Rp[iz] : Rm[iz]) * f;
-        else if (z > nzmin && z <= nzmax - 1)
-          f = rmin(pos ? Rm[iz - 1] : Rp[iz - 1], pos ? Rp[iz] : Rm[iz]) * f;
-        sLv[i * LW + iz] = f;
+    for (unsigned it = lane; it < items; it += kWarp) {
+      const unsigned t = it / c.nlay;
+      const int i = c.k0 + (int)(it - t * c.nlay);
+      const double2* __restrict__ Rn = reinterpret_cast<const double2*>(a.rpm) + (t0 + t) * a.sN + c.iz + i;
+      const R f = a.adfv[(t0 + t) * a.sW + c.iw + i];
+      const bool pos = bits64::sign_clear(f);
+      const double2 own = Rn[0];
+      R ae = pos ? own.x : own.y;
+      if (i > c.k0) {
+        const double2 above = Rn[-1];
+        ae = rmin(pos ? above.y : above.x, ae);
       }
+      sF[t * LW + i] = ae * f;
     }
+    if (lane < (int)kc) sF[lane * LW + c.nzmax - 1] = a.adfv[(t0 + lane) * a.sW + c.iw + c.nzmax - 1];
     __syncwarp();
-    for (int p = lane; 2 * p < m.LZ; p += kWarp) {
-      const int k0 = 2 * p, z0 = k0 + 1, z1 = k0 + 2;
-      const vec2<R> av = ld2(g.areasvol + n * LZ + k0);
-      const vec2<R> rd{rdt_vol(dt, av.x), rdt_vol(dt, av.y)};  // fast form only
-      const LayerDivisor vd0(av.x), vd1(av.y);                   // exact form only
-      R dh0[KC], dh1[KC];
-#pragma unroll
-      for (int i = 0; i < KC; ++i) dh0[i] = dh1[i] = R(0);
+    for (unsigned it = lane; it < items; it += kWarp) {
+      const unsigned t = it / c.nlay;
+      const int k = c.k0 + (int)(it - t * c.nlay), z = k + 1;
+      const R* __restrict__ adfh = a.adfh + (t0 + t) * a.sE + k;
+      const double2* __restrict__ Rg = reinterpret_cast<const double2*>(a.rpm) + (t0 + t) * a.sN + k;
+      const double2 own = Rg[c.iz];
+      const R av = g.areasvol[c.iz + k], hn = g.hnode[c.iz + k], hnn = g.hnode_new[c.iz + k];
+      const R lo = a.lo[(t0 + t) * a.sN + c.iz + k], Tn = a.T[(t0 + t) * a.sT + c.iz + k];
+      const LayerDivisor dv(av);        // exact form only
+      const R rd = rdt_vol(dt, av);     // fast form only
+      R dh = R(0);
 #pragma unroll 2
       for (int j = 0; j < nb.deg; ++j) {
         const Nbr q = nb.get(m, j);
-        const bool a0 = z0 >= q.lo && z0 <= q.hi, a1 = z1 >= q.lo && z1 <= q.hi;
-        const size_t o = (size_t)q.other * LZ + k0;
-#pragma unroll
-        for (int i = 0; i < KC; ++i) {
-          const vec2<R> f = ld2(a.adfh + (t0 + i) * a.sE + (size_t)q.e * LZ + k0);
-          const Q4<R> ro = ld4(a.rpm + 2 * ((t0 + i) * a.sN + o));
-          const vec2<R> rpo{ro.a, ro.c}, rmo{ro.b, ro.d};
-          const R rpn0 = sRp[i * LW + k0], rpn1 = sRp[i * LW + k0 + 1];
-          const R rmn0 = sRm[i * LW + k0], rmn1 = sRm[i * LW + k0 + 1];
-          // this node's factor and the other one's, for the flux's sign; the reference takes the
-          // first node's against the second node's
-          if (a0) {
-            const bool up = bits64::sign_clear(f.x) != (bool)q.role;
-            const R own = up ? rpn0 : rmn0, oth = up ? rmo.x : rpo.x;
-            const R x = dt_per_vol((q.role ? rmin(oth, own) : rmin(own, oth)) * f.x, dt, vd0, rd.x);
-            dh0[i] = q.role ? dh0[i] - x : dh0[i] + x;
-          }
-          if (a1) {
-            const bool up = bits64::sign_clear(f.y) != (bool)q.role;
-            const R own = up ? rpn1 : rmn1, oth = up ? rmo.y : rpo.y;
-            const R x = dt_per_vol((q.role ? rmin(oth, own) : rmin(own, oth)) * f.y, dt, vd1, rd.y);
-            dh1[i] = q.role ? dh1[i] - x : dh1[i] + x;
-          }
-        }
+        if (z < q.lo || z > q.hi) continue;
+        const R f = adfh[(size_t)q.e * LZ];
+        const double2 o = Rg[(size_t)q.other * LZ];
+        // this node's factor and the other one's, for the flux's sign; the reference takes the
+        // first node's against the second node's
+        const bool up = bits64::sign_clear(f) != (bool)q.role;
+        const R mine = up ? own.x : own.y, oth = up ? o.y : o.x;
+        const R x = dt_per_vol((q.role ? rmin(oth, mine) : rmin(mine, oth)) * f, dt, dv, rd);
+        dh = dh + bits64::negate_if(x, q.role);
       }
-      const vec2<R> hn = ld2(g.hnode + n * LZ + k0), hnn = ld2(g.hnode_new + n * LZ + k0);
-      const bool w0 = z0 >= nzmin && z0 <= nzmax - 1, w1 = z1 >= nzmin && z1 <= nzmax - 1;
-      const vec2<R> rh{FGB_FAST64 ? fdiv(R(1), hnn.x) : R(0), FGB_FAST64 ? fdiv(R(1), hnn.y) : R(0)};
-      const LayerDivisor hd0(hnn.x), hd1(hnn.y);
-#pragma unroll
-      for (int i = 0; i < KC; ++i) {
-        R* __restrict__ T = a.T + (t0 + i) * a.sT + n * LZ + k0;
-        const vec2<R> Tn = ld2(T);
-        const vec2<R> lo = ld2(a.lo + (t0 + i) * a.sN + n * LZ + k0);
-        const R* Lv = sLv + i * LW;
-        R* del = a.del ? a.del + (t0 + i) * a.sN + n * LZ + k0 : nullptr;
-        const vec2<R> d0 = del ? ld2(del) : vec2<R>{R(0), R(0)};
-        R dv0 = lo.x * hnn.x - Tn.x * hn.x;  // the reference's (0 - T hnode) + LO hnode_new
-        dv0 = dv0 + dt_per_vol(Lv[k0] - Lv[k0 + 1], dt, vd0, rd.x);
-        R dv1 = lo.y * hnn.y - Tn.y * hn.y;
-        dv1 = dv1 + dt_per_vol(Lv[k0 + 1] - Lv[k0 + 2], dt, vd1, rd.y);
-        const R e0 = (del ? d0.x + dh0[i] : dh0[i]) + dv0, e1 = (del ? d0.y + dh1[i] : dh1[i]) + dv1;
-        R n0 = Tn.x, n1v = Tn.y;
-        if constexpr (FGB_FAST64) {
-          if (w0) n0 = Tn.x + e0 * rh.x;
-          if (w1) n1v = Tn.y + e1 * rh.y;
-        } else {
-          if (w0) n0 = Tn.x + intdiv::divide(e0, hd0.d);
-          if (w1) n1v = Tn.y + intdiv::divide(e1, hd1.d);
-        }
-        st2(T, n0, n1v);
-        if (del) st2(del, w0 ? e0 : d0.x, w1 ? e1 : d0.y);
-        if (a.TAout) {
-          R* ta = a.TAout + (t0 + i) * a.sTA + n * LZ + k0;
-          if (a.ab2) st2(ta, a.ab_old * Tn.x + a.ab_new * n0, a.ab_old * Tn.y + a.ab_new * n1v);
-          else st2(ta, n0, n1v);
-        }
-      }
+      // the reference's (0 - T hnode) + LO hnode_new, then the vertical flux divergence
+      R e = lo * hnn - Tn * hn;
+      e = e + dt_per_vol(sF[t * LW + k] - sF[t * LW + k + 1], dt, dv, rd);
+      if (a.del) dh = a.del[(t0 + t) * a.sN + c.iz + k] + dh;
+      store_new(a, t0 + (int)t, c.iz + k, Tn, dh + e, hnn);
     }
-    __syncwarp();
   }
+  store_ab_below(m, a, c, lane);
 }
 
 // ---------------------------------------------------------------------------
 // Without a limiter: vertical HO flux on T_AB with w_e, flux divergence
 // (oce_tra_adv_flux2dtracer) and the tendency update in one pass.
 // ---------------------------------------------------------------------------
-template <typename R, int VER, int KC>
-__global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 8 : 4)) k_nofct_update(DMesh m, StepPtrs<R> a) {
+template <typename R, int VER>
+__global__ void __launch_bounds__(128, 6) k_nofct_update(DMesh m, StepPtrs<R> a, int kc_max) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kWarp - 1), wib = threadIdx.x / kWarp;
   const int vi = blockIdx.x * (blockDim.x / kWarp) + wib;
   if (vi >= m.N) return;
-  const int n = visit_node(m, vi);
-  const GeoPtrs<R>& g = GeoSel<R>::get(m);
+  const Column c(m, visit_node(m, vi));
+  const GeoPtrs<R>& g = m.g64;
   const size_t LZ = m.LZ, LW = m.LW;
-  const int nl = m.nl, nz = m.nz;
-  unsigned char* base = smem_raw + (size_t)wib * warp_smem<R>(nofct_slices(KC), m.LW, 0);
-  R* sl = reinterpret_cast<R*>(base);
-  R *sW = sl, *sA = sl + LW, *sHn = sl + 2 * LW, *sHnn = sl + 3 * LW, *sX = sl + 4 * LW, *sZ = sl + 5 * LW;
-  R* sTA = sl + 7 * LW;              // KC columns
-  R* sF = sTA + (size_t)KC * LW;     // KC columns
-  R* sTv = sF + (size_t)KC * LW;     // KC columns
-  const NbrList nb = stage_nbrs(m, n, reinterpret_cast<Nbr*>(base + nofct_slices(KC) * LW * sizeof(R)), lane);
-  stage(sW, a.we + n * LW, nl, lane);
-  stage(sA, g.area + n * LW, nl, lane);
-  if (VER == 3) {
-    stage(sHn, g.hnode + n * LZ, nz, lane);
-    stage(sHnn, g.hnode_new + n * LZ, nz, lane);
-  }
-  if (VER == 1) {
-    stage(sZ, g.Z3 + n * LZ, nz, lane);
-    stage(sX, g.zbar3 + n * LW, nl, lane);
-  }
-  const int nzmin = m.ulev[n], nzmax = m.nlev[n];
+  const int slices = nofct_slices(VER, kc_max);
+  unsigned char* base = smem_raw + (size_t)wib * warp_smem<R>(slices, m.LW, 0);
+  const VerGeo<VER> geo{reinterpret_cast<R*>(base), m.LW};
+  R* sTA = geo.s + ver_geo_slices(VER) * LW;
+  R* sF = sTA + kc_max * LW;
+  R* sS = sF + kc_max * LW;
+  R* sTV = sS + kc_max * LW;
+  const NbrList nb = stage_nbrs(m, c.n, reinterpret_cast<Nbr*>(base + slices * LW * sizeof(R)), lane);
+  geo.form(m, c, a.we, a.dt, lane);
   const R dt = a.dt;
-  for (int t0 = 0; t0 < a.K; t0 += KC) {
-#pragma unroll
-    for (int i = 0; i < KC; ++i) stage(sTA + i * LW, a.TA + (t0 + i) * a.sTA + n * LZ, nz, lane);
+  for (int t0 = 0; t0 < a.K; t0 += kc_max) {
+    const unsigned kc = min(kc_max, a.K - t0), items = kc * c.nlay;
     __syncwarp();
-    if constexpr (VER == 3) {
-      const Col<R> gc{nullptr, sW, sA, sHn, sHnn, sZ, sX, nullptr};
-      column_ppm_multi<R, KC>(gc, sTA, sTv, nullptr, sF, (int)LW, nl, nzmin, nzmax, dt, lane);
-    } else {
-      if constexpr (VER == 1) {
-        qr4c_slopes<R, KC>(sTA, sZ, sTv, (int)LW, nzmin, nzmax, lane);
-        __syncwarp();
-      }
-      for (int i = 0; i < KC; ++i) {
-        const Col<R> c{sTA + i * LW, sW, sA, sHn, sHnn, sZ, sX, sTv + i * LW};
-        column_ver_flux<R, VER>(c, nullptr, sF + i * LW, nl, nzmin, nzmax, a.pv, dt, lane);
-      }
+    for (unsigned it = lane; it < items; it += kWarp) {
+      const unsigned t = it / c.nlay;
+      const int k = c.k0 + (int)(it - t * c.nlay);
+      sTA[t * LW + k] = a.TA[(t0 + t) * a.sTA + c.iz + k];
     }
-    for (int p = lane; 2 * p < m.LZ; p += kWarp) {
-      const int k0 = 2 * p, z0 = k0 + 1, z1 = k0 + 2;
-      const vec2<R> av = ld2(g.areasvol + n * LZ + k0);
-      const vec2<R> rd{rdt_vol(dt, av.x), rdt_vol(dt, av.y)};  // fast form only
-      const LayerDivisor vd0(av.x), vd1(av.y);                   // exact form only
-      R dh0[KC], dh1[KC];
-#pragma unroll
-      for (int i = 0; i < KC; ++i) dh0[i] = dh1[i] = R(0);
+    __syncwarp();
+    ver_prepare<VER>(geo, c, sTA, sS, sTV, a.we, kc, lane);
+    for (unsigned it = lane; it < items; it += kWarp) {
+      const unsigned t = it / c.nlay;
+      const int i = c.k0 + (int)(it - t * c.nlay);
+      sF[t * LW + i] = ver_flux<VER>(geo, c, sTA + t * LW, sS + t * LW, sTV + t * LW, i, a.we[c.iw + i], g.area[c.iw + i],
+                                     a.pv, R(0));
+    }
+    if (lane < (int)kc) sF[lane * LW + c.nzmax - 1] = R(0);
+    __syncwarp();
+    for (unsigned it = lane; it < items; it += kWarp) {
+      const unsigned t = it / c.nlay;
+      const int k = c.k0 + (int)(it - t * c.nlay), z = k + 1;
+      const R* __restrict__ flux = a.adfh + (t0 + t) * a.sE + k;
+      const R av = g.areasvol[c.iz + k], hnn = g.hnode_new[c.iz + k], Tn = a.T[(t0 + t) * a.sT + c.iz + k];
+      const LayerDivisor dv(av);     // exact form only
+      const R rd = rdt_vol(dt, av);  // fast form only
+      R dh = R(0);
 #pragma unroll 2
       for (int j = 0; j < nb.deg; ++j) {
         const Nbr q = nb.get(m, j);
-        const bool a0 = z0 >= q.lo && z0 <= q.hi, a1 = z1 >= q.lo && z1 <= q.hi;
-#pragma unroll
-        for (int i = 0; i < KC; ++i) {
-          const vec2<R> f = ld2(a.adfh + (t0 + i) * a.sE + (size_t)q.e * LZ + k0);
-          if (q.role) {
-            if (a0) dh0[i] = dh0[i] - dt_per_vol(f.x, dt, vd0, rd.x);
-            if (a1) dh1[i] = dh1[i] - dt_per_vol(f.y, dt, vd1, rd.y);
-          } else {
-            if (a0) dh0[i] = dh0[i] + dt_per_vol(f.x, dt, vd0, rd.x);
-            if (a1) dh1[i] = dh1[i] + dt_per_vol(f.y, dt, vd1, rd.y);
-          }
-        }
+        if (z < q.lo || z > q.hi) continue;
+        dh = dh + bits64::negate_if(dt_per_vol(flux[(size_t)q.e * LZ], dt, dv, rd), q.role);
       }
-      const vec2<R> hnn = ld2(g.hnode_new + n * LZ + k0);
-      const bool w0 = z0 >= nzmin && z0 <= nzmax - 1, w1 = z1 >= nzmin && z1 <= nzmax - 1;
-      const vec2<R> rh{FGB_FAST64 ? fdiv(R(1), hnn.x) : R(0), FGB_FAST64 ? fdiv(R(1), hnn.y) : R(0)};
-      const LayerDivisor hd0(hnn.x), hd1(hnn.y);
-#pragma unroll
-      for (int i = 0; i < KC; ++i) {
-        const R* F = sF + i * LW;
-        R* __restrict__ T = a.T + (t0 + i) * a.sT + n * LZ + k0;
-        const vec2<R> Tn = ld2(T);
-        R* del = a.del ? a.del + (t0 + i) * a.sN + n * LZ + k0 : nullptr;
-        const vec2<R> d0 = del ? ld2(del) : vec2<R>{R(0), R(0)};
-        const R dv0 = dt_per_vol(F[k0] - F[k0 + 1], dt, vd0, rd.x);
-        const R dv1 = dt_per_vol(F[k0 + 1] - F[k0 + 2], dt, vd1, rd.y);
-        const R e0 = (del ? d0.x + dh0[i] : dh0[i]) + dv0, e1 = (del ? d0.y + dh1[i] : dh1[i]) + dv1;
-        R n0 = Tn.x, n1v = Tn.y;
-        if constexpr (FGB_FAST64) {
-          if (w0) n0 = Tn.x + e0 * rh.x;
-          if (w1) n1v = Tn.y + e1 * rh.y;
-        } else {
-          if (w0) n0 = Tn.x + intdiv::divide(e0, hd0.d);
-          if (w1) n1v = Tn.y + intdiv::divide(e1, hd1.d);
-        }
-        st2(T, n0, n1v);
-        if (del) st2(del, w0 ? e0 : d0.x, w1 ? e1 : d0.y);
-        if (a.TAout) {
-          R* ta = a.TAout + (t0 + i) * a.sTA + n * LZ + k0;
-          if (a.ab2) st2(ta, a.ab_old * Tn.x + a.ab_new * n0, a.ab_old * Tn.y + a.ab_new * n1v);
-          else st2(ta, n0, n1v);
-        }
-      }
+      const R e = dt_per_vol(sF[t * LW + k] - sF[t * LW + k + 1], dt, dv, rd);
+      if (a.del) dh = a.del[(t0 + t) * a.sN + c.iz + k] + dh;
+      store_new(a, t0 + (int)t, c.iz + k, Tn, dh + e, hnn);
     }
-    __syncwarp();
   }
+  store_ab_below(m, a, c, lane);
 }
 
 }  // inline namespace

@@ -44,63 +44,66 @@ void allow_smem(F* kernel, size_t bytes) {
   if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-template <typename R, int VER, int KC>
-void launch_lo(const DMesh& m, const StepPtrs<R>& a, int nw, cudaStream_t s) {
-  dim3 grid((m.N + nw - 1) / nw), block(nw * kWarp);
-  const size_t sm = nw * warp_smem<R>(lo_slices(KC), m.LW, 0);
-  allow_smem(k_fct_lo<R, VER, KC>, sm);
-  k_fct_lo<R, VER, KC><<<grid, block, sm, s>>>(m, a);
+constexpr int kNodeBlocks = 6;  // the node kernels' launch bound: blocks of kNodeWarps warps
+
+// Launches a node kernel. Tracers per chunk: the requested 1, 2 or 4 if it
+// divides K, else the most (up to 4) whose shared memory leaves room for
+// kNodeBlocks blocks on an SM; the lanes share (tracer, layer) pairs, so that
+// chunk need not divide K. Columns too deep for nw of them in a block's shared
+// memory take fewer. bytes(kc): shared memory of one warp.
+template <typename F, typename R, typename B>
+void launch_nodes(F* kernel, const DMesh& m, const StepPtrs<R>& a, int nw, int want, B bytes, cudaStream_t s) {
+  int kc = a.K < 4 ? a.K : 4;
+  if ((want == 1 || want == 2 || want == 4) && a.K % want == 0) kc = want;
+  else
+    while (kc > 1 && kNodeBlocks * kNodeWarps * bytes(kc) > (size_t)220 * 1024) --kc;
+  while (nw > 1 && nw * bytes(kc) > (size_t)227 * 1024) nw /= 2;
+  const size_t sm = nw * bytes(kc);
+  allow_smem(kernel, sm);
+  kernel<<<(m.N + nw - 1) / nw, nw * kWarp, sm, s>>>(m, a, kc);
 }
 
-template <typename R, int KC>
-void launch_ratio(const DMesh& m, const StepPtrs<R>& a, int nw, cudaStream_t s) {
-  dim3 grid((m.N + nw - 1) / nw), block(nw * kWarp);
-  const size_t sm = nw * warp_smem<R>(ratio_slices(KC), m.LW, kClBytes);
-  allow_smem(k_fct_ratio<R, KC>, sm);
-  k_fct_ratio<R, KC><<<grid, block, sm, s>>>(m, a);
+template <typename R, int VER>
+void launch_lo(const DMesh& m, const StepPtrs<R>& a, int nw, int want, cudaStream_t s) {
+  launch_nodes(k_fct_lo<R, VER>, m, a, nw, want,
+               [&](int kc) { return warp_smem<R>(lo_slices(VER, kc, a.TA != a.T), m.LW, 0); }, s);
 }
 
-template <typename R, int KC>
-void launch_update(const DMesh& m, const StepPtrs<R>& a, int nw, cudaStream_t s) {
-  dim3 grid((m.N + nw - 1) / nw), block(nw * kWarp);
-  const size_t sm = nw * warp_smem<R>(upd_slices(KC), m.LW, 0);
-  allow_smem(k_fct_update<R, KC>, sm);
-  k_fct_update<R, KC><<<grid, block, sm, s>>>(m, a);
+template <typename R>
+void launch_ratio(const DMesh& m, const StepPtrs<R>& a, int nw, int want, cudaStream_t s) {
+  launch_nodes(k_fct_ratio<R>, m, a, nw, want,
+               [&](int kc) { return warp_smem<R>(ratio_slices(kc), m.LW, kClBytes); }, s);
 }
 
-template <typename R, int VER, int KC>
-void launch_nofct(const DMesh& m, const StepPtrs<R>& a, int nw, cudaStream_t s) {
-  dim3 grid((m.N + nw - 1) / nw), block(nw * kWarp);
-  const size_t sm = nw * warp_smem<R>(nofct_slices(KC), m.LW, 0);
-  allow_smem(k_nofct_update<R, VER, KC>, sm);
-  k_nofct_update<R, VER, KC><<<grid, block, sm, s>>>(m, a);
+template <typename R>
+void launch_update(const DMesh& m, const StepPtrs<R>& a, int nw, int want, cudaStream_t s) {
+  launch_nodes(k_fct_update<R>, m, a, nw, want, [&](int kc) { return warp_smem<R>(upd_slices(kc), m.LW, 0); }, s);
 }
 
-template <typename R, int KC>
-void launch_lo_ver(const DMesh& m, const StepPtrs<R>& a, int ver, int nw, cudaStream_t s) {
+template <typename R, int VER>
+void launch_nofct(const DMesh& m, const StepPtrs<R>& a, int nw, int want, cudaStream_t s) {
+  launch_nodes(k_nofct_update<R, VER>, m, a, nw, want,
+               [&](int kc) { return warp_smem<R>(nofct_slices(VER, kc), m.LW, 0); }, s);
+}
+
+template <typename R>
+void launch_lo_ver(const DMesh& m, const StepPtrs<R>& a, int ver, int nw, int want, cudaStream_t s) {
   switch (ver) {
-    case FGB_VER_QR4C: launch_lo<R, 1, KC>(m, a, nw, s); break;
-    case FGB_VER_CDIFF: launch_lo<R, 2, KC>(m, a, nw, s); break;
-    case FGB_VER_PPM: launch_lo<R, 3, KC>(m, a, nw, s); break;
-    default: launch_lo<R, 0, KC>(m, a, nw, s); break;
+    case FGB_VER_QR4C: launch_lo<R, 1>(m, a, nw, want, s); break;
+    case FGB_VER_CDIFF: launch_lo<R, 2>(m, a, nw, want, s); break;
+    case FGB_VER_PPM: launch_lo<R, 3>(m, a, nw, want, s); break;
+    default: launch_lo<R, 0>(m, a, nw, want, s); break;
   }
 }
 
-template <typename R, int KC>
-void launch_nofct_ver(const DMesh& m, const StepPtrs<R>& a, int ver, int nw, cudaStream_t s) {
+template <typename R>
+void launch_nofct_ver(const DMesh& m, const StepPtrs<R>& a, int ver, int nw, int want, cudaStream_t s) {
   switch (ver) {
-    case FGB_VER_QR4C: launch_nofct<R, 1, KC>(m, a, nw, s); break;
-    case FGB_VER_CDIFF: launch_nofct<R, 2, KC>(m, a, nw, s); break;
-    case FGB_VER_PPM: launch_nofct<R, 3, KC>(m, a, nw, s); break;
-    default: launch_nofct<R, 0, KC>(m, a, nw, s); break;
+    case FGB_VER_QR4C: launch_nofct<R, 1>(m, a, nw, want, s); break;
+    case FGB_VER_CDIFF: launch_nofct<R, 2>(m, a, nw, want, s); break;
+    case FGB_VER_PPM: launch_nofct<R, 3>(m, a, nw, want, s); break;
+    default: launch_nofct<R, 0>(m, a, nw, want, s); break;
   }
-}
-
-// Tracers per node-kernel chunk: the requested value if it divides K, else the
-// largest of 4, 2, 1 that does.
-inline int pick_kc(int K, int want) {
-  if ((want == 1 || want == 2 || want == 4) && K % want == 0) return want;
-  return (K % 4 == 0) ? 4 : ((K % 2 == 0) ? 2 : 1);
 }
 
 template <typename R>
@@ -159,7 +162,6 @@ int launch_stages(const DMesh& m, const fgb_step_desc& d, int mask, cudaStream_t
   const int nw_lo = pick_w(d.cfg[1], 1, 2, 4, kNodeWarps);
   const int nw_ratio = pick_w(d.cfg[2], 1, 2, 4, kNodeWarps);
   const int nw_upd = pick_w(d.cfg[3], 1, 2, 4, kNodeWarps);
-  const int kc_lo = pick_kc(K, d.cfg[4]), kc_ratio = pick_kc(K, d.cfg[5]), kc_upd = pick_kc(K, d.cfg[6]);
   int launches = 0;
   const bool hflux = mask & FGB_STAGE_HFLUX, vflux = mask & FGB_STAGE_VFLUX;
   if (vflux && !hflux) {
@@ -186,9 +188,7 @@ int launch_stages(const DMesh& m, const fgb_step_desc& d, int mask, cudaStream_t
   }
   if (fct) {
     if (mask & FGB_STAGE_LO) {
-      if (kc_lo == 4) launch_lo_ver<R, 4>(m, a, d.ver, nw_lo, s);
-      else if (kc_lo == 2) launch_lo_ver<R, 2>(m, a, d.ver, nw_lo, s);
-      else launch_lo_ver<R, 1>(m, a, d.ver, nw_lo, s);
+      launch_lo_ver<R>(m, a, d.ver, nw_lo, d.cfg[4], s);
       ++launches;
       if (wsplit) {
         launch_vert_impl<R>(m, GeoSel<R>::get(m), a.lo, a.wi, K, 1, a.sN, a.dt, s);
@@ -196,21 +196,15 @@ int launch_stages(const DMesh& m, const fgb_step_desc& d, int mask, cudaStream_t
       }
     }
     if (mask & FGB_STAGE_RATIO) {
-      if (kc_ratio == 4) launch_ratio<R, 4>(m, a, nw_ratio, s);
-      else if (kc_ratio == 2) launch_ratio<R, 2>(m, a, nw_ratio, s);
-      else launch_ratio<R, 1>(m, a, nw_ratio, s);
+      launch_ratio<R>(m, a, nw_ratio, d.cfg[5], s);
       ++launches;
     }
     if (mask & FGB_STAGE_UPDATE) {
-      if (kc_upd == 4) launch_update<R, 4>(m, a, nw_upd, s);
-      else if (kc_upd == 2) launch_update<R, 2>(m, a, nw_upd, s);
-      else launch_update<R, 1>(m, a, nw_upd, s);
+      launch_update<R>(m, a, nw_upd, d.cfg[6], s);
       ++launches;
     }
   } else if (mask & FGB_STAGE_UPDATE) {
-    if (kc_upd == 4) launch_nofct_ver<R, 4>(m, a, d.ver, nw_upd, s);
-    else if (kc_upd == 2) launch_nofct_ver<R, 2>(m, a, d.ver, nw_upd, s);
-    else launch_nofct_ver<R, 1>(m, a, d.ver, nw_upd, s);
+    launch_nofct_ver<R>(m, a, d.ver, nw_upd, d.cfg[6], s);
     ++launches;
   }
   *nlaunch = launches;
