@@ -127,7 +127,7 @@ int launch_stages(const DMesh& m, const fgb_step_desc& d, int mask, cudaStream_t
   const bool fct = d.lim == FGB_LIM_FCT;
   const bool wsplit = fct && d.wi;
   if (wsplit) {
-    if (const char* why = vert_impl_check<R>(m)) { *err = why; return -1; }
+    if (const char* why = vert_impl_check(m)) { *err = why; return -1; }
   }
   char* ws = static_cast<char*>(d.workspace);
   StepPtrs<R> a;
@@ -191,7 +191,7 @@ int launch_stages(const DMesh& m, const fgb_step_desc& d, int mask, cudaStream_t
       launch_lo_ver<R>(m, a, d.ver, nw_lo, d.cfg[4], s);
       ++launches;
       if (wsplit) {
-        launch_vert_impl<R>(m, GeoSel<R>::get(m), a.lo, a.wi, K, 1, a.sN, a.dt, s);
+        launch_vert_impl<R>(m, a.lo, a.wi, K, a.sN, a.dt, s);
         ++launches;
       }
     }
