@@ -265,71 +265,123 @@ static __device__ __noinline__ double hor_flux_any(double v, double Tm1, double 
   return -((0.5 * (1.0 - ph)) * cHO) - ((v * ph) * 0.5) * (Tm1 + Tm2);
 }
 
+// The flux of edge q at layer k, all tracers. MEAN: outside the triangles' window (or without
+// triangles), the mean gradients around both nodes.
+template <int HOR, bool FCT, bool VF, bool GRAD, bool MEAN>
+__device__ __forceinline__ void hor_flux(const DMesh& m, const StepPtrs<double>& a, const double2* __restrict__ grad,
+                                         const EdgeTab& q, int k) {
+  const size_t LZ = m.LZ, ek = (size_t)q.e * LZ + k;
+  const bool ta_sep = a.TA != a.T, ph1 = a.ph == 1.0;
+  double v;
+  if (VF) {
+    v = edge_vflux(m, q, a.vel, k);
+    a.vf[ek] = v;
+  } else {
+    v = a.vf[ek];
+  }
+  const double B = bits64::half(ph1 ? v : v * a.ph);
+  const bool c1 = HOR == 2 || q.nb1 > k, c2 = HOR == 2 || q.nb2 > k;
+  const size_t i1 = q.n1 * LZ + k, i2 = q.n2 * LZ + k;
+  for (int t = 0; t < a.K; ++t) {
+    const double* __restrict__ T = a.T + t * a.sT;
+    const double* __restrict__ TA = ta_sep ? a.TA + t * a.sTA : T;
+    const double s1 = TA[i1], s2 = TA[i2];
+    double lo = 0.0;  // minus the low-order flux
+    if (FCT) lo = ta_sep ? bits64::upwind(v, T[i1], T[i2]) : bits64::upwind(v, s1, s2);
+    double h;
+    if (HOR == 0) {
+      h = -(FCT && !ta_sep ? lo : bits64::upwind(v, s1, s2));
+    } else {
+      const double2* __restrict__ G = GRAD ? grad + (size_t)t * m.M * LZ : nullptr;
+      double g1, g2, g3, g4;
+      if (MEAN) {
+        node_mean_grad<GRAD>(m, TA, G, q.n1, k, g1, g3);
+        node_mean_grad<GRAD>(m, TA, G, q.n2, k, g2, g4);
+      } else {
+        grad_at<GRAD>(m, TA, G, q.up, k, g1, g3);
+        grad_at<GRAD>(m, TA, G, q.dn, k, g2, g4);
+      }
+      const double d2 = bits64::twice(s2 - s1);
+      double r1 = sixth(d2 + q.ex * g1 + q.ey * g3), r2 = sixth(d2 + q.ex * g2 + q.ey * g4);
+      if (HOR == 1 && !(c1 && c2)) {
+        if (bits64::finite(r1, r2)) {
+          r1 = c1 ? r1 : 0.0;
+          r2 = c2 ? r2 : 0.0;
+        } else {
+          r1 = hw_product(r1, c1 ? 1.0 : 0.0);
+          r2 = hw_product(r2, c2 ? 1.0 : 0.0);
+        }
+      }
+      const double Tm1 = s1 + r1, Tm2 = s2 - r2;
+      // ph = 1: the upwind part is an exact zero (of finite values)
+      if (ph1 && bits64::finite(Tm1, Tm2) && bits64::finite(v)) h = -(B * (Tm1 + Tm2));
+      else h = hor_flux_any(v, Tm1, Tm2, a.ph);
+    }
+    a.adfh[t * a.sE + ek] = FCT ? h + lo : h;
+  }
+}
+
+// A tile's layers in three lists, each dealt to the threads by itself: those in the triangles'
+// window, those with mean gradients (some eight times the work: mixed into the first list, a
+// single one held its whole warp), and those below the edge, which are zero.
 template <typename R, int HOR, bool FCT, bool VF, bool GRAD>
 __global__ void __launch_bounds__(kEdgeThreads, 3) k_hflux(DMesh m, StepPtrs<R> a, const double2* __restrict__ grad) {
   __shared__ EdgeTab tab[kEdgeTile];
-  const int w0 = blockIdx.x * kEdgeTile, ne = min(kEdgeTile, m.E - w0);
-  if ((int)threadIdx.x < ne) tab[threadIdx.x] = load_edge<HOR>(m, w0 + threadIdx.x);
-  __syncthreads();
-  const size_t LZ = m.LZ;
-  const bool ta_sep = a.TA != a.T;
-  const bool ph1 = a.ph == R(1);
-  for (unsigned i = threadIdx.x; i < (unsigned)(ne * m.LZ); i += kEdgeThreads) {
-    const unsigned j = i / (unsigned)m.LZ;
-    const int k = (int)(i - j * (unsigned)m.LZ), z = k + 1;
-    const EdgeTab& q = tab[j];
-    const size_t ek = (size_t)q.e * LZ + k;
-    R v;
-    if (VF) {
-      v = edge_vflux(m, q, a.vel, k);
-      a.vf[ek] = v;
-    }
-    if (z > max(q.nl1, q.nl2)) {
-      for (int t = 0; t < a.K; ++t) a.adfh[t * a.sE + ek] = R(0);
-      continue;
-    }
-    if (!VF) v = a.vf[ek];
-    const R B = bits64::half(ph1 ? v : v * a.ph);
-    const bool tri = q.gm0 >= 0 && z >= q.gm0 && z <= q.gm1 - 1;
-    const bool c1 = HOR == 2 || q.nb1 - z >= 0, c2 = HOR == 2 || q.nb2 - z >= 0;
-    const size_t i1 = q.n1 * LZ + k, i2 = q.n2 * LZ + k;
-    for (int t = 0; t < a.K; ++t) {
-      const R* __restrict__ T = a.T + t * a.sT;
-      const R* __restrict__ TA = ta_sep ? a.TA + t * a.sTA : T;
-      const R s1 = TA[i1], s2 = TA[i2];
-      R lo = R(0);  // minus the low-order flux
-      if (FCT) lo = ta_sep ? bits64::upwind(v, T[i1], T[i2]) : bits64::upwind(v, s1, s2);
-      R h;
-      if (HOR == 0) {
-        h = -(FCT && !ta_sep ? lo : bits64::upwind(v, s1, s2));
-      } else {
-        const double2* __restrict__ G = GRAD ? grad + (size_t)t * m.M * LZ : nullptr;
-        R g1, g2, g3, g4;
-        if (tri) {
-          grad_at<GRAD>(m, TA, G, q.up, k, g1, g3);
-          grad_at<GRAD>(m, TA, G, q.dn, k, g2, g4);
-        } else {
-          node_mean_grad<GRAD>(m, TA, G, q.n1, k, g1, g3);
-          node_mean_grad<GRAD>(m, TA, G, q.n2, k, g2, g4);
-        }
-        const R d2 = bits64::twice(s2 - s1);
-        R r1 = sixth(d2 + q.ex * g1 + q.ey * g3), r2 = sixth(d2 + q.ex * g2 + q.ey * g4);
-        if (HOR == 1 && !(c1 && c2)) {
-          if (bits64::finite(r1, r2)) {
-            r1 = c1 ? r1 : R(0);
-            r2 = c2 ? r2 : R(0);
-          } else {
-            r1 = hw_product(r1, c1 ? R(1) : R(0));
-            r2 = hw_product(r2, c2 ? R(1) : R(0));
-          }
-        }
-        const R Tm1 = s1 + r1, Tm2 = s2 - r2;
-        // ph = 1: the upwind part is an exact zero (of finite values)
-        if (ph1 && bits64::finite(Tm1, Tm2) && bits64::finite(v)) h = -(B * (Tm1 + Tm2));
-        else h = hor_flux_any(v, Tm1, Tm2, a.ph);
+  __shared__ int win[kEdgeTile][2];         // the window's layers [first, end) per edge (0-based)
+  __shared__ int ptr[3][kEdgeTile + 1];     // starts of the edges' parts of the three lists
+  const int w0 = blockIdx.x * kEdgeTile, ne = min(kEdgeTile, m.E - w0), tid = threadIdx.x;
+  if (tid < kWarp) {
+    int cnt[3] = {0, 0, 0};
+    if (tid < ne) {
+      const EdgeTab q = load_edge<HOR>(m, w0 + tid);
+      tab[tid] = q;
+      const int hi = max(q.nl1, q.nl2);
+      int first = 0, end = hi;
+      if (HOR != 0) {
+        first = q.gm0 < 0 ? 0 : min(q.gm0 - 1, hi);
+        end = q.gm0 < 0 ? 0 : max(first, min(q.gm1 - 1, hi));
       }
-      a.adfh[t * a.sE + ek] = FCT ? h + lo : h;
+      win[tid][0] = first;
+      win[tid][1] = end;
+      cnt[0] = end - first;
+      cnt[1] = hi - cnt[0];
+      cnt[2] = m.LZ - hi;
     }
+#pragma unroll
+    for (int l = 0; l < 3; ++l) {
+#pragma unroll
+      for (int d = 1; d < kEdgeTile; d *= 2) {
+        const int x = __shfl_up_sync(0xffffffffu, cnt[l], d);
+        if (tid >= d) cnt[l] += x;
+      }
+      if (tid < kEdgeTile) ptr[l][tid + 1] = cnt[l];
+      if (tid == 0) ptr[l][0] = 0;
+    }
+  }
+  __syncthreads();
+  auto edge_of = [&](int l, int i) {  // the edge of a list's item i
+    int j = 0;
+#pragma unroll
+    for (int d = kEdgeTile / 2; d > 0; d /= 2)
+      if (i >= ptr[l][j + d]) j += d;
+    return j;
+  };
+  for (int i = tid; i < ptr[0][kEdgeTile]; i += kEdgeThreads) {
+    const int j = edge_of(0, i);
+    hor_flux<HOR, FCT, VF, GRAD, false>(m, a, grad, tab[j], win[j][0] + i - ptr[0][j]);
+  }
+  if (HOR != 0)
+    for (int i = tid; i < ptr[1][kEdgeTile]; i += kEdgeThreads) {
+      const int j = edge_of(1, i);
+      int k = i - ptr[1][j];
+      if (k >= win[j][0]) k += win[j][1] - win[j][0];
+      hor_flux<HOR, FCT, VF, GRAD, true>(m, a, grad, tab[j], k);
+    }
+  for (int i = tid; i < ptr[2][kEdgeTile]; i += kEdgeThreads) {
+    const int j = edge_of(2, i);
+    const size_t ek = (size_t)tab[j].e * m.LZ + max(tab[j].nl1, tab[j].nl2) + i - ptr[2][j];
+    if (VF) a.vf[ek] = R(0);
+    for (int t = 0; t < a.K; ++t) a.adfh[t * a.sE + ek] = R(0);
   }
 }
 
