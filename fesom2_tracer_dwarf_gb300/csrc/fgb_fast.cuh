@@ -272,6 +272,61 @@ static __global__ void __launch_bounds__(256) kf_vflux(DMesh m, const float* __r
   }
 }
 
+// The same with one thread per edge (in visit order) and four layers, for
+// meshes below kVfluxSmall edge-layers: as many threads as there is work for
+// and up to 96 bytes of loads in flight in each. 48x40x30 6.3 us against 12.4,
+// 256^2x64 47 / 68, pi mesh of 188,661 nodes and 47 layers 86 / 102; above,
+// the kernel above keeps more of the elements that neighbouring edges share in
+// L1 (closed 513^2x64 162 / 163, 1024^2x64 634 / 580).
+constexpr int kVfluxThreads = 256;
+constexpr long long kVfluxSmall = 1LL << 25;
+
+// Four layers of an element's velocity; 16-byte loads where the array is aligned for them.
+__device__ __forceinline__ void ld_uv4(const float* __restrict__ vel, unsigned i, bool wide, float2 (&u)[4]) {
+  if (wide) {
+    const float4* p = reinterpret_cast<const float4*>(vel) + (size_t)i / 2;
+    const float4 x = p[0], y = p[1];
+    u[0] = make_float2(x.x, x.y);
+    u[1] = make_float2(x.z, x.w);
+    u[2] = make_float2(y.x, y.y);
+    u[3] = make_float2(y.z, y.w);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) u[q] = reinterpret_cast<const float2*>(vel)[(size_t)i + q];
+  }
+}
+
+static __global__ void __launch_bounds__(kVfluxThreads) kf_vflux4(DMesh m, const float* __restrict__ vel,
+                                                                  float* __restrict__ vf) {
+  const unsigned q4 = (unsigned)m.LZ / 4, it = blockIdx.x * kVfluxThreads + threadIdx.x, w = it / q4;
+  if (w >= (unsigned)m.E) return;
+  const unsigned LZ = m.LZ, k = 4 * (it - w * q4);
+  const int e = m.edge_order ? m.edge_order[w] : (int)w;  // the edges of a node together: element reuse in L2
+  const int2 el = reinterpret_cast<const int2*>(m.edge_tri)[e];
+  const int4 lev = reinterpret_cast<const int4*>(m.edge_lev)[e];
+  const float4 cr = reinterpret_cast<const float4*>(m.g32.edge_cross)[e];
+  const bool wide = reinterpret_cast<uintptr_t>(vel) % 16 == 0;
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  float2 u1[4], u2[4];
+  float4 h1 = make_float4(0.f, 0.f, 0.f, 0.f), h2 = h1;
+  const bool a1 = (int)k < lev.y, a2 = (int)k < lev.w;  // layers 1..nl1 of element 1, 1..nl2 of element 2
+  if (a1) {
+    ld_uv4(vel, (unsigned)el.x * LZ + k, wide, u1);
+    h1 = reinterpret_cast<const float4*>(m.g32.helem)[((unsigned)el.x * LZ + k) / 4];
+  }
+  if (a2) {
+    ld_uv4(vel, (unsigned)el.y * LZ + k, wide, u2);
+    h2 = reinterpret_cast<const float4*>(m.g32.helem)[((unsigned)el.y * LZ + k) / 4];
+  }
+  const float g1[4] = {h1.x, h1.y, h1.z, h1.w}, g2[4] = {h2.x, h2.y, h2.z, h2.w};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if ((int)k + q < lev.y) v[q] = (-(u1[q].y * cr.x) + u1[q].x * cr.y) * g1[q];
+    if ((int)k + q < lev.w) v[q] = v[q] + (u2[q].y * cr.z - u2[q].x * cr.w) * g2[q];
+  }
+  reinterpret_cast<float4*>(vf)[((unsigned)e * LZ + k) / 4] = make_float4(v[0], v[1], v[2], v[3]);
+}
+
 // ---------------------------------------------------------------------------
 // Horizontal edge fluxes of all tracer groups (FCT: HO(T_AB) - LO(T), else
 // HO). HOR: 0 UPW1 (lib/oce_adv_tra_hor.F90:218-220), 1 MUSCL
@@ -285,6 +340,8 @@ static __global__ void __launch_bounds__(256) kf_vflux(DMesh m, const float* __r
 // Layers outside the triangles' common window use the area-weighted mean
 // gradient of the elements around each node (lib/oce_muscl_adv.F90:393-410).
 // ---------------------------------------------------------------------------
+// Three elements at a time: their index, table and value loads are in flight
+// together (an element that is not there or dry at the layer has weight zero).
 template <int KV>
 __device__ __forceinline__ void node_grad(const DMesh& m, const float* __restrict__ TA, int n, unsigned k,
                                           V<KV>& gx, V<KV>& gy) {
@@ -293,18 +350,26 @@ __device__ __forceinline__ void node_grad(const DMesh& m, const float* __restric
   const int z = (int)k + 1;
   float tvol = 0.f;
   V<KV> tx = splat<KV>(0.f), ty = splat<KV>(0.f);
-  for (int j = m.nie_ptr[n]; j < m.nie_ptr[n + 1]; ++j) {
-    const int el = m.nie_idx[j];
-    if (m.elem_nlev[el] - 1 < z) continue;
-    const int a = m.elem_nodes[3 * el], b = m.elem_nodes[3 * el + 1], c = m.elem_nodes[3 * el + 2];
-    const float* gs = g.grad_sca + 6 * (size_t)el;
-    const V<KV> ta = ld<KV>(TA, a * LZ + k), tb = ld<KV>(TA, b * LZ + k), tc = ld<KV>(TA, c * LZ + k);
-    const V<KV> ex = fmas(tc, gs[2], fmas(tb, gs[1], muls(ta, gs[0])));
-    const V<KV> ey = fmas(tc, gs[5], fmas(tb, gs[4], muls(ta, gs[3])));
-    const float ar = g.elem_area[el];
-    tvol += ar;
-    tx = fmas(ex, ar, tx);
-    ty = fmas(ey, ar, ty);
+  const int end = m.nie_ptr[n + 1];
+  for (int j = m.nie_ptr[n]; j < end; j += 3) {
+    float ar[3];
+    V<KV> ex[3], ey[3];
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      const int el = m.nie_idx[min(j + u, end - 1)];
+      const int a = m.elem_nodes[3 * el], b = m.elem_nodes[3 * el + 1], c = m.elem_nodes[3 * el + 2];
+      const float* gs = g.grad_sca + 6 * (size_t)el;
+      const V<KV> ta = ld<KV>(TA, a * LZ + k), tb = ld<KV>(TA, b * LZ + k), tc = ld<KV>(TA, c * LZ + k);
+      ex[u] = fmas(tc, gs[2], fmas(tb, gs[1], muls(ta, gs[0])));
+      ey[u] = fmas(tc, gs[5], fmas(tb, gs[4], muls(ta, gs[3])));
+      ar[u] = j + u < end && m.elem_nlev[el] - 1 >= z ? g.elem_area[el] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      tvol += ar[u];
+      tx = fmas(ex[u], ar[u], tx);
+      ty = fmas(ey[u], ar[u], ty);
+    }
   }
   const float inv = fdv(1.f, tvol);
   gx = muls(tx, inv);

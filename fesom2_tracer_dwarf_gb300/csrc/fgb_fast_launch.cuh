@@ -30,6 +30,11 @@ void launch_hflux_tile(const DMesh& m, const FastPtrs& a, cudaStream_t s) {
   const size_t sm = tile_smem_bytes(KV, FCT && a.TA != a.T, m.tile_max_nodes);
   allow_smem_f(kf_hflux_tile<HOR, FCT, KV>, sm);
   kf_hflux_tile<HOR, FCT, KV><<<m.ntiles, kTileThreads, sm, s>>>(m, a);
+  if constexpr (HOR != 0) {
+    constexpr int runs = kTileThreads / (2 * kMeanRun);
+    if (m.nmean > 0)
+      kf_hflux_mean<HOR, FCT, KV><<<dim3((m.nmean + runs - 1) / runs, a.G), kTileThreads, 0, s>>>(m, a);
+  }
 }
 
 template <int KV, int HOR>
@@ -150,14 +155,18 @@ template <int KV>
 int launch_fast(const DMesh& m, const FastPtrs& a, const LaunchArgs& L, cudaStream_t s) {
   int launches = 0;
   if (L.mask & FGB_STAGE_VFLUX) {
-    kf_vflux<<<(m.E + 8 * kW - 1) / (8 * kW), 8 * kW, 0, s>>>(m, a.vel, a.vf);
+    const long long items = (long long)m.E * (m.LZ / 4);
+    if (4 * items < kVfluxSmall)
+      kf_vflux4<<<(unsigned)((items + kVfluxThreads - 1) / kVfluxThreads), kVfluxThreads, 0, s>>>(m, a.vel, a.vf);
+    else
+      kf_vflux<<<(m.E + 8 * kW - 1) / (8 * kW), 8 * kW, 0, s>>>(m, a.vel, a.vf);
     ++launches;
   }
   if (L.mask & FGB_STAGE_HFLUX) {
     if (L.hor == FGB_HOR_UPW1) launch_hflux_ns<KV, 0>(m, a, L, s);
     else if (L.hor == FGB_HOR_MUSCL) launch_hflux_ns<KV, 1>(m, a, L, s);
     else launch_hflux_ns<KV, 2>(m, a, L, s);
-    ++launches;
+    launches += L.hflux_tile && m.ntiles > 0 && L.hor != FGB_HOR_UPW1 && m.nmean > 0 ? 2 : 1;
   }
   if (L.fct) {
     if (L.mask & FGB_STAGE_LO) {

@@ -113,12 +113,12 @@ int launch_stages_f32(const DMesh& m, const fgb_step_desc& d, int mask, cudaStre
   L.vimpl_thomas = d.cfg[8] == 1;
   // Edge fluxes: the tiled kernel unless cfg[0] or cfg[7] asks for a shape of
   // the per-edge one. A block of the tiled kernel holds at most 32 edges, so a
-  // small mesh still fills the GPU, and a layer outside its triangles' window
-  // costs its own lane the element gradients around the nodes, not the whole
-  // warp. Edge stage, per-edge kernel against tiled: 48x40x30, 3 tracers, 103
-  // against 35 us; closed 513^2x64, 2 tracers, 930 / 477 us; pi refined to
-  // 188,661 nodes, 47 layers, 4 tracers, 670 / 438 us; 250x230x47, 2 tracers,
-  // 149 / 91 us; 256^2x64, 4 tracers, 162 / 125 us; no size was slower.
+  // small mesh still fills the GPU, and layers outside their triangles' window
+  // go to a kernel of their own. Edge stage, per-edge kernel against tiled:
+  // 48x40x30, 3 tracers, 103 against 20 us; closed 513^2x64, 2 tracers, 930 /
+  // 370 us; pi refined to 188,661 nodes, 47 layers, 4 tracers, 670 / 305 us;
+  // 250x230x47, 2 tracers, 149 / 85 us; 256^2x64, 4 tracers, 162 / 121 us; no
+  // size was slower.
   // The tiled kernel stages rows with 16-byte asynchronous copies; fields on
   // other addresses take the per-edge kernel.
   auto al16 = [](const void* p) { return p == nullptr || reinterpret_cast<uintptr_t>(p) % 16 == 0; };
