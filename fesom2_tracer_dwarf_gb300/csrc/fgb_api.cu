@@ -612,3 +612,46 @@ int fgb_tracer_stats_grouped(const fgb_mesh* m, const float* T, long long stride
 }
 
 }  // extern "C"
+
+// ---------------------------------------------------------------------------
+// Rows of the reference's arrays to and from the padded layouts.
+// ---------------------------------------------------------------------------
+namespace fgb {
+namespace {
+constexpr int kRowThreads = 256;
+template <typename R>
+__global__ void __launch_bounds__(kRowThreads) k_pad_rows(const double* __restrict__ src, long long rows, int ncol,
+                                                          int ld, R* __restrict__ dst) {
+  for (long long i = (long long)blockIdx.x * kRowThreads + threadIdx.x; i < rows * ld;
+       i += (long long)gridDim.x * kRowThreads) {
+    const long long r = i / ld, k = i - r * ld;
+    dst[i] = k < ncol ? (R)src[r * ncol + k] : R(0);
+  }
+}
+template <typename R>
+__global__ void __launch_bounds__(kRowThreads) k_pack_rows(const R* __restrict__ src, long long rows, int ncol, int ld,
+                                                           double* __restrict__ dst) {
+  for (long long i = (long long)blockIdx.x * kRowThreads + threadIdx.x; i < rows * ncol;
+       i += (long long)gridDim.x * kRowThreads) {
+    const long long r = i / ncol, k = i - r * ncol;
+    dst[i] = (double)src[r * ld + k];
+  }
+}
+unsigned row_blocks(long long n) {
+  return (unsigned)std::min<long long>(std::max<long long>((n + kRowThreads - 1) / kRowThreads, 1), 152 * 16);
+}
+}  // namespace
+
+int pad_rows(const double* src, long long rows, int ncol, int ld, bool fp32, void* dst) {
+  const unsigned b = row_blocks(rows * ld);
+  if (fp32) k_pad_rows<<<b, kRowThreads>>>(src, rows, ncol, ld, static_cast<float*>(dst));
+  else k_pad_rows<<<b, kRowThreads>>>(src, rows, ncol, ld, static_cast<double*>(dst));
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+int pack_rows(const void* src, long long rows, int ncol, int ld, bool fp32, double* dst) {
+  const unsigned b = row_blocks(rows * ncol);
+  if (fp32) k_pack_rows<<<b, kRowThreads>>>(static_cast<const float*>(src), rows, ncol, ld, dst);
+  else k_pack_rows<<<b, kRowThreads>>>(static_cast<const double*>(src), rows, ncol, ld, dst);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+}  // namespace fgb

@@ -74,12 +74,13 @@ struct State {
   long long ws_bytes = 0;
   bool device_ready = false;   // device buffers allocated for the current configuration
   bool mesh_dirty = true;      // levels or thicknesses changed: rebuild the device mesh
-  bool inputs_dirty = true;    // fields changed since the last upload
+  unsigned inputs_dirty = 7;   // fields changed since the last upload (kDirty*)
   bool values_on_device = false;  // tracer 1 values newer on the device than on the host
   int dev_precision = -1;
 };
 
 State g;
+constexpr unsigned kDirtyT = 1, kDirtyVel = 2, kDirtyW = 4, kDirtyAll = 7;
 
 int fail(const char* msg) {
   std::fprintf(stderr, "### error: %s\n", msg);
@@ -110,89 +111,88 @@ void free_device() {
 
 int node_size() { return g.myDim + g.eDim; }
 
-const fgb::HostMesh* hm() { return g.hmesh ? g.hmesh->m : nullptr; }
-
-// Host (nl-1, n) column-major -> device (n, LZ) padded, in the form's precision.
-template <typename R>
-std::vector<R> pad_cols(const double* src, int n, int nrow, int ld) {
-  std::vector<R> out((size_t)n * ld, R(0));
-  for (int j = 0; j < n; ++j)
-    for (int i = 0; i < nrow; ++i) out[(size_t)j * ld + i] = (R)src[(size_t)j * nrow + i];
-  return out;
+// Host rows of ncol values (columns of the reference's arrays) to rows of ld
+// on the device, in the form's precision. The rows go over as they are, through
+// the step's workspace (idle between steps), and a kernel pads and converts
+// them: padding every array on the host took most of a small step's time.
+int upload_rows(const double* src, size_t rows, int ncol, int ld, void* dst) {
+  const size_t row = (size_t)ncol * sizeof(double), at_once = (size_t)g.ws_bytes / row;
+  const size_t out = (size_t)ld * (g.dev_precision == FGB_FP32 ? 4 : 8);
+  if (at_once == 0) return fail("a column does not fit the workspace");
+  for (size_t r = 0; r < rows; r += at_once) {
+    const size_t n = std::min(at_once, rows - r);
+    if (cudaMemcpy(g.dws, src + r * ncol, n * row, cudaMemcpyHostToDevice) != cudaSuccess ||
+        fgb::pad_rows(static_cast<const double*>(g.dws), (long long)n, ncol, ld, g.dev_precision == FGB_FP32,
+                      static_cast<char*>(dst) + r * out))
+      return fail("cudaMemcpy to the device failed");
+  }
+  return 0;
+}
+// The way back: device rows of ld to host rows of ncol values.
+int download_rows(const void* src, size_t rows, int ncol, int ld, double* dst) {
+  const size_t row = (size_t)ncol * sizeof(double), at_once = (size_t)g.ws_bytes / row;
+  const size_t in = (size_t)ld * (g.dev_precision == FGB_FP32 ? 4 : 8);
+  if (at_once == 0) return fail("a column does not fit the workspace");
+  for (size_t r = 0; r < rows; r += at_once) {
+    const size_t n = std::min(at_once, rows - r);
+    if (fgb::pack_rows(static_cast<const char*>(src) + r * in, (long long)n, ncol, ld, g.dev_precision == FGB_FP32,
+                       static_cast<double*>(g.dws)) ||
+        cudaMemcpy(dst + r * ncol, g.dws, n * row, cudaMemcpyDeviceToHost) != cudaSuccess)
+      return fail("cudaMemcpy from the device failed");
+  }
+  return 0;
 }
 
-int copy_to_device(void* dst, const void* src, size_t bytes) {
-  return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess ? 0 : -1;
-}
-
-template <typename R>
+// Uploads the fields that changed.
 int upload_inputs() {
-  const fgb::HostMesh& h = *hm();
   int dims[8];
   fgb_mesh_dims(g.dmesh, dims);
   const int N = dims[0], M = dims[2], nz = dims[4], LZ = dims[5], LW = dims[6], nl = nz + 1;
-  const Tracer& t = g.tr[0];
-  auto T = pad_cols<R>(t.values.data(), N, nz, LZ);
-  auto TA = pad_cols<R>(t.valuesAB.data(), N, nz, LZ);
-  // The step reads the uv buffer as vel(2, nl-1, elem2D) (sequence association).
-  std::vector<R> vel((size_t)M * LZ * 2, R(0));
-  if (g.have_uv)
-    for (int el = 0; el < M; ++el)
-      for (int z = 0; z < nz; ++z)
-        for (int c = 0; c < 2; ++c) vel[((size_t)el * LZ + z) * 2 + c] = (R)g.uv[(size_t)c + 2 * ((size_t)z + (size_t)nz * el)];
-  std::vector<R> w((size_t)N * LW, R(0)), we((size_t)N * LW, R(0)), wi((size_t)N * LW, R(0));
-  auto cols = [&](const std::vector<double>& src, std::vector<R>& dst) {
-    for (int n = 0; n < N; ++n)
-      for (int z = 0; z < nl; ++z) dst[(size_t)n * LW + z] = (R)src[(size_t)n * nl + z];
+  const size_t s = g.dev_precision == FGB_FP32 ? 4 : 8;
+  auto zero = [](void* p, size_t bytes) {
+    return cudaMemset(p, 0, bytes) == cudaSuccess ? 0 : fail("cudaMemset on the device failed");
   };
-  if (g.have_w) cols(g.w, w);
-  if (g.have_we) cols(g.we, we);
-  if (g.use_wsplit && g.wi.size() == (size_t)N * nl) cols(g.wi, wi);
-  (void)h;
-  if (copy_to_device(g.dT, T.data(), T.size() * sizeof(R)) || copy_to_device(g.dTA, TA.data(), TA.size() * sizeof(R)) ||
-      copy_to_device(g.dvel, vel.data(), vel.size() * sizeof(R)) || copy_to_device(g.dw, w.data(), w.size() * sizeof(R)) ||
-      copy_to_device(g.dwe, we.data(), we.size() * sizeof(R)) || copy_to_device(g.dwi, wi.data(), wi.size() * sizeof(R)))
-    return fail("cudaMemcpy to the device failed");
+  if (g.inputs_dirty & kDirtyT) {
+    const Tracer& t = g.tr[0];
+    if (upload_rows(t.values.data(), N, nz, LZ, g.dT) || upload_rows(t.valuesAB.data(), N, nz, LZ, g.dTA)) return -1;
+  }
+  if (g.inputs_dirty & kDirtyVel) {
+    // The step reads the uv buffer as vel(2, nl-1, elem2D) (sequence association).
+    if (g.have_uv ? upload_rows(g.uv.data(), M, 2 * nz, 2 * LZ, g.dvel) : zero(g.dvel, (size_t)M * LZ * 2 * s)) return -1;
+  }
+  if (g.inputs_dirty & kDirtyW) {
+    const size_t bytes = (size_t)N * LW * s;
+    auto put = [&](bool have, const std::vector<double>& src, void* dst) {
+      return have ? upload_rows(src.data(), N, nl, LW, dst) : zero(dst, bytes);
+    };
+    if (put(g.have_w, g.w, g.dw) || put(g.have_we, g.we, g.dwe) ||
+        put(g.use_wsplit && g.wi.size() == (size_t)N * nl, g.wi, g.dwi))
+      return -1;
+  }
   if (g.del_pending) {  // the restart's del_ttf, once
-    auto del = pad_cols<R>(g.del.data(), N, nz, LZ);
-    if (copy_to_device(g.ddel, del.data(), del.size() * sizeof(R))) return fail("cudaMemcpy to the device failed");
+    if (upload_rows(g.del.data(), N, nz, LZ, g.ddel)) return -1;
     g.del_pending = false;
   }
   return 0;
 }
 
 // del_ttf of the device (the step's accumulated tendency) into g.del.
-template <typename R>
 int download_del() {
   int dims[8];
   fgb_mesh_dims(g.dmesh, dims);
-  const int N = dims[0], nz = dims[4], LZ = dims[5];
-  std::vector<R> D((size_t)N * LZ);
-  if (cudaMemcpy(D.data(), g.ddel, D.size() * sizeof(R), cudaMemcpyDeviceToHost) != cudaSuccess)
-    return fail("cudaMemcpy from the device failed");
-  g.del.assign((size_t)N * nz, 0.0);
-  for (int n = 0; n < N; ++n)
-    for (int z = 0; z < nz; ++z) g.del[(size_t)n * nz + z] = (double)D[(size_t)n * LZ + z];
-  return 0;
+  g.del.assign((size_t)dims[0] * dims[4], 0.0);
+  return download_rows(g.ddel, dims[0], dims[4], dims[5], g.del.data());
 }
 
-template <typename R>
 int download_values() {
   int dims[8];
   fgb_mesh_dims(g.dmesh, dims);
-  const int N = dims[0], nz = dims[4], LZ = dims[5];
-  std::vector<R> T((size_t)N * LZ);
-  if (cudaMemcpy(T.data(), g.dT, T.size() * sizeof(R), cudaMemcpyDeviceToHost) != cudaSuccess)
-    return fail("cudaMemcpy from the device failed");
-  std::vector<double>& v = g.tr[0].values;
-  for (int n = 0; n < N; ++n)
-    for (int z = 0; z < nz; ++z) v[(size_t)n * nz + z] = (double)T[(size_t)n * LZ + z];
-  return 0;
+  return download_rows(g.dT, dims[0], dims[4], dims[5], g.tr[0].values.data());
 }
 
 int sync_values_to_host() {
   if (!g.values_on_device) return 0;
-  int rc = g.dev_precision == FGB_FP32 ? download_values<float>() : download_values<double>();
+  int rc = download_values();
   if (rc == 0) g.values_on_device = false;
   return rc;
 }
@@ -244,13 +244,12 @@ int prepare_device() {
     }
     g.device_ready = true;
     g.dev_precision = g.precision;
-    g.inputs_dirty = true;
+    g.inputs_dirty = kDirtyAll;
   }
   if (g.inputs_dirty) {
-    int rc = g.precision == FGB_FP32 ? upload_inputs<float>() : upload_inputs<double>();
-    if (rc) return rc;
-    g.inputs_dirty = false;
-    g.values_on_device = false;
+    if (upload_inputs()) return -1;
+    if (g.inputs_dirty & kDirtyT) g.values_on_device = false;
+    g.inputs_dirty = 0;
   }
   return 0;
 }
@@ -344,7 +343,8 @@ int adopt_restart(const std::string& npepath, fgb::restart::Record&& rm, fgb::re
   g.rdyn = std::move(rd);
   g.rtracer = rt ? std::move(*rt) : fgb::restart::Record();
   g.initialized = true;
-  g.mesh_dirty = g.inputs_dirty = true;
+  g.mesh_dirty = true;
+  g.inputs_dirty = kDirtyAll;
   return 0;
 }
 
@@ -380,7 +380,7 @@ int adopt_tracers(const fgb::restart::Record& rt) {
   g.del_pending = del && del->dims == dim_v;
   g.del = g.del_pending ? del->vr : std::vector<double>();
   g.values_on_device = false;
-  g.inputs_dirty = true;
+  g.inputs_dirty = kDirtyAll;
   return 0;
 }
 
@@ -515,8 +515,7 @@ int tracer_get_values(double* values, int nz, int nn) {
   if (nz > g.nl - 1 || nn > node_size() || nz < 0 || nn < 0) return fail("requested size exceeds the tracer array");
   if (sync_values_to_host()) return -1;
   const std::vector<double>& v = g.tr[0].values;
-  for (int j = 0; j < nn; ++j)
-    for (int i = 0; i < nz; ++i) values[(size_t)j * nz + i] = v[(size_t)j * (g.nl - 1) + i];
+  for (int j = 0; j < nn; ++j) std::copy_n(v.data() + (size_t)j * (g.nl - 1), nz, values + (size_t)j * nz);
   return 0;
 }
 
@@ -528,7 +527,7 @@ int tracer_finalize(const char* output_dir) {
   const fgb::HostMesh& h = *g.hmesh->m;
   if (sync_values_to_host()) return -1;
   if (g.device_ready && g.ddel) {
-    const int rc = g.dev_precision == FGB_FP32 ? download_del<float>() : download_del<double>();
+    const int rc = download_del();
     if (rc) return rc;
   }
   const std::string out = c2s(output_dir), npepath = out + "/np" + std::to_string(g.npes);
@@ -616,7 +615,8 @@ int tracer_set_levels(const int* nlevels, const int* ulevels, int nod2D) {
   if (sync_values_to_host()) return -1;
   g.set_nlev.assign(nlevels, nlevels + nod2D);
   g.set_ulev.assign(ulevels, ulevels + nod2D);
-  g.mesh_dirty = g.inputs_dirty = true;
+  g.mesh_dirty = true;
+  g.inputs_dirty = kDirtyAll;
   return 0;
 }
 
@@ -625,7 +625,8 @@ int tracer_set_thickness(const double* hnode, int nl, int nod2D) {
   if (sync_values_to_host()) return -1;
   g.hnode_new.assign(hnode, hnode + (size_t)(nl - 1) * nod2D);
   g.have_hnode_new = true;
-  g.mesh_dirty = g.inputs_dirty = true;
+  g.mesh_dirty = true;
+  g.inputs_dirty = kDirtyAll;
   return 0;
 }
 
@@ -647,7 +648,7 @@ int tracer_allocate_tracers(int num_tracers, int nl, int nod2D, int AB_order) {
   g.ab_order = AB_order;
   if (g.nl == 0) g.nl = nl;
   g.values_on_device = false;
-  g.inputs_dirty = true;
+  g.inputs_dirty = kDirtyAll;
   g.del_pending = false;
   g.del.clear();
   if (g.device_ready && g.ddel) {  // del_ttf is re-zeroed with the work arrays
@@ -668,11 +669,9 @@ int tracer_set_values(int tracer_id, const double* values, int nl, int nod2D) {
   const size_t n = (size_t)(nl - 1) * nod2D;
   if (n > t.values.size()) return fail("values larger than the tracer array");
   if (tracer_id == 1 && sync_values_to_host()) return -1;
-  for (size_t i = 0; i < n; ++i) {
-    t.values[i] = values[i];
-    t.valuesAB[i] = values[i];
-  }
-  g.inputs_dirty = true;
+  std::copy(values, values + n, t.values.begin());
+  std::copy(values, values + n, t.valuesAB.begin());
+  g.inputs_dirty |= kDirtyT;
   return 0;
 }
 
@@ -690,7 +689,7 @@ int tracer_set_velocity_zero(int nl, int nod2D, int edge2D) {
   g.have_uv = g.have_w = true;
   g.have_we = false;
   std::fill(g.wi.begin(), g.wi.end(), 0.0);
-  g.inputs_dirty = true;
+  g.inputs_dirty |= kDirtyVel | kDirtyW;
   return 0;
 }
 
@@ -706,7 +705,7 @@ int tracer_set_velocity(const double* uv, const double* w, int nl, int nod2D, in
   g.have_uv = g.have_w = true;
   g.have_we = false;  // w_e = w_i = 0 (:735-736)
   std::fill(g.wi.begin(), g.wi.end(), 0.0);
-  g.inputs_dirty = true;
+  g.inputs_dirty |= kDirtyVel | kDirtyW;
   return 0;
 }
 
@@ -770,7 +769,8 @@ int tracer_load_mesh_from_files(const char* mesh_path) {
   g.set_nlev.clear();
   g.set_ulev.clear();
   g.initialized = true;  // :856-857
-  g.mesh_dirty = g.inputs_dirty = true;
+  g.mesh_dirty = true;
+  g.inputs_dirty = kDirtyAll;
   std::printf("Mesh loaded successfully from partition files\n");
   std::printf("  Mesh: nl=%8d, nod2D=%8d, edge2D=%8d\n", m.nl, m.N, m.E);
   std::printf("  Partition: myDim=%8d, eDim=%8d\n", m.N, 0);
@@ -788,7 +788,8 @@ int tracer_init_ale_arrays(void) {
   g.hnode_new = h.hnode_new;
   g.helem = h.helem;
   g.have_hnode = g.have_hnode_new = g.have_helem = true;
-  g.mesh_dirty = g.inputs_dirty = true;
+  g.mesh_dirty = true;
+  g.inputs_dirty = kDirtyAll;
   return 0;
 }
 
@@ -832,7 +833,8 @@ int tracer_generate_analytic_mesh(int nx, int ny, int nl, int periodic) {
   g.set_nlev.clear();
   g.set_ulev.clear();
   g.initialized = true;  // a loaded mesh marks the system initialised (:856-857)
-  g.mesh_dirty = g.inputs_dirty = true;
+  g.mesh_dirty = true;
+  g.inputs_dirty = kDirtyAll;
   return 0;
 }
 
@@ -863,7 +865,7 @@ int tracer_set_precision(int precision) {
   if (precision != FGB_FP64 && precision != FGB_FP32) return fail("precision must be 0 (FP64) or 1 (FP32)");
   if (sync_values_to_host()) return -1;
   g.precision = precision;
-  g.inputs_dirty = true;
+  g.inputs_dirty = kDirtyAll;
   return 0;
 }
 

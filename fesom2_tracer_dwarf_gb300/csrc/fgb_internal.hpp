@@ -47,6 +47,11 @@ int launch_stages_f64fast(const DMesh& m, const fgb_step_desc& d, int mask, cuda
 
 void set_error(const std::string& msg);
 
+// On the default stream: rows of ncol FP64 values to rows of ld values (zeros
+// behind) in FP64 or FP32, and back. 0 or -1.
+int pad_rows(const double* src, long long rows, int ncol, int ld, bool fp32, void* dst);
+int pack_rows(const void* src, long long rows, int ncol, int ld, bool fp32, double* dst);
+
 }  // namespace fgb
 
 struct fgb_hmesh {
