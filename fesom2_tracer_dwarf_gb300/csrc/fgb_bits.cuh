@@ -33,17 +33,23 @@ __device__ __forceinline__ unsigned mag_hi(double x) { return (unsigned)(to_bits
 __device__ __forceinline__ bool finite(double x) { return mag_hi(x) < 0x7ff00000u; }
 __device__ __forceinline__ bool finite(double x, double y) { return max(mag_hi(x), mag_hi(y)) < 0x7ff00000u; }
 
-// The floating-point expressions behind the integer ones: out of line, because
-// the compiler would otherwise predicate these few instructions into the common
-// path, where they occupy the FP64 pipe all the same.
-static __device__ __noinline__ double hw_lesser(double a, double b) { return a < b ? a : b; }
-static __device__ __noinline__ double hw_greater(double a, double b) { return a > b ? a : b; }
-static __device__ __noinline__ bool hw_exceeds(double a, double b) { return a > b; }
-static __device__ __noinline__ double hw_scale(double x, double s) { return x * s; }
-static __device__ __noinline__ double hw_upwind(double v, double t1, double t2) {
-  return 0.5 * (t1 * (v + fabs(v)) + t2 * (v - fabs(v)));
+// The floating-point expressions behind the integer ones (see one_turn).
+using intdiv::behind_branch;
+static __device__ __noinline__ double hw_lesser(double a, double b) {
+  return behind_branch<double>([&] { return a < b ? a : b; });
 }
-static __device__ __noinline__ bool hw_product_positive(double a, double b) { return a * b > 0.0; }
+static __device__ __noinline__ double hw_greater(double a, double b) {
+  return behind_branch<double>([&] { return a > b ? a : b; });
+}
+static __device__ __noinline__ bool hw_exceeds(double a, double b) {
+  return behind_branch<bool>([&] { return a > b; });
+}
+static __device__ __noinline__ double hw_upwind(double v, double t1, double t2) {
+  return behind_branch<double>([&] { return 0.5 * (t1 * (v + fabs(v)) + t2 * (v - fabs(v))); });
+}
+static __device__ __noinline__ bool hw_product_positive(double a, double b) {
+  return behind_branch<bool>([&] { return a * b > 0.0; });
+}
 
 // a < b ? a : b
 __device__ __forceinline__ double lesser(double a, double b) {
@@ -68,14 +74,14 @@ __device__ __forceinline__ double twice(double x) {
   const uint64_t b = to_bits(x);
   const unsigned e = (unsigned)(b >> 32) & 0x7ff00000u;
   if ((b << 1) == 0) return x;
-  if (e - 0x00100000u >= 0x7fd00000u) return hw_scale(x, 2.0);
+  if (e - 0x00100000u >= 0x7fd00000u) return intdiv::hw_mul(x, 2.0);
   return from_bits(b + (1ull << 52));
 }
 __device__ __forceinline__ double half(double x) {
   const uint64_t b = to_bits(x);
   const unsigned e = (unsigned)(b >> 32) & 0x7ff00000u;
   if ((b << 1) == 0) return x;
-  if (e - 0x00200000u >= 0x7fd00000u) return hw_scale(x, 0.5);
+  if (e - 0x00200000u >= 0x7fd00000u) return intdiv::hw_mul(x, 0.5);
   return from_bits(b - (1ull << 52));
 }
 

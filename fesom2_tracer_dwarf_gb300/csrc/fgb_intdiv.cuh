@@ -1,4 +1,4 @@
-// Correctly rounded FP64 division on the integer pipe.
+// Correctly rounded FP64 division and multiplication on the integer pipe.
 //
 // This GPU issues one FP64 warp instruction per 16 cycles and SM (about two
 // lanes a cycle), against four integer warp instructions per cycle: a hardware
@@ -36,9 +36,15 @@
 namespace fgb {
 namespace intdiv {
 
+// The bits of a double, by a move that the compiler does not see through: it
+// turns integer tests of a double's bits (is it zero, is it finite) back into
+// floating-point ones, which occupy the FP64 pipe (two instructions each: with
+// them the step above took 8.88 ms).
 FGB_HD uint64_t to_bits(double x) {
 #ifdef __CUDA_ARCH__
-  return (uint64_t)__double_as_longlong(x);
+  uint64_t u;
+  asm("mov.b64 %0, %1;" : "=l"(u) : "d"(x));
+  return u;
 #else
   uint64_t u;
   std::memcpy(&u, &x, 8);
@@ -54,6 +60,7 @@ FGB_HD double from_bits(uint64_t u) {
   return x;
 #endif
 }
+FGB_HD int max_of(int a, int b) { return a > b ? a : b; }
 FGB_HD uint32_t mulhi32(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
 FGB_HD uint64_t mulhi64(uint64_t a, uint64_t b) {
 #ifdef __CUDA_ARCH__
@@ -71,6 +78,31 @@ FGB_HD float rcp32(float f) {
 #else
   return FGB_HOST_RCP32(f);
 #endif
+}
+
+// The floating-point expressions behind the integer paths are rarely taken and
+// must stay behind a branch: predicated into the common path, as the compiler
+// does with a few instructions even of a function that is not inlined, they
+// occupy the FP64 pipe there all the same. A loop is not predicated; this one
+// runs once (a lane index is below 32), which the compiler does not know
+// (512^2 x 48, 2 tracers: step 7.73 ms, without the loop 7.82).
+FGB_HD uint32_t one_turn() {
+#ifdef __CUDA_ARCH__
+  uint32_t lane;
+  asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
+  return (lane >> 5) + 1;
+#else
+  return 1;
+#endif
+}
+template <typename T, typename F>
+FGB_HD T behind_branch(F f) {
+  T r;
+  uint32_t n = one_turn();
+  do {
+    r = f();
+  } while (--n);
+  return r;
 }
 
 FGB_COLD double hw_div(double a, double b) { return a / b; }
@@ -143,6 +175,39 @@ FGB_HD double divide(double a, const Divisor& d) {
 }
 
 FGB_HD double divide(double a, double b) { return divide(a, prepare(b)); }
+
+// a * b, rounded to nearest even, for kernels whose FP64 pipe is the bound
+// while the integer pipe has room (some 35 integer instructions): gradients,
+// volume fluxes and MUSCL increments with some of their products here 3.7 ms
+// against 4.5 for 512^2 x 48, 2 tracers.
+FGB_COLD double hw_mul(double a, double b) {
+  return behind_branch<double>([&] { return a * b; });
+}
+// What the truncated product leaves open: the exact product's high half, rounded with its low
+// half as the tie breaker.
+FGB_COLD uint64_t round_product(uint64_t A, uint64_t B, uint32_t sh) {
+  const uint64_t hi = mulhi64(A, B), R = (hi + (1ull << (sh - 1))) >> sh;
+  const bool tie = (hi << (64 - sh)) == (1ull << 63) && A * B == 0;
+  return tie ? R & ~1ull : R;
+}
+FGB_HD double multiply(double a, double b) {
+  const uint64_t ua = to_bits(a), ub = to_bits(b), A = significand(ua), B = significand(ub);
+  const int ea = (int)(ua >> 52) & 0x7ff, eb = (int)(ub >> 52) & 0x7ff;
+  // the product of the significands / 2^64, in [2^62, 2^64), low by less than 3 units (dropped parts)
+  const uint32_t Ahi = (uint32_t)(A >> 32), Alo = (uint32_t)A, Bhi = (uint32_t)(B >> 32), Blo = (uint32_t)B;
+  const uint64_t Q = (uint64_t)Ahi * Bhi + mulhi32(Ahi, Blo) + mulhi32(Alo, Bhi);
+  const uint32_t big = (uint32_t)(Q >> 63), sh = 10 + big;
+  const int e = ea + eb - 1024 + (int)big;  // the exponent field less one
+  if ((unsigned)(ea - 1) >= 2046u || (unsigned)(eb - 1) >= 2046u || (unsigned)e >= 2045u) {
+    if (((ua << 1) == 0 || (ub << 1) == 0) && max_of(ea, eb) < 2047) return from_bits((ua ^ ub) & (1ull << 63));
+    return hw_mul(a, b);
+  }
+  const uint64_t t = Q + (512u << big);
+  uint64_t R = t >> sh;
+  // up to 3 units below a rounding boundary, or on it (a tie)
+  if (((uint32_t)t << (32 - sh)) + (3u << (32 - sh)) < (4u << (32 - sh))) R = round_product(A, B, sh);
+  return from_bits((((uint64_t)(uint32_t)e << 52) + R) | ((ua ^ ub) & (1ull << 63)));
+}
 
 }  // namespace intdiv
 }  // namespace fgb

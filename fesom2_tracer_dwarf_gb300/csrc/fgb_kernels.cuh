@@ -60,6 +60,14 @@ __device__ __forceinline__ R rabs(R a) { return bits64::magnitude(a); }
 // integer pipe.
 template <typename R>
 __device__ __forceinline__ R fdiv(R a, R b) { return intdiv::divide(a, b); }
+// a * b on the integer pipe in the exact form, where a kernel keeps the FP64
+// pipe busy and the integer pipe idle (the update kernel, with more integer
+// work per FP64 instruction, slowed down: 1.85 against 1.61 ms); the fast form
+// fuses it with an addition.
+__device__ __forceinline__ double imul(double a, double b) {
+  if constexpr (FGB_FAST64) return a * b;
+  else return intdiv::multiply(a, b);
+}
 // A divisor shared by several quotients: prepared once in the exact form (the
 // fast form multiplies with reciprocals instead).
 struct LayerDivisor {
@@ -147,12 +155,12 @@ __device__ __forceinline__ double edge_vflux(const DMesh& m, const EdgeTab& q, c
   if (s1) {
     const size_t i = (size_t)q.el1 * m.LZ + k;
     const double u = vel[2 * i], w = vel[2 * i + 1];
-    v1 = (-(w * q.dX1) + u * q.dY1) * m.g64.helem[i];
+    v1 = imul(-(w * q.dX1) + imul(u, q.dY1), m.g64.helem[i]);
   }
   if (s2) {
     const size_t i = (size_t)q.el2 * m.LZ + k;
     const double u = vel[2 * i], w = vel[2 * i + 1];
-    v2 = (w * q.dX2 - u * q.dY2) * m.g64.helem[i];
+    v2 = imul(w * q.dX2 - imul(u, q.dY2), m.g64.helem[i]);
   }
   return s1 && s2 ? v1 + v2 : (s1 ? v1 : v2);
 }
@@ -204,7 +212,7 @@ __global__ void __launch_bounds__(kEdgeThreads) k_elem_grad(DMesh m, StepPtrs<R>
     for (int t = 0; t < a.K; ++t) {
       const R* __restrict__ T = a.TA + t * a.sTA + k;
       const R ta = T[na * LZ], tb = T[nb * LZ], tc = T[nc * LZ];
-      out[((size_t)t * m.M + el) * LZ + k] = make_double2(x0 * ta + x1 * tb + x2 * tc, y0 * ta + y1 * tb + y2 * tc);
+      out[((size_t)t * m.M + el) * LZ + k] = make_double2(x0 * ta + imul(x1, tb) + imul(x2, tc), y0 * ta + imul(y1, tb) + imul(y2, tc));
     }
   }
 }
@@ -257,12 +265,12 @@ __device__ __forceinline__ void node_mean_grad(const DMesh& m, const double* __r
 // pipe. 512^2 x 48, 2 tracers: volume fluxes, gradients and edge fluxes 4.4 ms
 // together against 10.9.
 // ---------------------------------------------------------------------------
-// The slow forms behind it, out of line (see bits64): the reconstruction's mask as a
-// product where a value is infinite or NaN, and the flux for any ph.
-static __device__ __noinline__ double hw_product(double a, double b) { return a * b; }
+// The flux for any ph and for infinite and NaN values.
 static __device__ __noinline__ double hor_flux_any(double v, double Tm1, double Tm2, double ph) {
-  const double cHO = (v + fabs(v)) * Tm1 + (v - fabs(v)) * Tm2;
-  return -((0.5 * (1.0 - ph)) * cHO) - ((v * ph) * 0.5) * (Tm1 + Tm2);
+  return intdiv::behind_branch<double>([&] {
+    const double cHO = (v + fabs(v)) * Tm1 + (v - fabs(v)) * Tm2;
+    return -((0.5 * (1.0 - ph)) * cHO) - ((v * ph) * 0.5) * (Tm1 + Tm2);
+  });
 }
 
 // The flux of edge q at layer k, all tracers. MEAN: outside the triangles' window (or without
@@ -279,7 +287,7 @@ __device__ __forceinline__ void hor_flux(const DMesh& m, const StepPtrs<double>&
   } else {
     v = a.vf[ek];
   }
-  const double B = bits64::half(ph1 ? v : v * a.ph);
+  const double B = bits64::half(ph1 ? v : intdiv::hw_mul(v, a.ph));
   const bool c1 = HOR == 2 || q.nb1 > k, c2 = HOR == 2 || q.nb2 > k;
   const size_t i1 = q.n1 * LZ + k, i2 = q.n2 * LZ + k;
   for (int t = 0; t < a.K; ++t) {
@@ -302,14 +310,14 @@ __device__ __forceinline__ void hor_flux(const DMesh& m, const StepPtrs<double>&
         grad_at<GRAD>(m, TA, G, q.dn, k, g2, g4);
       }
       const double d2 = bits64::twice(s2 - s1);
-      double r1 = sixth(d2 + q.ex * g1 + q.ey * g3), r2 = sixth(d2 + q.ex * g2 + q.ey * g4);
+      double r1 = sixth(d2 + imul(q.ex, g1) + imul(q.ey, g3)), r2 = sixth(d2 + imul(q.ex, g2) + imul(q.ey, g4));
       if (HOR == 1 && !(c1 && c2)) {
         if (bits64::finite(r1, r2)) {
           r1 = c1 ? r1 : 0.0;
           r2 = c2 ? r2 : 0.0;
         } else {
-          r1 = hw_product(r1, c1 ? 1.0 : 0.0);
-          r2 = hw_product(r2, c2 ? 1.0 : 0.0);
+          r1 = intdiv::hw_mul(r1, c1 ? 1.0 : 0.0);
+          r2 = intdiv::hw_mul(r2, c2 ? 1.0 : 0.0);
         }
       }
       const double Tm1 = s1 + r1, Tm2 = s2 - r2;
@@ -325,7 +333,7 @@ __device__ __forceinline__ void hor_flux(const DMesh& m, const StepPtrs<double>&
 // window, those with mean gradients (some eight times the work: mixed into the first list, a
 // single one held its whole warp), and those below the edge, which are zero.
 template <typename R, int HOR, bool FCT, bool VF, bool GRAD>
-__global__ void __launch_bounds__(kEdgeThreads, 3) k_hflux(DMesh m, StepPtrs<R> a, const double2* __restrict__ grad) {
+__global__ void __launch_bounds__(kEdgeThreads, 4) k_hflux(DMesh m, StepPtrs<R> a, const double2* __restrict__ grad) {
   __shared__ EdgeTab tab[kEdgeTile];
   __shared__ int win[kEdgeTile][2];         // the window's layers [first, end) per edge (0-based)
   __shared__ int ptr[3][kEdgeTile + 1];     // starts of the edges' parts of the three lists
@@ -461,12 +469,16 @@ struct Column {
 // ---------------------------------------------------------------------------
 // The expressions of infinite and NaN values and of any num_ord, out of line.
 static __device__ __noinline__ double qr4c_any(double W, double tm1, double tm2, double num_ord, double A) {
-  const double tm = (W + fabs(W)) * tm1 + (W - fabs(W)) * tm2;
-  return (-((0.5 * (1.0 - num_ord)) * tm) - (num_ord * (0.5 * (tm1 + tm2))) * W) * A;
+  return intdiv::behind_branch<double>([&] {
+    const double tm = (W + fabs(W)) * tm1 + (W - fabs(W)) * tm2;
+    return (-((0.5 * (1.0 - num_ord)) * tm) - (num_ord * (0.5 * (tm1 + tm2))) * W) * A;
+  });
 }
 static __device__ __noinline__ double hw_ppm_bottom(double Tu, double Tl, double W) {
-  const double s = copysign(1.0, W);
-  return -(Tu * (s < 0.0 ? s : 0.0)) + Tl * (s > 0.0 ? s : 0.0);
+  return intdiv::behind_branch<double>([&] {
+    const double s = copysign(1.0, W);
+    return -(Tu * (s < 0.0 ? s : 0.0)) + Tl * (s > 0.0 ? s : 0.0);
+  });
 }
 
 // What a vertical scheme needs of a column's geometry, for all its tracers.
@@ -595,8 +607,8 @@ __device__ __forceinline__ void ver_prepare(const VerGeo<VER>& g, const Column& 
 __device__ __forceinline__ double ver_upw1(const double* T, int i, int k0, double W, double A) {
   const double T0 = T[i], Tu = i == k0 ? T0 : T[i - 1];
   double x = bits64::upwind(W, T0, Tu);
-  if (i == k0 && !bits64::finite(T0, W)) x = hw_product(W, T0);  // the surface: W T as written
-  return -(x * A);
+  if (i == k0 && !bits64::finite(T0, W)) x = intdiv::hw_mul(W, T0);  // the surface: W T as written
+  return -imul(x, A);
 }
 
 // The flux of a layer's parabola through one of its interfaces (:598-632) for
@@ -604,7 +616,7 @@ __device__ __forceinline__ double ver_upw1(const double* T, int i, int k0, doubl
 __device__ __forceinline__ double ppm_layer(double aL, double aR, double T0, double hx, double cx, bool upper, double A,
                                             double W) {
   if (!bits64::product_positive(aR - T0, T0 - aL) &&
-      ((bits64::finite(aR, aL) && bits64::finite(T0)) || hw_product(aR - T0, T0 - aL) <= 0.0)) {
+      ((bits64::finite(aR, aL) && bits64::finite(T0)) || intdiv::hw_mul(aR - T0, T0 - aL) <= 0.0)) {
     aL = T0;
     aR = T0;
   }
@@ -640,11 +652,11 @@ __device__ __forceinline__ double ver_flux(const VerGeo<VER>& g, const Column& c
     double x = Tu, y = T0;
     if (mid) {
       const double q2 = bits64::twice(S[i]);
-      y = T0 + third((q2 + S[i + 1]) * g.at(g.A1, i));
-      x = Tu + third((q2 + S[i - 1]) * g.at(g.A2, i));
+      y = T0 + third(imul(q2 + S[i + 1], g.at(g.A1, i)));
+      x = Tu + third(imul(q2 + S[i - 1], g.at(g.A2, i)));
     }
     const double mean = i == c.k0 ? T0 : bits64::half(x + y);
-    double ho = -((mean * W) * A);
+    double ho = -imul(mean * W, A);
     // num_ord = 1: the upwind part is an exact zero (of finite values)
     if (mid && !(num_ord == 1.0 && bits64::finite(x, y) && bits64::finite(W))) ho = qr4c_any(W, y, x, num_ord, A);
     const double f = ho - f0;
@@ -729,7 +741,7 @@ __global__ void __launch_bounds__(128, 6) k_fct_lo(DMesh m, StepPtrs<R> a, int k
       if constexpr (FGB_FAST64) {
         l = (tn * hn + (acc + dF) * rdt_vol(dt, av)) * fdiv(R(1), hnn);
       } else {
-        l = fdiv(tn * hn + fdiv((acc + dF) * dt, av), hnn);
+        l = fdiv(imul(tn, hn) + fdiv(imul(acc + dF, dt), av), hnn);
       }
       a.lo[(t0 + t) * a.sN + c.iz + k] = l;
     }

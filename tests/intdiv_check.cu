@@ -1,4 +1,4 @@
-// Compares intdiv::divide (and, on the device, the helpers of bits64) with the
+// Compares intdiv::divide and multiply (and, on the device, the helpers of bits64) with the
 // floating-point hardware: random operands, quotients next to midpoints, extreme
 // significands and exponents, special values. Compiled as C++ it checks the host
 // build and prints the number of differing results; compiled by nvcc into a
@@ -82,7 +82,8 @@ static __global__ void k_check(int n, unsigned long long seed, unsigned long lon
   for (int i = 0; i < n; ++i) {
     double a, b;
     operands(i & 7, s, a, b);
-    int d = !same(divide(a, b), a / b, true);
+    int d = !same(divide(a, b), a / b, true) + !same(multiply(a, b), a * b, true);
+    d += !same(multiply(a, from_bits(to_bits(b) & ~((1ull << 27) - 1))), a * from_bits(to_bits(b) & ~((1ull << 27) - 1)), true);
     d += !same(B::lesser(a, b), a < b ? a : b, false) + !same(B::greater(a, b), a > b ? a : b, false);
     d += !same(B::twice(a), a + a, true) + !same(B::half(a), a * 0.5, true) + !same(B::magnitude(a), fabs(a), true);
     if (d) atomicAdd(bad, (unsigned long long)d);
@@ -104,7 +105,12 @@ int main(int argc, char** argv) {
   for (long long i = 0; i < n; ++i) {
     double a, b;
     operands((int)(i & 7), s, a, b);
-    bad += !same(divide(a, b), a / b, true);
+    bad += !same(divide(a, b), a / b, true) + !same(multiply(a, b), a * b, true);
+    // short significands: exact products and ties
+    for (int cut = 20; cut < 32; cut += 3) {
+      const double x = from_bits(to_bits(a) >> cut << cut), y = from_bits(to_bits(b) >> (53 - cut) << (53 - cut));
+      bad += !same(multiply(x, y), x * y, true);
+    }
   }
   std::printf("%lld\n", bad);
   return bad != 0;

@@ -1,4 +1,4 @@
-"""The FP64 division and comparisons on the integer pipe (csrc/fgb_intdiv.cuh,
+"""The FP64 division, multiplication and comparisons on the integer pipe (csrc/fgb_intdiv.cuh,
 fgb_bits.cuh) give the hardware's results bit for bit: on the host build with
 the reciprocal estimate as it is and pushed off by a unit either way, and on the
 GPU."""
