@@ -194,6 +194,23 @@ __device__ __forceinline__ void two_sum(V<KV>& s, V<KV>& c, const V<KV>& x) {
   c = add(c, e);
 }
 
+// The pointers of tracer group gi alone. The kernels named ..._g take the group
+// from blockIdx.y instead of their own loop: on a mesh of less than a wave of
+// warps a group's work in turn only adds to the latency (see by_group).
+__device__ __forceinline__ FastPtrs group_of(FastPtrs a, int gi) {
+  a.T += gi * a.gT;
+  a.TA += gi * a.gTA;
+  if (a.TAout) a.TAout += gi * a.gTA;
+  a.adfh += gi * a.gE;
+  a.lo += gi * a.gN;
+  a.adfv += gi * a.gW;
+  a.rpm += 2 * gi * a.gN;
+  if (a.del) a.del += gi * a.gN;
+  if (a.Tlo) a.Tlo += gi * a.gT;
+  a.G = 1;
+  return a;
+}
+
 // Division by the fast single-precision reciprocal (about 2 ulp); the FP32
 // form's bar is a tolerance against FP64, not bit parity.
 __device__ __forceinline__ float fdv(float a, float b) { return __fdividef(a, b); }
@@ -1256,7 +1273,7 @@ __host__ __device__ constexpr size_t ratio64_warp_bytes(int KV) { return (size_t
 // COMP: the +/- sums of the antidiffusive fluxes are compensated sums.
 // Shared memory: ratio64_warp_bytes per warp, where the finished bounds wait.
 template <int KV, bool LEAN, bool COMP>
-__global__ void __launch_bounds__(128, LEAN ? 8 : 7) kf_ratio64(DMesh m, FastPtrs a) {
+__device__ __forceinline__ void ratio64_column(const DMesh& m, const FastPtrs& a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kW - 1);
   const int vi = blockIdx.x * (blockDim.x / kW) + threadIdx.x / kW;
@@ -1422,6 +1439,15 @@ __global__ void __launch_bounds__(128, LEAN ? 8 : 7) kf_ratio64(DMesh m, FastPtr
     }
   }
 }
+template <int KV, bool LEAN, bool COMP>
+__global__ void __launch_bounds__(128, LEAN ? 8 : 7) kf_ratio64(DMesh m, FastPtrs a) {
+  ratio64_column<KV, LEAN, COMP>(m, a);
+}
+template <int KV, bool LEAN, bool COMP>
+__global__ void __launch_bounds__(128) kf_ratio64_g(DMesh m, FastPtrs a) {
+  ratio64_column<KV, LEAN, COMP>(m, group_of(a, blockIdx.y));
+}
+
 
 // ---------------------------------------------------------------------------
 // FCT stage 3: limiting b3 (lib/oce_adv_tra_fct.F90:396-471), flux divergence
@@ -1661,6 +1687,7 @@ __global__ void __launch_bounds__(128, (NS == 1 ? (COMP || RES ? 8 : 9) : 4)) kf
     __syncwarp();
   }
 }
+
 
 // ---------------------------------------------------------------------------
 // Without a limiter: vertical HO flux on T_AB with w_e, flux divergence and

@@ -16,6 +16,18 @@ inline void allow_smem_f(F* kernel, size_t bytes) {
   if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Several groups of one or two tracers on less than a wave of columns (152 SMs
+// of 28 warps): the edge fluxes and the limiting factors take a block per
+// group (48x40x30, 3 tracers: 18.4 against 20.4 us and 10.2 against 12.6). On
+// larger meshes a warp's tables serve its groups in turn. The LO and update
+// kernels keep their loop: written as a function of two kernels they lose more
+// on large meshes (update 344 -> 352 us on the 188,661-node pi mesh, LO 2.01 ->
+// 2.03 ms at 1024^2x64) than the 1 to 2 us that they would gain.
+template <int KV>
+bool by_group(const DMesh& m, const FastPtrs& a) {
+  return KV <= 2 && a.G > 1 && m.N <= 152 * 28;
+}
+
 template <int KV, int HOR, int NS>
 void launch_hflux_f(const DMesh& m, const FastPtrs& a, bool fct, int ew, cudaStream_t s) {
   const int per_block = ew * kW;  // edges per block: 32 per warp
@@ -28,8 +40,16 @@ void launch_hflux_f(const DMesh& m, const FastPtrs& a, bool fct, int ew, cudaStr
 template <int KV, int HOR, bool FCT>
 void launch_hflux_tile(const DMesh& m, const FastPtrs& a, cudaStream_t s) {
   const size_t sm = tile_smem_bytes(KV, FCT && a.TA != a.T, m.tile_max_nodes);
-  allow_smem_f(kf_hflux_tile<HOR, FCT, KV>, sm);
-  kf_hflux_tile<HOR, FCT, KV><<<m.ntiles, kTileThreads, sm, s>>>(m, a);
+  auto go = [&](auto* kernel, unsigned groups) {
+    allow_smem_f(kernel, sm);
+    kernel<<<dim3(m.ntiles, groups), kTileThreads, sm, s>>>(m, a);
+  };
+  if constexpr (KV <= 2) {
+    if (by_group<KV>(m, a)) go(kf_hflux_tile_g<HOR, FCT, KV>, a.G);
+    else go(kf_hflux_tile<HOR, FCT, KV>, 1);
+  } else {
+    go(kf_hflux_tile<HOR, FCT, KV>, 1);
+  }
   if constexpr (HOR != 0) {
     constexpr int runs = kTileThreads / (2 * kMeanRun);
     if (m.nmean > 0)
@@ -109,10 +129,17 @@ void launch_update_f(const DMesh& m, const FastPtrs& a, int nw, cudaStream_t s) 
 
 template <int KV, bool LEAN>
 void launch_ratio64(const DMesh& m, const FastPtrs& a, int nw, cudaStream_t s) {
-  const unsigned grid = (m.N + nw - 1) / nw;
   const size_t sm = nw * ratio64_warp_bytes(KV);
-  if (a.comp & 4) kf_ratio64<KV, LEAN, true><<<grid, nw * kW, sm, s>>>(m, a);
-  else kf_ratio64<KV, LEAN, false><<<grid, nw * kW, sm, s>>>(m, a);
+  auto go = [&](auto* kernel, unsigned groups) { kernel<<<dim3((m.N + nw - 1) / nw, groups), nw * kW, sm, s>>>(m, a); };
+  if constexpr (KV <= 2 && !LEAN) {
+    if (by_group<KV>(m, a)) {
+      if (a.comp & 4) go(kf_ratio64_g<KV, LEAN, true>, a.G);
+      else go(kf_ratio64_g<KV, LEAN, false>, a.G);
+      return;
+    }
+  }
+  if (a.comp & 4) go(kf_ratio64<KV, LEAN, true>, 1);
+  else go(kf_ratio64<KV, LEAN, false>, 1);
 }
 
 template <int KV, int VER, bool TASEP, bool WESEP, bool COMP>

@@ -60,7 +60,7 @@ __device__ __forceinline__ V<KV> tile_flux(const V<KV>& s1, const V<KV>& s2, con
 }
 
 template <int HOR, bool FCT, int KV>
-__global__ void __launch_bounds__(kTileThreads) kf_hflux_tile(DMesh m, FastPtrs a) {
+__device__ __forceinline__ void hflux_tile(const DMesh& m, const FastPtrs& a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   EdgeRec* recs = reinterpret_cast<EdgeRec*>(smem_raw);
   // row starts of n1 | n2 and of the upwind triangle's two other vertices (rsA), of
@@ -174,6 +174,15 @@ __global__ void __launch_bounds__(kTileThreads) kf_hflux_tile(DMesh m, FastPtrs 
     }
   }
 }
+template <int HOR, bool FCT, int KV>
+__global__ void __launch_bounds__(kTileThreads) kf_hflux_tile(DMesh m, FastPtrs a) {
+  hflux_tile<HOR, FCT, KV>(m, a);
+}
+template <int HOR, bool FCT, int KV>
+__global__ void __launch_bounds__(kTileThreads) kf_hflux_tile_g(DMesh m, FastPtrs a) {
+  hflux_tile<HOR, FCT, KV>(m, group_of(a, blockIdx.y));
+}
+
 
 // The edges' layers outside their triangles' window (or of edges without
 // triangles), after kf_hflux_tile: the mean gradients around both nodes. Such a
