@@ -156,7 +156,7 @@ void launch_lo64(const DMesh& m, const FastPtrs& a, cudaStream_t s) {
 
 template <int KV, int VER>
 void launch_lo_ns(const DMesh& m, const FastPtrs& a, const LaunchArgs& L, cudaStream_t s) {
-  if (L.ns_lo == 3) {  // whole column per warp (at most 64 layers, no w_split)
+  if (L.ns_lo == 3) {  // whole column per warp (at most 64 layers)
     const bool tasep = a.TA != a.T, wesep = a.we != a.w;
     if (tasep) {
       if (wesep) launch_lo64<KV, VER, true, true>(m, a, s);

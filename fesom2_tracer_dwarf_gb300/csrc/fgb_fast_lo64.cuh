@@ -241,7 +241,15 @@ __global__ void __launch_bounds__(kLo64Warps * kW, 7) kf_lo64(DMesh m, FastPtrs 
         }
       }
       sF[iz] = lo;
-      const V<KV> d = sub(ho, lo);
+      V<KV> lf = lo;
+      if (WESEP && a.wi && in && z < nzmax) {
+        // w_split: the antidiffusive flux takes the upwind flux of the full w
+        // (lib/oce_adv_tra_driver.F90:221-231)
+        const float W = w[s], A = ar[s];
+        lf = z == nzmin ? muls(t[s], -(W * A))
+                        : fmas(Tup, -0.5f * (W - fabsf(W)) * A, muls(t[s], -0.5f * (W + fabsf(W)) * A));
+      }
+      const V<KV> d = sub(ho, lf);
       if (iz < nl) st<KV>(adfv, (unsigned)n * LW + iz, twice ? sub(ho, d) : d);
     }
     if (lane == 0 && nl - 1 >= 2 * kW) {  // the bottom interface of 65-interface columns

@@ -103,9 +103,16 @@ int launch_stages_f32(const DMesh& m, const fgb_step_desc& d, int mask, cudaStre
   L.nw_upd = pick(d.cfg[3], 1, 2, 4, 4);
   auto ns = [](int want, int def) { return (want == 1 || want == 2) ? want : def; };
   L.ns_h = ns(d.cfg[7], 2);
-  // LO: 3 (the default where it applies) the whole-column kernel for columns
-  // of at most 64 layers without w_split; 1 or 2 layers per lane per pass
-  L.ns_lo = (d.cfg[4] == 1 || d.cfg[4] == 2) ? d.cfg[4] : (m.LZ <= 64 && !(d.lim == FGB_LIM_FCT && d.wi) ? 3 : 2);
+  // LO: 3 (the default where it applies) the whole-column kernel for columns of
+  // at most 64 layers; 1 or 2 layers per lane per pass. Under w_split the
+  // whole-column kernel leaves the implicit step to a second kernel
+  // (kf_vert_pcr), the two-layer one solves it in the same pass: from a wave of
+  // columns on (152 SMs of 28 warps) the two kernels are faster (256^2x64: 146
+  // / 150 us for one tracer, 205 / 213 for four, 323 / 379 for eight; closed
+  // 200^2x47, two tracers, 96 / 109), below it the second launch costs more
+  // (48^2x47, four tracers, 17.2 / 14.6).
+  const bool whole = m.LZ <= 64 && (!wsplit || m.N > 152 * 28 || d.cfg[4] == 3);
+  L.ns_lo = (d.cfg[4] == 1 || d.cfg[4] == 2) ? d.cfg[4] : (whole ? 3 : 2);
   // ratio: 1 or 2 layers per lane with shared-memory staging, or 3 (the default)
   // the whole column per warp without shared memory
   L.ns_ratio = (d.cfg[5] >= 1 && d.cfg[5] <= 4) ? d.cfg[5] : 0;

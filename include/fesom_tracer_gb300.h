@@ -258,10 +258,12 @@ typedef struct {
    * cfg[1..3]  warps (node columns) per block of the LO, ratio and update
    *            kernels: 1, 2, 4 (default 4)
    * cfg[4..6]  FP64 form: tracers per chunk of the same three kernels: 1, 2,
-   *            4, used when it divides ntracers (default: the largest of 4, 2,
-   *            1 that does). FP32 form (one tracer group at a time): layers
+   *            4, used when it divides ntracers (default: up to 4, as many as
+   *            the shared memory has room for). FP32 form (one tracer group at a time): layers
    *            per lane per pass, 1 or 2 with the column staged in shared
-   *            memory (defaults: LO 2, update 1), or for the ratio kernel
+   *            memory (update: default 1), for the LO kernel 3 the whole column
+   *            per warp (columns of at most 64 layers; its default, under
+   *            w_split on meshes of more than 4256 columns), or for the ratio kernel
    *            3 (its default) / 4 without shared memory, 4 with fewer
    *            registers (columns of at most 64 layers).
    * cfg[7]     FP32 form: layers per lane per pass of the per-edge edge-flux
