@@ -680,9 +680,13 @@ __device__ __forceinline__ double ver_flux(const VerGeo<VER>& g, const Column& c
 // horizontal edge fluxes are formed here from T and the edge volume fluxes,
 // with the expression adv_tra_hor_upw1 uses (lib/oce_adv_tra_hor.F90:218-220).
 // kc: tracers per chunk.
+// Blocks per SM: QR4C keeps its values in 72 registers without a spill and the
+// seventh block covers gather latency (512^2x48, 2 tracers, whole step 7694 ->
+// 7603 us); PPM loses more to the tighter allocation than it gains (321^2 basin,
+// fast form, 4530 -> 4555 us), so the other schemes stay at six.
 // ---------------------------------------------------------------------------
 template <typename R, int VER>
-__global__ void __launch_bounds__(128, 6) k_fct_lo(DMesh m, StepPtrs<R> a, int kc_max) {
+__global__ void __launch_bounds__(128, VER == 1 ? 7 : 6) k_fct_lo(DMesh m, StepPtrs<R> a, int kc_max) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kWarp - 1), wib = threadIdx.x / kWarp;
   const int vi = blockIdx.x * (blockDim.x / kWarp) + wib;
@@ -922,9 +926,12 @@ __device__ __forceinline__ void store_ab_below(const DMesh& m, const StepPtrs<R>
 // and the caller's tendency update (src/fesom_analytic.F90:419-437 or, with a
 // persistent del_ttf, lib/tracer_c_interface.F90:194-214). The limiting
 // factors are at most 1 (or NaN), so the reference's min(1, a, b) is min(a, b).
+// Seven blocks per SM: 72 registers (77 with six blocks, 36 % of the warps in
+// flight, gathers as long a wait as the FP64 pipe) still hold everything; the
+// 512^2x48 step with 2 tracers 7785 -> 7694 us. Eight (64) would spill.
 // ---------------------------------------------------------------------------
 template <typename R>
-__global__ void __launch_bounds__(128, 6) k_fct_update(DMesh m, StepPtrs<R> a, int kc_max) {
+__global__ void __launch_bounds__(128, 7) k_fct_update(DMesh m, StepPtrs<R> a, int kc_max) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kWarp - 1), wib = threadIdx.x / kWarp;
   const int vi = blockIdx.x * (blockDim.x / kWarp) + wib;
