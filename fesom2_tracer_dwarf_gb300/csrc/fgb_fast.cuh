@@ -362,7 +362,9 @@ static __global__ void __launch_bounds__(kVfluxThreads) kf_vflux4(DMesh m, const
 // gradient of the elements around each node (lib/oce_muscl_adv.F90:393-410).
 // ---------------------------------------------------------------------------
 // Three elements at a time: their index, table and value loads are in flight
-// together (an element that is not there or dry at the layer has weight zero).
+// together. An element that is not there or dry at the layer adds a gradient
+// of zero with weight zero: its vertices' values may be anything, a NaN fill
+// too, so they are deselected and not only weighted.
 template <int KV>
 __device__ __forceinline__ void node_grad(const DMesh& m, const float* __restrict__ TA, int n, unsigned k,
                                           V<KV>& gx, V<KV>& gy) {
@@ -381,9 +383,10 @@ __device__ __forceinline__ void node_grad(const DMesh& m, const float* __restric
       const int a = m.elem_nodes[3 * el], b = m.elem_nodes[3 * el + 1], c = m.elem_nodes[3 * el + 2];
       const float* gs = g.grad_sca + 6 * (size_t)el;
       const V<KV> ta = ld<KV>(TA, a * LZ + k), tb = ld<KV>(TA, b * LZ + k), tc = ld<KV>(TA, c * LZ + k);
-      ex[u] = fmas(tc, gs[2], fmas(tb, gs[1], muls(ta, gs[0])));
-      ey[u] = fmas(tc, gs[5], fmas(tb, gs[4], muls(ta, gs[3])));
-      ar[u] = j + u < end && m.elem_nlev[el] - 1 >= z ? g.elem_area[el] : 0.f;
+      const bool wet = j + u < end && m.elem_nlev[el] - 1 >= z;
+      ex[u] = wet ? fmas(tc, gs[2], fmas(tb, gs[1], muls(ta, gs[0]))) : splat<KV>(0.f);
+      ey[u] = wet ? fmas(tc, gs[5], fmas(tb, gs[4], muls(ta, gs[3]))) : splat<KV>(0.f);
+      ar[u] = wet ? g.elem_area[el] : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < 3; ++u) {
