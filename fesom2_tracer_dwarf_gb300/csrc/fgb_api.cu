@@ -348,16 +348,15 @@ int fgb_mesh_create(const fgb_hmesh* hm, fgb_mesh** out) {
   for (int p = 0; p < h.E; ++p) {
     const int e = h.edge_order[p];
     const int hi = std::max(h.edge_lev[4 * (size_t)e + 1], h.edge_lev[4 * (size_t)e + 3]);
-    const int gm0 = h.edge_gm[2 * (size_t)e], gm1 = h.edge_gm[2 * (size_t)e + 1];
+    const TriangleWindow w = triangle_window(h.edge_gm[2 * (size_t)e], h.edge_gm[2 * (size_t)e + 1], hi);
     auto runs = [&](int from, int to) {
       for (int k = from; k < to; k += fgb::fast::kMeanRun) {
         mean_seg.push_back(e);
         mean_seg.push_back(k | std::min(fgb::fast::kMeanRun, to - k) << 16);
       }
     };
-    const int w0 = gm0 < 0 ? hi : std::min(gm0 - 1, hi), w1 = gm0 < 0 ? hi : std::max(w0, std::min(gm1 - 1, hi));
-    runs(0, w0);
-    runs(w1, hi);
+    runs(0, w.first);
+    runs(w.end, hi);
   }
   d.nmean = (int)(mean_seg.size() / 2);
   bool ok = !upload(mm, mean_seg.data(), mean_seg.size(), &d.mean_seg) && !upload(mm, tile_ptr.data(), tile_ptr.size(), &d.tile_ptr) &&

@@ -3,6 +3,8 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "fgb_window.hpp"
+
 namespace fgb {
 
 // Geometry in the storage precision of a form (FP64 and FP32 copies).

@@ -344,14 +344,10 @@ __global__ void __launch_bounds__(kEdgeThreads, 4) k_hflux(DMesh m, StepPtrs<R> 
       const EdgeTab q = load_edge<HOR>(m, w0 + tid);
       tab[tid] = q;
       const int hi = max(q.nl1, q.nl2);
-      int first = 0, end = hi;
-      if (HOR != 0) {
-        first = q.gm0 < 0 ? 0 : min(q.gm0 - 1, hi);
-        end = q.gm0 < 0 ? 0 : max(first, min(q.gm1 - 1, hi));
-      }
-      win[tid][0] = first;
-      win[tid][1] = end;
-      cnt[0] = end - first;
+      const TriangleWindow w = HOR != 0 ? triangle_window(q.gm0, q.gm1, hi) : TriangleWindow{0, hi};
+      win[tid][0] = w.first;
+      win[tid][1] = w.end;
+      cnt[0] = w.end - w.first;
       cnt[1] = hi - cnt[0];
       cnt[2] = m.LZ - hi;
     }
