@@ -345,6 +345,7 @@ int fgb_mesh_create(const fgb_hmesh* hm, fgb_mesh** out) {
   }
   // The layers of the edges that take mean gradients (MUSCL/MFCT), in runs, in visit order.
   std::vector<int> mean_seg;
+  d.windows_wet = 1;
   for (int p = 0; p < h.E; ++p) {
     const int e = h.edge_order[p];
     const int hi = std::max(h.edge_lev[4 * (size_t)e + 1], h.edge_lev[4 * (size_t)e + 3]);
@@ -357,6 +358,9 @@ int fgb_mesh_create(const fgb_hmesh* hm, fgb_mesh** out) {
     };
     runs(0, w.first);
     runs(w.end, hi);
+    if (w.end > w.first &&
+        w.end > std::min(h.nlevels[h.edge_updn[2 * (size_t)e]], h.nlevels[h.edge_updn[2 * (size_t)e + 1]]) - 1)
+      d.windows_wet = 0;
   }
   d.nmean = (int)(mean_seg.size() / 2);
   bool ok = !upload(mm, mean_seg.data(), mean_seg.size(), &d.mean_seg) && !upload(mm, tile_ptr.data(), tile_ptr.size(), &d.tile_ptr) &&

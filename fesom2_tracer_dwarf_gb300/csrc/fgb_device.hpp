@@ -72,6 +72,9 @@ struct DMesh {
   // {edge, first layer (0-based) | layers << 16} of at most kMeanRun layers.
   int nmean;
   const int* mean_seg;
+  // Every window lies within the layers of its edge's two triangles, so that an
+  // array of the wet layers' element gradients holds all that the windows read.
+  int windows_wet;
   GeoPtrs<double> g64;
   GeoPtrs<float> g32;
 };

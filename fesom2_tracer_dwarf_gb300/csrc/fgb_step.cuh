@@ -173,10 +173,12 @@ int launch_stages(const DMesh& m, const fgb_step_desc& d, int mask, cudaStream_t
     // flux and limiting-factor arrays (consecutive in the workspace), when this
     // call writes those afterwards or no stage reads them, and they fit (two
     // elements per node at most, as in any triangulation of the plane or torus).
+    // They hold wet layers only: level tables with windows below a triangle (a
+    // restart record may have some) take each edge's gradients from its values.
     const long long room = wl.total - wl.off[3], need = (long long)K * m.M * m.LZ * 2 * (long long)sizeof(R);
     const int later = FGB_STAGE_LO | FGB_STAGE_RATIO;
     double2* grad = nullptr;
-    if (d.hor != FGB_HOR_UPW1 && need <= room && (!fct || (mask & later) == later)) {
+    if (d.hor != FGB_HOR_UPW1 && m.windows_wet && need <= room && (!fct || (mask & later) == later)) {
       grad = reinterpret_cast<double2*>(ws + wl.off[3]);
       k_elem_grad<R><<<(m.M + kElemTile - 1) / kElemTile, kEdgeThreads, 0, s>>>(m, a, grad);
       ++launches;

@@ -1,7 +1,8 @@
 """Edges whose layer window of triangle gradients comes from a restart record
 that no mesh builder would write: a window that starts above the surface
-(ulevels_nod2D_max = 0) or ends there (nlevels_nod2D_min = 0). CPU: the window
-function over every small window. GPU: the step's values."""
+(ulevels_nod2D_max = 0) or ends there (nlevels_nod2D_min = 0), and one that
+reaches below its up- or downwind triangle (nlevels_nod2D_min too deep). CPU:
+the window function over every small window. GPU: the step's values."""
 import os
 import shutil
 import subprocess
@@ -11,7 +12,7 @@ import pytest
 
 from fesom2_tracer_dwarf_gb300.demo_tracer import FESOMTracerAdvection
 
-from test_restart import MESH, frame, read_record
+from test_restart import MESH, frame, parse_tracer, read_record
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "fesom2_tracer_dwarf_gb300", "csrc")
@@ -102,3 +103,29 @@ def test_windows_from_above_the_surface(tracer, tmp_path, schemes, precision):
     empty = _step(tracer, tmp_path / "d", precision)
     assert np.array_equal(_step(tracer, tmp_path / "c", precision), empty)
     assert not np.array_equal(empty, _step(tracer, tmp_path / "a", precision))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("schemes", [("MUSCL", "PPM", "FCT"), ("MFCT", "QR4C", "FCT"), ("MUSCL", "CDIFF", "NONE")])
+def test_windows_below_a_triangle(tracer, tmp_path, schemes):
+    """Shallow elements beside deep ones, and a record whose windows go on below
+    them: the gradients there come from the nodes' values, in FP64 as in FP32."""
+    nl = 12
+    _restart(tracer, tmp_path, schemes, nl)
+    path = tmp_path / "np1" / "t_mesh.0"
+    payload = read_record(path)
+    at = _offsets(payload)
+    get = lambda name, dt="<i4", s=4: np.frombuffer(payload, dt, at[name][1], at[name][0])  # noqa: E731
+    M, N = at["nlevels"][1], at["nlevels_nod2D"][1]
+    nlev = np.random.default_rng(4).integers(4, nl + 1, M).astype("<i4")
+    en = get("elem2D_nodes").reshape(M, 3) - 1
+    deepest = np.zeros(N, "<i4")
+    np.maximum.at(deepest, en.reshape(-1), np.repeat(nlev, 3))
+    _patch(path, nlevels=nlev, nlevels_nod2D=deepest, nlevels_nod2D_min=deepest)
+    tri = parse_tracer(read_record(tmp_path / "np1" / "t_tracer.0"))["work%edge_up_dn_tri"] - 1
+    edges = get("edges").reshape(-1, 2) - 1
+    both = (tri >= 0).all(axis=0)
+    assert (np.minimum(deepest[edges[both, 0]], deepest[edges[both, 1]]) > nlev[tri[:, both]].min(axis=0)).any()
+    a, b = _step(tracer, tmp_path, 0), _step(tracer, tmp_path, 1)
+    wet = np.arange(nl - 1)[:, None] < deepest[None, :] - 1
+    assert np.abs(a - b)[wet].max() <= 1e-5 * np.abs(a[wet]).max()
