@@ -351,9 +351,9 @@ int fgb_mesh_create(const fgb_hmesh* hm, fgb_mesh** out) {
     const int hi = std::max(h.edge_lev[4 * (size_t)e + 1], h.edge_lev[4 * (size_t)e + 3]);
     const TriangleWindow w = triangle_window(h.edge_gm[2 * (size_t)e], h.edge_gm[2 * (size_t)e + 1], hi);
     auto runs = [&](int from, int to) {
-      for (int k = from; k < to; k += fgb::fast::kMeanRun) {
+      for (int k = from; k < to; k += kMeanRun) {
         mean_seg.push_back(e);
-        mean_seg.push_back(k | std::min(fgb::fast::kMeanRun, to - k) << 16);
+        mean_seg.push_back(k | std::min(kMeanRun, to - k) << 16);
       }
     };
     runs(0, w.first);

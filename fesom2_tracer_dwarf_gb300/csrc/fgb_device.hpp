@@ -115,7 +115,6 @@ namespace fast {
 // 6.13 ms with tiles of 64/96, 48/72, 40/64 and 32/48 edges/nodes.
 constexpr int kTileEdges = 32;  // edges per tile of the tiled edge kernel
 constexpr int kTileNodes = 48;  // distinct nodes per tile
-constexpr int kMeanRun = 8;     // layers per run of DMesh::mean_seg
 
 // Pointers of one launch. Group g of a per-tracer array starts at
 // base + g * stride (floats); offsets inside a group are in units of KV floats.

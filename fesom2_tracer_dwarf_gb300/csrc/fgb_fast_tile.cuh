@@ -196,9 +196,9 @@ __global__ void __launch_bounds__(kTileThreads) kf_hflux_tile_g(DMesh m, FastPtr
 // 370 / 476; 48x40x30, 3 tracers (its seam) 20 / 35.
 template <int HOR, bool FCT, int KV>
 __global__ void __launch_bounds__(kTileThreads) kf_hflux_mean(DMesh m, FastPtrs a) {
-  const int i = (blockIdx.x * kTileThreads + threadIdx.x) / 2, side = threadIdx.x & 1;
-  const int2 seg = i / kMeanRun < m.nmean ? reinterpret_cast<const int2*>(m.mean_seg)[i / kMeanRun] : make_int2(0, 0);
-  const int l = i % kMeanRun;
+  const MeanItem it = mean_item(blockIdx.x, kTileThreads, threadIdx.x);
+  const int2 seg = it.run < m.nmean ? reinterpret_cast<const int2*>(m.mean_seg)[it.run] : make_int2(0, 0);
+  const int l = it.layer, side = it.side;
   const bool act = l < (seg.y >> 16);
   const int e = seg.x, n1 = m.edge_nodes[2 * e], n2 = m.edge_nodes[2 * e + 1];
   const unsigned LZ = m.LZ, k = (unsigned)(seg.y & 0xffff) + (act ? l : 0);

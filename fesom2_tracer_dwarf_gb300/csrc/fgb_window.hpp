@@ -1,4 +1,5 @@
-// Layer windows of the MUSCL/MFCT edges (host and device, no CUDA header).
+// Layer windows of the MUSCL/MFCT edges and work items of their mean-gradient
+// layers (host and device, no CUDA header).
 #pragma once
 #ifdef __CUDACC__
 #define FGB_HOST_DEVICE __host__ __device__ inline
@@ -20,6 +21,19 @@ FGB_HOST_DEVICE TriangleWindow triangle_window(int gm0, int gm1, int hi) {
   auto below = [hi](int z) { return (z < 1 ? 1 : (z <= hi ? z : hi + 1)) - 1; };  // layers above layer z
   const int first = gm0 < 0 ? hi : below(gm0), end = gm0 < 0 ? hi : below(gm1);
   return TriangleWindow{first, end > first ? end : first};
+}
+
+// Work item of a thread of the mean-gradient kernel: two threads (one per node)
+// for each of the kMeanRun layers of a run. The run's index is formed from the
+// block's, so that it does not overflow for any list that int can count (a
+// thread index over the whole grid wrapped at 2^28 runs).
+constexpr int kMeanRun = 8;  // layers per run of DMesh::mean_seg
+struct MeanItem {
+  int run, layer, side;
+};
+FGB_HOST_DEVICE MeanItem mean_item(unsigned block, unsigned threads, unsigned thread) {
+  return MeanItem{(int)(block * (threads / (2 * kMeanRun)) + thread / (2 * kMeanRun)), (int)(thread / 2 % kMeanRun),
+                  (int)(thread & 1)};
 }
 
 }  // namespace fgb
