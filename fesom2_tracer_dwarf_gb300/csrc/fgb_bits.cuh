@@ -32,6 +32,9 @@ __device__ __forceinline__ unsigned mag_hi(double x) { return (unsigned)(to_bits
 // Neither infinite nor NaN.
 __device__ __forceinline__ bool finite(double x) { return mag_hi(x) < 0x7ff00000u; }
 __device__ __forceinline__ bool finite(double x, double y) { return max(mag_hi(x), mag_hi(y)) < 0x7ff00000u; }
+// Below 2^511 in magnitude (so not a NaN): twice the product of two such numbers is finite.
+__device__ __forceinline__ bool moderate(double x) { return mag_hi(x) < 0x5fe00000u; }
+__device__ __forceinline__ bool moderate(double x, double y) { return max(mag_hi(x), mag_hi(y)) < 0x5fe00000u; }
 
 // The floating-point expressions behind the integer ones (see one_turn).
 using intdiv::behind_branch;
@@ -87,13 +90,19 @@ __device__ __forceinline__ double half(double x) {
 
 // (t1 (v + |v|) + t2 (v - |v|)) / 2, the upwind product of a first-order flux:
 // one factor in brackets is zero and the other 2 v, so it is v times the
-// upwind value, one FP64 instruction (the same bits unless the product is
-// subnormal). Infinities, NaNs and numbers whose double overflows by the
-// expression as written.
-__device__ __forceinline__ double upwind(double v, double t1, double t2) {
-  if (max(mag_hi(v), max(mag_hi(t1), mag_hi(t2))) >= 0x7fe00000u)
-    return hw_upwind(v, t1, t2);
-  return (sign_clear(v) ? t1 : t2) * v;
+// upwind value, one FP64 instruction. Where that is not the expression's value
+// bit for bit (a subnormal product, whose double rounds first; a double that
+// overflows; infinities and NaNs) the expression as written, or with `plain`
+// v * t1 (the surface flux, t1 = t2).
+__device__ __forceinline__ double upwind(double v, double t1, double t2, bool plain = false) {
+  const bool first = sign_clear(v);
+  const double p = (first ? t1 : t2) * v;
+  const unsigned rest = max(mag_hi(v), mag_hi(first ? t2 : t1));
+  if (rest >= 0x7fe00000u || mag_hi(p) - 0x00100000u >= 0x7fd00000u) {
+    if ((to_bits(p) << 1) == 0 && rest < 0x7fe00000u) return p;  // zero times a number
+    return plain ? intdiv::hw_mul(v, t1) : hw_upwind(v, t1, t2);
+  }
+  return p;
 }
 // a * b > 0, from the signs; factors small enough for the product to vanish by multiplication.
 __device__ __forceinline__ bool product_positive(double a, double b) {

@@ -265,7 +265,7 @@ __device__ __forceinline__ void node_mean_grad(const DMesh& m, const double* __r
 // pipe. 512^2 x 48, 2 tracers: volume fluxes, gradients and edge fluxes 4.4 ms
 // together against 10.9.
 // ---------------------------------------------------------------------------
-// The flux for any ph and for infinite and NaN values.
+// The flux for any ph and for very large, infinite and NaN values.
 static __device__ __noinline__ double hor_flux_any(double v, double Tm1, double Tm2, double ph) {
   return intdiv::behind_branch<double>([&] {
     const double cHO = (v + fabs(v)) * Tm1 + (v - fabs(v)) * Tm2;
@@ -321,8 +321,8 @@ __device__ __forceinline__ void hor_flux(const DMesh& m, const StepPtrs<double>&
         }
       }
       const double Tm1 = s1 + r1, Tm2 = s2 - r2;
-      // ph = 1: the upwind part is an exact zero (of finite values)
-      if (ph1 && bits64::finite(Tm1, Tm2) && bits64::finite(v)) h = -(B * (Tm1 + Tm2));
+      // ph = 1: the upwind part is an exact zero (unless its products overflow)
+      if (ph1 && bits64::moderate(Tm1, Tm2) && bits64::moderate(v)) h = -(B * (Tm1 + Tm2));
       else h = hor_flux_any(v, Tm1, Tm2, a.ph);
     }
     a.adfh[t * a.sE + ek] = FCT ? h + lo : h;
@@ -463,7 +463,7 @@ struct Column {
 // Vertical high-order fluxes (lib/oce_adv_tra_ver.F90:248-712).
 // VER: 0 UPW1, 1 QR4C, 2 CDIFF, 3 PPM.
 // ---------------------------------------------------------------------------
-// The expressions of infinite and NaN values and of any num_ord, out of line.
+// The expressions of very large, infinite and NaN values and of any num_ord, out of line.
 static __device__ __noinline__ double qr4c_any(double W, double tm1, double tm2, double num_ord, double A) {
   return intdiv::behind_branch<double>([&] {
     const double tm = (W + fabs(W)) * tm1 + (W - fabs(W)) * tm2;
@@ -602,9 +602,7 @@ __device__ __forceinline__ void ver_prepare(const VerGeo<VER>& g, const Column& 
 // First-order upwind flux through interface i (0-based, above layer i).
 __device__ __forceinline__ double ver_upw1(const double* T, int i, int k0, double W, double A) {
   const double T0 = T[i], Tu = i == k0 ? T0 : T[i - 1];
-  double x = bits64::upwind(W, T0, Tu);
-  if (i == k0 && !bits64::finite(T0, W)) x = intdiv::hw_mul(W, T0);  // the surface: W T as written
-  return -imul(x, A);
+  return -imul(bits64::upwind(W, T0, Tu, i == k0), A);
 }
 
 // The flux of a layer's parabola through one of its interfaces (:598-632) for
@@ -653,8 +651,8 @@ __device__ __forceinline__ double ver_flux(const VerGeo<VER>& g, const Column& c
     }
     const double mean = i == c.k0 ? T0 : bits64::half(x + y);
     double ho = -imul(mean * W, A);
-    // num_ord = 1: the upwind part is an exact zero (of finite values)
-    if (mid && !(num_ord == 1.0 && bits64::finite(x, y) && bits64::finite(W))) ho = qr4c_any(W, y, x, num_ord, A);
+    // num_ord = 1: the upwind part is an exact zero (unless its products overflow)
+    if (mid && !(num_ord == 1.0 && bits64::moderate(x, y) && bits64::moderate(W))) ho = qr4c_any(W, y, x, num_ord, A);
     const double f = ho - f0;
     return z == c.nzmin + 1 && z == c.nzmax - 1 ? ho - f : f;  // written twice (:405-411)
   }
