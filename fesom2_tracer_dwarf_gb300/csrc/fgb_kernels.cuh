@@ -662,7 +662,8 @@ __device__ __forceinline__ double ver_flux(const VerGeo<VER>& g, const Column& c
   }
   // PPM
   if (i == c.k0) return -((TV[i] * W) * A) - f0;
-  if ((bits64::to_bits(W) << 1) == 0) return 0.0 - f0;
+  // neither W > 0 nor W < 0 (:598-632): zero, and NaN, the bits above infinity's
+  if ((bits64::to_bits(W) << 1) - 1 >= 0xffe0000000000000ull) return 0.0 - f0;
   const bool up = bits64::sign_clear(W);
   const int L = up ? i : i - 1;  // the layer whose parabola crosses the interface
   return ppm_layer(TV[L], TV[L + 1], T[L], g.at(g.HX, i), g.at(g.CX, i), up, A, W) - f0;

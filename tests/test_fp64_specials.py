@@ -21,6 +21,7 @@ SPECIALS = {
     "tracer_nan": dict(T=[((1, 17, 2), NAN)]),
     "velocity_nan": dict(vel=[((31, 1, 0), NAN)]),
     "velocity_inf": dict(vel=[((31, 1, 0), INF), ((60, 0, 1), -INF)]),
+    "w_nan": dict(w=[((17, 1), NAN), ((40, 2), NAN), ((23, 3), NAN), ((50, 0), NAN)]),
     "w_inf": dict(w=[((17, 1), INF), ((44, 2), INF)]),
     "w_-inf": dict(w=[((17, 1), -INF), ((44, 2), -INF)]),
     "signed_zeros": dict(T=[((0,), 0.0), ((1,), -0.0)], w=[((slice(None, None, 2),), -0.0)],
