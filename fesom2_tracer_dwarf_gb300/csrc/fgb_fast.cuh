@@ -361,11 +361,15 @@ static __global__ void __launch_bounds__(kVfluxThreads) kf_vflux4(DMesh m, const
 // Layers outside the triangles' common window use the area-weighted mean
 // gradient of the elements around each node (lib/oce_muscl_adv.F90:393-410).
 // ---------------------------------------------------------------------------
-// Three elements at a time: their index, table and value loads are in flight
+// U elements at a time: their index, table and value loads are in flight
 // together. An element that is not there or dry at the layer adds a gradient
 // of zero with weight zero: its vertices' values may be anything, a NaN fill
-// too, so they are deselected and not only weighted.
-template <int KV>
+// too, so they are deselected and not only weighted. kf_hflux_mean takes three;
+// kf_hflux, which holds an edge's window values beside them, one: with three
+// it spills (up to 136 bytes) and its edge stage takes 860 against 643 us on
+// the pi mesh of 188,661 nodes, 47 layers, 4 tracers (cfg[0] = 2, cfg[7] = 1),
+// 1020 against 920 us on the closed 513^2x64, 2 tracers (8, 1).
+template <int KV, int U>
 __device__ __forceinline__ void node_grad(const DMesh& m, const float* __restrict__ TA, int n, unsigned k,
                                           V<KV>& gx, V<KV>& gy) {
   const GeoPtrs<float>& g = m.g32;
@@ -373,26 +377,42 @@ __device__ __forceinline__ void node_grad(const DMesh& m, const float* __restric
   const int z = (int)k + 1;
   float tvol = 0.f;
   V<KV> tx = splat<KV>(0.f), ty = splat<KV>(0.f);
-  const int end = m.nie_ptr[n + 1];
-  for (int j = m.nie_ptr[n]; j < end; j += 3) {
-    float ar[3];
-    V<KV> ex[3], ey[3];
-#pragma unroll
-    for (int u = 0; u < 3; ++u) {
-      const int el = m.nie_idx[min(j + u, end - 1)];
-      const int a = m.elem_nodes[3 * el], b = m.elem_nodes[3 * el + 1], c = m.elem_nodes[3 * el + 2];
-      const float* gs = g.grad_sca + 6 * (size_t)el;
-      const V<KV> ta = ld<KV>(TA, a * LZ + k), tb = ld<KV>(TA, b * LZ + k), tc = ld<KV>(TA, c * LZ + k);
-      const bool wet = j + u < end && m.elem_nlev[el] - 1 >= z;
-      ex[u] = wet ? fmas(tc, gs[2], fmas(tb, gs[1], muls(ta, gs[0]))) : splat<KV>(0.f);
-      ey[u] = wet ? fmas(tc, gs[5], fmas(tb, gs[4], muls(ta, gs[3]))) : splat<KV>(0.f);
-      ar[u] = wet ? g.elem_area[el] : 0.f;
+  auto grad = [&](int el, V<KV>& ex, V<KV>& ey) {
+    const int a = m.elem_nodes[3 * el], b = m.elem_nodes[3 * el + 1], c = m.elem_nodes[3 * el + 2];
+    const float* gs = g.grad_sca + 6 * (size_t)el;
+    const V<KV> ta = ld<KV>(TA, a * LZ + k), tb = ld<KV>(TA, b * LZ + k), tc = ld<KV>(TA, c * LZ + k);
+    ex = fmas(tc, gs[2], fmas(tb, gs[1], muls(ta, gs[0])));
+    ey = fmas(tc, gs[5], fmas(tb, gs[4], muls(ta, gs[3])));
+  };
+  auto add_elem = [&](const V<KV>& ex, const V<KV>& ey, float ar) {
+    tvol += ar;
+    tx = fmas(ex, ar, tx);
+    ty = fmas(ey, ar, ty);
+  };
+  if constexpr (U == 1) {
+    for (int j = m.nie_ptr[n]; j < m.nie_ptr[n + 1]; ++j) {
+      const int el = m.nie_idx[j];
+      if (m.elem_nlev[el] - 1 < z) continue;
+      V<KV> ex, ey;
+      grad(el, ex, ey);
+      add_elem(ex, ey, g.elem_area[el]);
     }
+  } else {
+    const int end = m.nie_ptr[n + 1];
+    for (int j = m.nie_ptr[n]; j < end; j += U) {
+      float ar[U];
+      V<KV> ex[U], ey[U];
 #pragma unroll
-    for (int u = 0; u < 3; ++u) {
-      tvol += ar[u];
-      tx = fmas(ex[u], ar[u], tx);
-      ty = fmas(ey[u], ar[u], ty);
+      for (int u = 0; u < U; ++u) {
+        const int el = m.nie_idx[min(j + u, end - 1)];
+        const bool wet = j + u < end && m.elem_nlev[el] - 1 >= z;
+        grad(el, ex[u], ey[u]);
+        ex[u] = wet ? ex[u] : splat<KV>(0.f);
+        ey[u] = wet ? ey[u] : splat<KV>(0.f);
+        ar[u] = wet ? g.elem_area[el] : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) add_elem(ex[u], ey[u], ar[u]);
     }
   }
   const float inv = fdv(1.f, tvol);
@@ -534,9 +554,9 @@ __global__ void __launch_bounds__(256, (NS == 1 ? 3 : 2)) kf_hflux(DMesh m, Fast
               p2 = fmas(d2, wd.z, fmas(d1, wd.y, fmas(s2[i], wd.x, dT3)));
             } else if (act[i]) {
               V<KV> gx, gy;
-              node_grad<KV>(m, TAg, n1, kk[i], gx, gy);
+              node_grad<KV, 1>(m, TAg, n1, kk[i], gx, gy);
               p1 = fmas(fmas(gy, ey, muls(gx, ex)), 1.f / 6.f, dT3);
-              node_grad<KV>(m, TAg, n2, kk[i], gx, gy);
+              node_grad<KV, 1>(m, TAg, n2, kk[i], gx, gy);
               p2 = fmas(fmas(gy, ey, muls(gx, ex)), 1.f / 6.f, dT3);
             } else {
               p1 = splat<KV>(0.f);

@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kTileThreads) kf_hflux_mean(DMesh m, FastPtrs 
   const float* __restrict__ Tg = a.T + blockIdx.y * a.gT;
   const float* __restrict__ TAg = a.TA != a.T ? a.TA + blockIdx.y * a.gTA : Tg;
   V<KV> gx = splat<KV>(0.f), gy = gx;
-  if (act) node_grad<KV>(m, TAg, side ? n2 : n1, k, gx, gy);
+  if (act) node_grad<KV, 3>(m, TAg, side ? n2 : n1, k, gx, gy);
   const float ex = m.g32.edge_dxa[2 * e], ey = m.g32.edge_dxa[2 * e + 1];
   const V<KV> p = muls(fmas(gy, ey, muls(gx, ex)), 1.f / 6.f);
   const V<KV> o = shfl_v(p, threadIdx.x ^ 1);  // the other node's

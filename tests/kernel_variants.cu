@@ -1,0 +1,22 @@
+// More variants of the FP32 step's kernels, instantiated alone so that
+// tests/test_kernel_variants.py can read ptxas's spill report for them.
+#include "fgb_fast_launch.cuh"
+
+namespace fgb {
+namespace fast {
+
+// per-edge edge fluxes (fields without 16-byte alignment, launch shapes asked for)
+template __global__ void kf_hflux<1, true, 4, 1>(DMesh, FastPtrs);
+template __global__ void kf_hflux<1, true, 4, 2>(DMesh, FastPtrs);
+template __global__ void kf_hflux<2, true, 4, 1>(DMesh, FastPtrs);
+template __global__ void kf_hflux<2, true, 4, 2>(DMesh, FastPtrs);
+template __global__ void kf_hflux<1, true, 2, 1>(DMesh, FastPtrs);
+// mean-gradient layers
+template __global__ void kf_hflux_mean<1, true, 4>(DMesh, FastPtrs);
+template __global__ void kf_hflux_mean<2, true, 2>(DMesh, FastPtrs);
+
+// volume fluxes, a thread per four layers
+void* keep_vflux4() { return reinterpret_cast<void*>(&kf_vflux4); }
+
+}  // namespace fast
+}  // namespace fgb
