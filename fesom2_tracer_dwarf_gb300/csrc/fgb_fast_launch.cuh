@@ -144,7 +144,7 @@ void launch_ratio64(const DMesh& m, const FastPtrs& a, int nw, cudaStream_t s) {
 
 template <int KV, int VER, bool TASEP, bool WESEP, bool COMP>
 void launch_lo64c(const DMesh& m, const FastPtrs& a, cudaStream_t s) {
-  const size_t sm = kLo64Warps * lo64_warp_bytes(KV, VER, TASEP);
+  const size_t sm = kLo64Warps * lo64_warp_bytes(KV, VER & 3, TASEP);
   allow_smem_f(kf_lo64<VER, KV, TASEP, WESEP, COMP>, sm);
   kf_lo64<VER, KV, TASEP, WESEP, COMP><<<(m.N + kLo64Warps - 1) / kLo64Warps, kLo64Warps * kW, sm, s>>>(m, a);
 }
@@ -159,10 +159,12 @@ void launch_lo_ns(const DMesh& m, const FastPtrs& a, const LaunchArgs& L, cudaSt
   if (L.ns_lo == 3) {  // whole column per warp (at most 64 layers)
     const bool tasep = a.TA != a.T, wesep = a.we != a.w;
     if (tasep) {
-      if (wesep) launch_lo64<KV, VER, true, true>(m, a, s);
+      if (wesep && a.wi) launch_lo64<KV, VER + 4, true, true>(m, a, s);
+      else if (wesep) launch_lo64<KV, VER, true, true>(m, a, s);
       else launch_lo64<KV, VER, true, false>(m, a, s);
     } else {
-      if (wesep) launch_lo64<KV, VER, false, true>(m, a, s);
+      if (wesep && a.wi) launch_lo64<KV, VER + 4, false, true>(m, a, s);
+      else if (wesep) launch_lo64<KV, VER, false, true>(m, a, s);
       else launch_lo64<KV, VER, false, false>(m, a, s);
     }
   } else if (L.ns_lo == 1) {

@@ -35,8 +35,13 @@ __host__ __device__ constexpr size_t lo64_warp_bytes(int KV, int ver, bool tasep
          (ver == 3 ? 2 * 64 * 4 : 0) + (ver == 1 ? (64 + 68) * 4 : 0) + 2 * 64 * 4 + kMaxDegF * sizeof(int2);
 }
 
-template <int VER, int KV, bool TASEP, bool WESEP, bool COMP>
+// VERW: the vertical scheme, + 4 under w_split with a w_e of its own (the
+// explicit flux of the full w then joins the antidiffusive flux; as a test in
+// the same kernel it cost calls without w_split up to a third of this stage).
+template <int VERW, int KV, bool TASEP, bool WESEP, bool COMP>
 __global__ void __launch_bounds__(kLo64Warps * kW, 7) kf_lo64(DMesh m, FastPtrs a) {
+  constexpr int VER = VERW & 3;
+  constexpr bool WS = VERW >= 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kW - 1), wib = threadIdx.x / kW;
   const int vi = blockIdx.x * kLo64Warps + wib;
@@ -242,7 +247,7 @@ __global__ void __launch_bounds__(kLo64Warps * kW, 7) kf_lo64(DMesh m, FastPtrs 
       }
       sF[iz] = lo;
       V<KV> lf = lo;
-      if (WESEP && a.wi && in && z < nzmax) {
+      if (WS && in && z < nzmax) {
         // w_split: the antidiffusive flux takes the upwind flux of the full w
         // (lib/oce_adv_tra_driver.F90:221-231)
         const float W = w[s], A = ar[s];

@@ -14,6 +14,10 @@ template __global__ void kf_hflux<1, true, 2, 1>(DMesh, FastPtrs);
 // mean-gradient layers
 template __global__ void kf_hflux_mean<1, true, 4>(DMesh, FastPtrs);
 template __global__ void kf_hflux_mean<2, true, 2>(DMesh, FastPtrs);
+// LO stage, QR4C and PPM, separate T_AB and w_e without w_split
+template __global__ void kf_lo64<1, 4, true, true, false>(DMesh, FastPtrs);
+template __global__ void kf_lo64<3, 4, true, true, false>(DMesh, FastPtrs);
+template __global__ void kf_lo64<1, 2, false, true, false>(DMesh, FastPtrs);
 
 // volume fluxes, a thread per four layers
 void* keep_vflux4() { return reinterpret_cast<void*>(&kf_vflux4); }

@@ -18,6 +18,9 @@ EXPECTED = {
     "kf_hflux<1, true, 2, 1>": 0,
     "kf_hflux_mean<1, true, 4>": 0,
     "kf_hflux_mean<2, true, 2>": 0,
+    "kf_lo64<1, 4, true, true, false>": 0,
+    "kf_lo64<3, 4, true, true, false>": 0,
+    "kf_lo64<1, 2, false, true, false>": 0,
     "kf_vflux4": 0,
 }
 
