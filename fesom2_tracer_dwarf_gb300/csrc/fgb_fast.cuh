@@ -120,17 +120,20 @@ __device__ __forceinline__ V<KV> add(const V<KV>& a, const V<KV>& b) {
   }
   return r;
 }
-// a - b as fma(b, -1, a), the same rounding: the packed addition takes no
-// negated operand, so a pair of negations would go with each (with the signed
-// volume flux of kf_lo64's gather: LO stage 2.10 -> 2.01 ms at 1024^2x64, 4
-// tracers, compensated; 565 -> 505 us on eight meshes, 8 tracers, QR4C).
-template <int KV>
+// a - b. F: as fma(b, -1, a), the same rounding: the packed addition takes no
+// negated operand, so a pair of negations goes with each. That saves
+// instructions and usually time (kf_lo64 with the signed volume flux of its
+// gather: LO stage 2.10 -> 2.01 ms at 1024^2x64, 4 tracers, compensated), but
+// ties the operands to other registers: at a tight bound ptxas may then move or
+// spill more than the negations cost. The kernels that lose by it say so.
+template <int KV, bool F = true>
 __device__ __forceinline__ V<KV> sub(const V<KV>& a, const V<KV>& b) {
   V<KV> r;
   if constexpr (KV % 2 == 0) {
 #pragma unroll
     for (int j = 0; j < KV; j += 2) {
-      const float2 t = __ffma2_rn(FGB_F2(b, j), make_float2(-1.f, -1.f), FGB_F2(a, j));
+      const float2 t = F ? __ffma2_rn(FGB_F2(b, j), make_float2(-1.f, -1.f), FGB_F2(a, j))
+                         : __fadd2_rn(FGB_F2(a, j), make_float2(-b.v[j], -b.v[j + 1]));
       r.v[j] = t.x;
       r.v[j + 1] = t.y;
     }
@@ -184,12 +187,12 @@ __device__ __forceinline__ V<KV> muls(const V<KV>& a, float s) {
 // Error-free addition (Knuth's TwoSum: six additions, exact for any order of
 // magnitudes): s + x = s' + e exactly; s <- s', c <- c + e. Summing with it
 // keeps each sum's rounding error in c, so a compensated sum (s, c) of FP32
-// terms is exact to the rounding of c.
-template <int KV>
+// terms is exact to the rounding of c. F: the form of its subtractions.
+template <bool F = true, int KV>
 __device__ __forceinline__ void two_sum(V<KV>& s, V<KV>& c, const V<KV>& x) {
   const V<KV> t = add(s, x);
-  const V<KV> bp = sub(t, s);
-  const V<KV> e = add(sub(s, sub(t, bp)), sub(x, bp));
+  const V<KV> bp = sub<KV, F>(t, s);
+  const V<KV> e = add(sub<KV, F>(s, sub<KV, F>(t, bp)), sub<KV, F>(x, bp));
   s = t;
   c = add(c, e);
 }
@@ -1073,9 +1076,12 @@ __global__ void __launch_bounds__(128, 7) kf_lo(DMesh m, FastPtrs a) {
 #pragma unroll
           for (int c = 0; c < KV; ++c) tu.v[c] = own_up ? tnk[i].v[c] : to[i].v[c];
           const V<KV> p = muls(tu, v[i]);
-          // with COMP the sum carries its rounding error (TwoSum)
-          if (COMP) two_sum(acc[i], accc[i], role ? p : sub(splat<KV>(0.f), p));
-          else acc[i] = role ? add(acc[i], p) : sub(acc[i], p);
+          // With COMP the sum carries its rounding error (TwoSum). Two layers per lane fill the
+          // 72 registers: the sums' subtractions as additions (220^2, 4 tracers, 75 layers: LO
+          // stage 11 to 15 % shorter than with fma), with one layer as fma (3 % shorter).
+          constexpr bool F = NS == 1;
+          if (COMP) two_sum<F>(acc[i], accc[i], role ? p : sub<KV, F>(splat<KV>(0.f), p));
+          else acc[i] = role ? add(acc[i], p) : sub<KV, F>(acc[i], p);
         }
       }
       V<KV> lk[NS];
@@ -1238,8 +1244,8 @@ __global__ void __launch_bounds__(128, (NS == 1 ? 10 : 7)) kf_ratio(DMesh m, Fas
               xp.v[t] = fmaxf(0.f, x);
               xm.v[t] = fminf(0.f, x);
             }
-            two_sum(pl[i], plc[i], xp);
-            two_sum(mi[i], mic[i], xm);
+            two_sum<KV != 2>(pl[i], plc[i], xp);  // two tracers: 2 % shorter with additions
+            two_sum<KV != 2>(mi[i], mic[i], xm);
           } else {
 #pragma unroll
             for (int t = 0; t < KV; ++t) {
@@ -1423,8 +1429,8 @@ __device__ __forceinline__ void ratio64_column(const DMesh& m, const FastPtrs& a
             xp.v[t] = fmaxf(0.f, x);
             xm.v[t] = fminf(0.f, x);
           }
-          two_sum(pl[i], plc[i], xp);
-          two_sum(mi[i], mic[i], xm);
+          two_sum<KV != 2>(pl[i], plc[i], xp);
+          two_sum<KV != 2>(mi[i], mic[i], xm);
         } else {
 #pragma unroll
           for (int t = 0; t < KV; ++t) {

@@ -35,13 +35,34 @@ __host__ __device__ constexpr size_t lo64_warp_bytes(int KV, int ver, bool tasep
          (ver == 3 ? 2 * 64 * 4 : 0) + (ver == 1 ? (64 + 68) * 4 : 0) + 2 * 64 * 4 + kMaxDegF * sizeof(int2);
 }
 
+// The gather adds v T_up or subtracts it. True: the sign goes onto the volume
+// flux before the product; false: the sum or the product takes it. Both give
+// the same bits, and at the 72 registers of seven blocks per SM the difference
+// is what ptxas makes of each variant, so the choice is from measurement, all
+// variants at 220^2x64 (periodic) and 220^2x47 (closed basin); LO stage with the
+// sign first against after: one tracer, plain sums, CDIFF 0.90, UPW1 0.99, PPM
+// 1.01 to 1.03, compensated sums 1.00 to 1.08; two tracers, plain sums, CDIFF
+// 0.80 to 0.86, QR4C 0.80 to 0.97, PPM 1.02 to 1.05, compensated 0.97 to 1.10;
+// four tracers 0.87 to 0.99 but for the two named variants (1.05, 1.02).
+__host__ __device__ constexpr bool lo64_sign_first(int VER, int KV, bool TASEP, bool WESEP, bool COMP) {
+  if (KV != 4) return !COMP && VER != 3;
+  return COMP || WESEP || (VER != 2 && VER != 1) || (VER == 2) == TASEP;
+}
+// Subtractions as fma (see sub): with four tracers and compensated sums, LO
+// stage against additions 0.98 for UPW1 and PPM (1.02 to 1.08 with a w_e of its
+// own), 1.04 to 1.06 for QR4C and CDIFF (0.94 with a w_e of its own), 0.96 under
+// w_split; with two tracers 1.0 to 1.25.
+__host__ __device__ constexpr bool lo64_fma_sub(int VER, int KV, bool WESEP, bool WS) {
+  return KV == 4 && (WS || ((VER == 0 || VER == 3) != WESEP));
+}
+
 // VERW: the vertical scheme, + 4 under w_split with a w_e of its own (the
 // explicit flux of the full w then joins the antidiffusive flux; as a test in
 // the same kernel it cost calls without w_split up to a third of this stage).
 template <int VERW, int KV, bool TASEP, bool WESEP, bool COMP>
 __global__ void __launch_bounds__(kLo64Warps * kW, 7) kf_lo64(DMesh m, FastPtrs a) {
   constexpr int VER = VERW & 3;
-  constexpr bool WS = VERW >= 4;
+  constexpr bool WS = VERW >= 4, F = lo64_fma_sub(VER, KV, WESEP, WS);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kW - 1), wib = threadIdx.x / kW;
   const int vi = blockIdx.x * kLo64Warps + wib;
@@ -162,7 +183,7 @@ __global__ void __launch_bounds__(kLo64Warps * kW, 7) kf_lo64(DMesh m, FastPtrs 
           const float Q2 = r4 * (dz * (dzm + dz)) * r2;
           const float Q3 = r4 * (dzp * (dzp + dzpp)) * r3;
           const V<KV> Tu = sTA[j0];
-          e = fmas(sD[j0], Q3, fmas(sD[j0 + 1], -Q2, fmas(sub(ta[s], Tu), P, Tu)));
+          e = fmas(sD[j0], Q3, fmas(sD[j0 + 1], -Q2, fmas(sub<KV, F>(ta[s], Tu), P, Tu)));
         } else if (z == nzmax) {
           e = sTA[nzmax - 2];
         } else if (z == nzmax - 1) {
@@ -220,7 +241,7 @@ __global__ void __launch_bounds__(kLo64Warps * kW, 7) kf_lo64(DMesh m, FastPtrs 
             const float wp = W + fabsf(W), wm = W - fabsf(W);
             const float cA = -(0.5f * (1.f - a.pv)) * A, cB = -(a.pv * 0.5f) * W * A;
             const V<KV> T0 = ta[s], Tm1 = TAup, Tm2 = sTA[z - 3], Tp1 = sTA[z];
-            const V<KV> qc = muls(sub(Tm1, T0), ic), qu = muls(sub(T0, Tp1), iu), qd = muls(sub(Tm2, Tm1), idn);
+            const V<KV> qc = muls(sub<KV, F>(Tm1, T0), ic), qu = muls(sub<KV, F>(T0, Tp1), iu), qd = muls(sub<KV, F>(Tm2, Tm1), idn);
             const V<KV> tm1 = fmas(fmas(qc, 2.f, qu), a1, T0);
             const V<KV> tm2 = fmas(fmas(qc, 2.f, qd), a2, Tm1);
             const V<KV> tm = fmas(tm2, wm, muls(tm1, wp));
@@ -254,8 +275,8 @@ __global__ void __launch_bounds__(kLo64Warps * kW, 7) kf_lo64(DMesh m, FastPtrs 
         lf = z == nzmin ? muls(t[s], -(W * A))
                         : fmas(Tup, -0.5f * (W - fabsf(W)) * A, muls(t[s], -0.5f * (W + fabsf(W)) * A));
       }
-      const V<KV> d = sub(ho, lf);
-      if (iz < nl) st<KV>(adfv, (unsigned)n * LW + iz, twice ? sub(ho, d) : d);
+      const V<KV> d = sub<KV, F>(ho, lf);
+      if (iz < nl) st<KV>(adfv, (unsigned)n * LW + iz, twice ? sub<KV, F>(ho, d) : d);
     }
     if (lane == 0 && nl - 1 >= 2 * kW) {  // the bottom interface of 65-interface columns
       sF[nl - 1] = splat<KV>(0.f);
@@ -290,15 +311,14 @@ __global__ void __launch_bounds__(kLo64Warps * kW, 7) kf_lo64(DMesh m, FastPtrs 
         V<KV> tu;
 #pragma unroll
         for (int c = 0; c < KV; ++c) tu.v[c] = own_up ? t[s].v[c] : to[s].v[c];
-        if constexpr (COMP && KV == 2) {
-          // the sign after the product: with it before, this variant is slower
-          // (closed 513^2x64: LO stage 420 against 402 us)
-          const V<KV> p = muls(tu, v[s]);
-          two_sum(acc[s], accc[s], role ? p : sub(splat<KV>(0.f), p));
-        } else {
+        if constexpr (lo64_sign_first(VER, KV, TASEP, WESEP, COMP)) {
           const V<KV> p = muls(tu, role ? v[s] : -v[s]);
-          if (COMP) two_sum(acc[s], accc[s], p);
+          if (COMP) two_sum<F>(acc[s], accc[s], p);
           else acc[s] = add(acc[s], p);
+        } else {
+          const V<KV> p = muls(tu, v[s]);
+          if (COMP) two_sum<F>(acc[s], accc[s], role ? p : sub<KV, F>(splat<KV>(0.f), p));
+          else acc[s] = role ? add(acc[s], p) : sub<KV, F>(acc[s], p);
         }
       }
     }
@@ -310,7 +330,7 @@ __global__ void __launch_bounds__(kLo64Warps * kW, 7) kf_lo64(DMesh m, FastPtrs 
       // the increment LO - T = (fluxes) dt / (areasvol hnode_new) + T (hnode / hnode_new - 1)
       V<KV> l = splat<KV>(0.f);
       if (z >= nzmin && z <= nzmax - 1)
-        l = fmas(add(COMP ? add(acc[s], accc[s]) : acc[s], sub(sF[k[s]], sF[k[s] + 1])), sRb[k[s]],
+        l = fmas(add(COMP ? add(acc[s], accc[s]) : acc[s], sub<KV, F>(sF[k[s]], sF[k[s] + 1])), sRb[k[s]],
                  muls(t[s], sRa[k[s]] - 1.f));
       st<KV>(lo, (unsigned)n * LZ + k[s], l);
     }
