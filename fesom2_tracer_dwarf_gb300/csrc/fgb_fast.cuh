@@ -1244,7 +1244,7 @@ __global__ void __launch_bounds__(128, (NS == 1 ? 10 : 7)) kf_ratio(DMesh m, Fas
               xp.v[t] = fmaxf(0.f, x);
               xm.v[t] = fminf(0.f, x);
             }
-            two_sum<KV != 2>(pl[i], plc[i], xp);  // two tracers: 2 % shorter with additions
+            two_sum<KV != 2>(pl[i], plc[i], xp);  // for two tracers: see ratio64_column
             two_sum<KV != 2>(mi[i], mic[i], xm);
           } else {
 #pragma unroll
@@ -1303,7 +1303,9 @@ __host__ __device__ constexpr size_t ratio64_warp_bytes(int KV) { return (size_t
 // Gathers in flight per warp, from measurement: groups of one or two tracers
 // take four cluster nodes and six edges at a time (closed 513^2x64, 2 tracers:
 // 420 us; two of each 451, seven nodes and six edges 445), groups of four two
-// of each (three nodes: 494 against 430 us on the 188,661-node pi mesh).
+// of each (three nodes: 494 against 430 us on the 188,661-node pi mesh). Two
+// tracers with compensated sums: two of each, and subtractions as additions
+// (220^2x64: 86 us; four and six 98, with fma subtractions 95).
 // Shared memory: ratio64_warp_bytes per warp, where the finished bounds wait.
 template <int KV, bool LEAN, bool COMP>
 __device__ __forceinline__ void ratio64_column(const DMesh& m, const FastPtrs& a) {
@@ -1347,7 +1349,7 @@ __device__ __forceinline__ void ratio64_column(const DMesh& m, const FastPtrs& a
       mn[i] = splat<KV>(-m0);
       lo[i] = live[i] ? add(ld<KV>(Tg, n * LZ + kk[i]), ld<KV>(Lg, n * LZ + kk[i])) : splat<KV>(0.f);  // LO = T + (LO - T)
     }
-#pragma unroll(LEAN ? 1 : (KV <= 2 ? 4 : 2))
+#pragma unroll(LEAN ? 1 : (KV <= 2 && !(KV == 2 && COMP) ? 4 : 2))
     for (int j = 0; j < ncl; ++j) {
       const int c = m.cl_node[c0 + j], lev = m.cl_lev[c0 + j];
       V<KV> lv[2], tv[2];
@@ -1411,7 +1413,7 @@ __device__ __forceinline__ void ratio64_column(const DMesh& m, const FastPtrs& a
       plc[i] = splat<KV>(0.f);
       mic[i] = plc[i];
     }
-#pragma unroll(LEAN ? 1 : (KV <= 2 ? 6 : 2))
+#pragma unroll(LEAN ? 1 : (KV <= 2 && !(KV == 2 && COMP) ? 6 : 2))
     for (int j = 0; j < deg; ++j) {
       const int code = m.ne_code[j0 + j];
       const unsigned ed = (unsigned)(code >> 1);
@@ -1538,7 +1540,9 @@ __device__ __forceinline__ void finish_node(const DMesh& m, const FastPtrs& a, i
 // fetched together with the first neighbours, and two incident edges are in
 // flight per round, three for groups of one or two tracers (closed 513^2x64, 2
 // tracers: 470 against 489 us; four tracers, 1024^2x64: 2.68 against 2.63 ms,
-// and 2.81 or more with fewer warps of more registers).
+// and 2.81 or more with fewer warps of more registers), but two for one tracer
+// with a compensated divergence (220^2x64: 74 against 92 us) and where a lane
+// holds two layers (two tracers with the residual: 16 % shorter).
 // DEL: a persistent del_ttf is read and written (the reference C interface).
 // COMP: the limited edge fluxes are formed as one rounded product p = ae * f,
 // the same number at both ends of the edge (+p at the first node, -p at the
@@ -1644,7 +1648,7 @@ __global__ void __launch_bounds__(128, (NS == 1 ? (COMP || RES ? 8 : 9) : 4)) kf
           hn[i] = g.hnode[n * LZ + kk[i]];
         }
       }
-#pragma unroll(KV <= 2 ? 3 : 2)
+#pragma unroll(KV <= 2 && NS == 1 && !(KV == 1 && COMP) ? 3 : 2)
       for (int j = 0; j < nb.deg; ++j) {
         const int2 q = nb.get(m, j);
         const unsigned ed = (unsigned)(q.x >> 1);

@@ -21,6 +21,10 @@ EXPECTED = {
     "kf_lo64<1, 4, true, true, false>": 0,
     "kf_lo64<3, 4, true, true, false>": 0,
     "kf_lo64<1, 2, false, true, false>": 0,
+    "kf_ratio64<2, false, true>": 0,
+    "kf_ratio64<1, false, true>": 0,
+    "kf_update<1, 1, false, true, false>": 0,
+    "kf_update<2, 1, false, false, false>": 8,
     "kf_vflux4": 0,
 }
 
