@@ -70,11 +70,11 @@ struct DMesh {
   const unsigned char* tile_slots;
   // The layers of MUSCL/MFCT edges outside their triangles' window: nmean runs
   // {edge, first layer (0-based) | layers << 16} of at most kMeanRun layers.
-  int nmean;
+  // windows_wet: every window lies within the layers of its edge's two triangles,
+  // so that an array of the wet layers' element gradients holds all that the
+  // windows read.
+  int nmean, windows_wet;
   const int* mean_seg;
-  // Every window lies within the layers of its edge's two triangles, so that an
-  // array of the wet layers' element gradients holds all that the windows read.
-  int windows_wet;
   GeoPtrs<double> g64;
   GeoPtrs<float> g32;
 };
