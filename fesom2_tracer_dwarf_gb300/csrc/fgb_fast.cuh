@@ -589,6 +589,10 @@ __global__ void __launch_bounds__(256, (NS == 1 ? 3 : 2)) kf_hflux(DMesh m, Fast
 
 // ---------------------------------------------------------------------------
 // Column staging and vertical fluxes (lib/oce_adv_tra_ver.F90:248-712).
+// Their subtractions are additions (see sub): as fma the LO stage that solves
+// the implicit step in the same pass took 149 us against 141 (220^2x64, four
+// tracers, QR4C), the update without a limiter 122 against 117 (two tracers,
+// PPM, two layers per lane).
 // ---------------------------------------------------------------------------
 struct ColF {
   const float* W;
@@ -639,7 +643,7 @@ __device__ __forceinline__ V<KV> ppm_edge(const V<KV>* T, const V<KV>* D, const 
     const float P = c0 + ci * c1;
     const float Q2 = ci * fdv(dz * (dzm + dz), 2.f * dz + dzp);
     const float Q3 = ci * fdv(dzp * (dzp + dzpp), dz + 2.f * dzp);
-    const V<KV> d = sub(T[j0 + 1], T[j0]);
+    const V<KV> d = sub<KV, false>(T[j0 + 1], T[j0]);
     return fmas(D[j0], Q3, fmas(D[j0 + 1], -Q2, fmas(d, P, T[j0])));
   }
   if (z == nzmax) return T[nzmax - 2];
@@ -739,7 +743,7 @@ __device__ void vert_flux(const ColF& c, const V<KV>* T, V<KV>* D, V<KV>* TV, co
   if (lane == 0) {
     // z = nl: the column's last interface (zero flux, CDIFF leaves it) or below the column
     const V<KV> f0 = fold ? fold[last] : splat<KV>(0.f);
-    out[last] = (nzmax == nl && VER != 2) ? sub(splat<KV>(0.f), f0) : f0;
+    out[last] = (nzmax == nl && VER != 2) ? sub<KV, false>(splat<KV>(0.f), f0) : f0;
   }
   for (int iz = lane; iz < last; iz += kW) {
     const int z = iz + 1;
@@ -748,19 +752,19 @@ __device__ void vert_flux(const ColF& c, const V<KV>* T, V<KV>* D, V<KV>* TV, co
     if (z >= nzmin && z <= nzmax) {
       const float W = c.W[iz], ar = c.area[iz];
       if (VER == 0) {
-        if (z == nzmin) r = sub(muls(T[z - 1], -(W * ar)), f0);
-        else if (z == nzmax) r = sub(splat<KV>(0.f), f0);
+        if (z == nzmin) r = sub<KV, false>(muls(T[z - 1], -(W * ar)), f0);
+        else if (z == nzmax) r = sub<KV, false>(splat<KV>(0.f), f0);
         else
-          r = sub(fmas(T[z - 2], -0.5f * (W - fabsf(W)) * ar, muls(T[z - 1], -0.5f * (W + fabsf(W)) * ar)), f0);
+          r = sub<KV, false>(fmas(T[z - 2], -0.5f * (W - fabsf(W)) * ar, muls(T[z - 1], -0.5f * (W + fabsf(W)) * ar)), f0);
       } else if (VER == 1) {
         if (z == nzmin) {
-          r = sub(muls(T[z - 1], -(W * ar)), f0);
+          r = sub<KV, false>(muls(T[z - 1], -(W * ar)), f0);
         } else if (z == nzmax) {
-          r = sub(splat<KV>(0.f), f0);
+          r = sub<KV, false>(splat<KV>(0.f), f0);
         } else if (z == nzmin + 1 || z == nzmax - 1) {
           const V<KV> x = muls(add(T[z - 2], T[z - 1]), -0.5f * W * ar);
-          r = sub(x, f0);
-          if (nzmin + 1 == nzmax - 1) r = sub(x, r);  // written twice (lib/oce_adv_tra_ver.F90:405-411)
+          r = sub<KV, false>(x, f0);
+          if (nzmin + 1 == nzmax - 1) r = sub<KV, false>(x, r);  // written twice (lib/oce_adv_tra_ver.F90:405-411)
         } else {
           const float Z0 = c.Z[z - 1], Zm1 = c.Z[z - 2], Zm2 = c.Z[z - 3], Zp1 = c.Z[z];
           const float ic = fdv(1.f, Zm1 - Z0), iu = fdv(1.f, Z0 - Zp1), idn = fdv(1.f, Zm2 - Zm1);
@@ -769,16 +773,16 @@ __device__ void vert_flux(const ColF& c, const V<KV>* T, V<KV>* D, V<KV>* TV, co
           const float wp = W + fabsf(W), wm = W - fabsf(W);
           const float cA = -(0.5f * (1.f - num_ord)) * ar, cB = -(num_ord * 0.5f) * W * ar;
           const V<KV> T0 = T[z - 1], Tm1 = T[z - 2], Tm2 = T[z - 3], Tp1 = T[z];
-          const V<KV> qc = muls(sub(Tm1, T0), ic), qu = muls(sub(T0, Tp1), iu), qd = muls(sub(Tm2, Tm1), idn);
+          const V<KV> qc = muls(sub<KV, false>(Tm1, T0), ic), qu = muls(sub<KV, false>(T0, Tp1), iu), qd = muls(sub<KV, false>(Tm2, Tm1), idn);
           const V<KV> tm1 = fmas(fmas(qc, 2.f, qu), a1, T0);
           const V<KV> tm2 = fmas(fmas(qc, 2.f, qd), a2, Tm1);
           const V<KV> tm = fmas(tm2, wm, muls(tm1, wp));
-          r = sub(fmas(add(tm1, tm2), cB, muls(tm, cA)), f0);
+          r = sub<KV, false>(fmas(add(tm1, tm2), cB, muls(tm, cA)), f0);
         }
       } else if (VER == 2) {
         const int nzc = nzmax - 1;  // lib/oce_adv_tra_ver.F90:689
-        if (z == nzmin) r = sub(muls(T[z - 1], -(W * ar)), f0);
-        else if (z <= nzc) r = sub(muls(add(T[z - 2], T[z - 1]), -0.5f * W * ar), f0);
+        if (z == nzmin) r = sub<KV, false>(muls(T[z - 1], -(W * ar)), f0);
+        else if (z <= nzc) r = sub<KV, false>(muls(add(T[z - 2], T[z - 1]), -0.5f * W * ar), f0);
       } else {
         V<KV> tvert = splat<KV>(0.f);
         if (z == nzmin) {
@@ -790,7 +794,7 @@ __device__ void vert_flux(const ColF& c, const V<KV>* T, V<KV>* D, V<KV>* TV, co
           const float x = fminf(fdv(fabsf(W) * dt, c.hn[zl]), 1.f);
           tvert = ppm_flux<KV>(TV[zl], TV[zl + 1], T[zl], x, up, ar * W);
         }
-        r = sub(tvert, f0);
+        r = sub<KV, false>(tvert, f0);
       }
     }
     out[iz] = r;
@@ -954,6 +958,10 @@ __device__ __forceinline__ void vimpl_row(int k, int k0, int k1, float W0, float
 // ---------------------------------------------------------------------------
 template <int VER, int KV, int NS, bool WSPLIT, bool COMP>
 __global__ void __launch_bounds__(128, 7) kf_lo(DMesh m, FastPtrs a) {
+  // Two layers per lane fill the 72 registers: subtractions as additions (220^2, 4 tracers, 75
+  // layers, compensated: LO stage 11 to 15 % shorter than with fma; the w_split pass 3 to 6 % for
+  // QR4C), with one layer as fma (3 % shorter).
+  constexpr bool F = NS == 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kW - 1), wib = threadIdx.x / kW;
   const int vi = blockIdx.x * (blockDim.x / kW) + wib;
@@ -1076,10 +1084,7 @@ __global__ void __launch_bounds__(128, 7) kf_lo(DMesh m, FastPtrs a) {
 #pragma unroll
           for (int c = 0; c < KV; ++c) tu.v[c] = own_up ? tnk[i].v[c] : to[i].v[c];
           const V<KV> p = muls(tu, v[i]);
-          // With COMP the sum carries its rounding error (TwoSum). Two layers per lane fill the
-          // 72 registers: the sums' subtractions as additions (220^2, 4 tracers, 75 layers: LO
-          // stage 11 to 15 % shorter than with fma), with one layer as fma (3 % shorter).
-          constexpr bool F = NS == 1;
+          // with COMP the sum carries its rounding error (TwoSum)
           if (COMP) two_sum<F>(acc[i], accc[i], role ? p : sub<KV, F>(splat<KV>(0.f), p));
           else acc[i] = role ? add(acc[i], p) : sub<KV, F>(acc[i], p);
         }
@@ -1096,7 +1101,7 @@ __global__ void __launch_bounds__(128, 7) kf_lo(DMesh m, FastPtrs a) {
         if (z >= nzmin && z <= nzmax - 1) {
           const float hn = hnv[i], hnn = hnnv[i], av = avv[i];
           const float ra = hn / hnn, rb = fdv(dt, av * hnn);  // ra IEEE: exactly 1 for an unchanged layer
-          l = fmas(add(COMP ? add(acc[i], accc[i]) : acc[i], sub(sFlo[k], sFlo[k + 1])), rb, muls(tn, ra - 1.f));
+          l = fmas(add(COMP ? add(acc[i], accc[i]) : acc[i], sub<KV, F>(sFlo[k], sFlo[k + 1])), rb, muls(tn, ra - 1.f));
         }
         if (WSPLIT && NS == 2 && a.wsplit_fused) lk[i] = l;
         else st<KV>(lo, n * LZ + k, l);
@@ -1126,7 +1131,7 @@ __global__ void __launch_bounds__(128, 7) kf_lo(DMesh m, FastPtrs a) {
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             const unsigned k = base + lane + kW * r;
-            if (k < LZ) st<KV>(lo, n * LZ + k, act[r] ? sub(dv[r], tnk[r]) : lk[r]);
+            if (k < LZ) st<KV>(lo, n * LZ + k, act[r] ? sub<KV, F>(dv[r], tnk[r]) : lk[r]);
           }
         }
       }
@@ -1790,14 +1795,14 @@ __global__ void __launch_bounds__(128, 8) kf_nofct(DMesh m, FastPtrs a) {
 #pragma unroll
         for (int i = 0; i < NS; ++i) {
           const V<KV> f = ld<KV>(Fg, ed * LZ + kk[i]);
-          dh[i] = role ? sub(dh[i], f) : add(dh[i], f);
+          dh[i] = role ? sub<KV, NS == 1>(dh[i], f) : add(dh[i], f);
         }
       }
 #pragma unroll
       for (int i = 0; i < NS; ++i) {
         const unsigned k = base + lane + kW * i;
         if (k >= LZ) continue;
-        finish_node<KV>(m, a, gi, n, k, nzmin, nzmax, dh[i], sub(sF[k], sF[k + 1]), nullptr, false);
+        finish_node<KV>(m, a, gi, n, k, nzmin, nzmax, dh[i], sub<KV, NS == 1>(sF[k], sF[k + 1]), nullptr, false);
       }
     }
     __syncwarp();
