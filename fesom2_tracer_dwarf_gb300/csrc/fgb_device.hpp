@@ -109,6 +109,8 @@ struct StepPtrs {
 };
 
 namespace fast {
+
+constexpr int kWaveColumns = 152 * 28;  // node columns in flight at once: 152 SMs of seven blocks of four warps
 // Tiles this small keep a block's staged rows near 32 KB, so the register
 // limit (seven blocks of 128 threads) rather than shared memory sets the
 // kernel's occupancy; at 2048^2 x 64 the edge stage took 7.65 / 6.90 / 6.57 /

@@ -25,7 +25,7 @@ inline void allow_smem_f(F* kernel, size_t bytes) {
 // 2.03 ms at 1024^2x64) than the 1 to 2 us that they would gain.
 template <int KV>
 bool by_group(const DMesh& m, const FastPtrs& a) {
-  return KV <= 2 && a.G > 1 && m.N <= 152 * 28;
+  return KV <= 2 && a.G > 1 && m.N <= kWaveColumns;
 }
 
 template <int KV, int HOR, int NS>

@@ -106,12 +106,19 @@ int launch_stages_f32(const DMesh& m, const fgb_step_desc& d, int mask, cudaStre
   // LO: 3 (the default where it applies) the whole-column kernel for columns of
   // at most 64 layers; 1 or 2 layers per lane per pass. Under w_split the
   // whole-column kernel leaves the implicit step to a second kernel
-  // (kf_vert_pcr), the two-layer one solves it in the same pass: from a wave of
-  // columns on (152 SMs of 28 warps) the two kernels are faster (256^2x64: 146
-  // / 150 us for one tracer, 205 / 213 for four, 323 / 379 for eight; closed
-  // 200^2x47, two tracers, 96 / 109), below it the second launch costs more
-  // (48^2x47, four tracers, 17.2 / 14.6).
-  const bool whole = m.LZ <= 64 && (!wsplit || m.N > 152 * 28 || d.cfg[4] == 3);
+  // (kf_vert_pcr), the two-layer one solves it in the same pass. What the whole
+  // column saves is the scheme's work, most for PPM, and its tables, which
+  // several groups share; the second kernel costs a pass over the LO field,
+  // groups of four tracers most. Two-layer kernel's time over the two kernels',
+  // 48^2 to 400^2 columns of 20 to 64 layers: PPM 1.04 to 1.4; several groups of
+  // one or two tracers 1.0 to 1.3; QR4C one tracer 1.0 to 1.1, eight 1.0 to 1.2,
+  // two 0.87 to 1.07, four 0.95 to 1.2 (0.95 to 0.99 at 220^2); UPW1 and CDIFF
+  // 0.85 to 1.07 for one and two tracers, 0.8 to 1.05 for four and eight. Below
+  // a wave of columns the second launch costs more than either saves.
+  const int groups = K / KV;
+  const bool whole_pays = d.ver == FGB_VER_PPM || (d.ver == FGB_VER_QR4C && (KV == 1 || groups > 1)) ||
+                          (KV <= 2 && groups > 1);
+  const bool whole = m.LZ <= 64 && (!wsplit || (m.N > kWaveColumns && whole_pays) || d.cfg[4] == 3);
   L.ns_lo = (d.cfg[4] == 1 || d.cfg[4] == 2) ? d.cfg[4] : (whole ? 3 : 2);
   // ratio: 1 or 2 layers per lane with shared-memory staging, or 3 (the default)
   // the whole column per warp without shared memory

@@ -263,7 +263,8 @@ typedef struct {
    *            per lane per pass, 1 or 2 with the column staged in shared
    *            memory (update: default 1), for the LO kernel 3 the whole column
    *            per warp (columns of at most 64 layers; its default, under
-   *            w_split on meshes of more than 4256 columns), or for the ratio kernel
+   *            w_split on meshes of more than 4256 columns where that is
+   *            the faster form for the scheme and the groups), or for the ratio kernel
    *            3 (its default) / 4 without shared memory, 4 with fewer
    *            registers (columns of at most 64 layers).
    * cfg[7]     FP32 form: layers per lane per pass of the per-edge edge-flux
