@@ -1,5 +1,6 @@
 // FP32 form of the step: argument checks and dispatch to the kernels of the
 // tracer-group width (fgb_fast.cuh).
+#include <algorithm>
 #include <cstdint>
 
 #include "fgb_internal.hpp"
@@ -12,6 +13,27 @@ int launch_fast_kv4(const DMesh& m, const FastPtrs& a, const LaunchArgs& L, cuda
 }  // namespace fast
 
 WorkspaceLayout workspace_layout_f32(const DMesh& m, int K) { return workspace_layout<float>(m, K); }
+
+// UPW1 edge fluxes: whether the per-edge kernel is the faster one. It takes two
+// layers per lane, 64 at a time; groups of two and four tracers fill its loads
+// on larger meshes. Its time over the tiled kernel's, 24^2 to 724^2 columns of
+// 20 to 64 layers: with a T_AB of its own (two rows to stage per node), four
+// tracers 3.1 .. 1.0 up to 300,000 node-layers and 0.66 to 0.97 from 590,000 on,
+// eight 1.1 at 590,000 to 770,000, 0.66 to 1.06 from 1.0 million on, two 1.2 at
+// 590,000, 0.76 to 1.1 from 1.0 million on, six 1.1 to 1.3 at 1.0 to 1.3
+// million, 0.73 to 1.1 above 2 million; no limiter, T_AB shared, four and eight
+// tracers 1.0 to 1.2 up to 2 million, 0.80 to 1.09 above; with the limiter (and
+// for six tracers without) 0.88 to 0.96 at 16.8 million and 64 layers, 1.0 to 1.4
+// with fewer layers or columns; two tracers 0.97 to 2.8 with T_AB shared, one
+// 1.04 to 3.4 everywhere.
+bool upw1_per_edge(const DMesh& m, int KV, int groups, bool fct, bool own_ta) {
+  const long long cells = (long long)m.N * m.LZ;
+  if (KV == 1) return false;
+  if (fct && own_ta) return cells > (1LL << 19) * (4 / KV) * std::min(groups, 2);
+  if (!fct && KV == 4) return cells > 1LL << 21;
+  return (KV == 4 || groups > 1) && cells >= 1LL << 24 &&
+         4 * m.LZ > 3 * ((m.LZ + 63) / 64 * 64);  // most of its lanes at work
+}
 
 int launch_stages_f32(const DMesh& m, const fgb_step_desc& d, int mask, cudaStream_t s, int* nlaunch,
                       std::string* err) {
@@ -132,11 +154,14 @@ int launch_stages_f32(const DMesh& m, const fgb_step_desc& d, int mask, cudaStre
   // 48x40x30, 3 tracers, 103 against 20 us; closed 513^2x64, 2 tracers, 930 /
   // 370 us; pi refined to 188,661 nodes, 47 layers, 4 tracers, 670 / 305 us;
   // 250x230x47, 2 tracers, 149 / 85 us; 256^2x64, 4 tracers, 162 / 121 us; no
-  // size was slower.
+  // size was slower with MUSCL or MFCT. UPW1 reads an edge's two nodes only, so
+  // staging rows gains less: see upw1_per_edge.
   // The tiled kernel stages rows with 16-byte asynchronous copies; fields on
   // other addresses take the per-edge kernel.
   auto al16 = [](const void* p) { return p == nullptr || reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-  const bool tile = d.cfg[9] == 1 || (d.cfg[0] == 0 && d.cfg[7] == 0);
+  const bool tile = d.cfg[9] == 1 || (d.cfg[0] == 0 && d.cfg[7] == 0 &&
+                                      !(d.hor == FGB_HOR_UPW1 && upw1_per_edge(m, KV, groups, d.lim == FGB_LIM_FCT,
+                                                                               a.TA != a.T)));
   L.hflux_tile = tile && al16(d.T) && al16(d.TA) && al16(d.workspace) && (d.strideT * 4) % 16 == 0 &&
                  (!d.TA || (d.strideTA * 4) % 16 == 0);
   L.hor = d.hor;

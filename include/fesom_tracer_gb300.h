@@ -274,7 +274,8 @@ typedef struct {
    *            the other solver), 1 Thomas sweeps, one lane per column
    * cfg[9]     FP32 form: 1 edge fluxes by the tiled kernel (each tile's node
    *            rows staged once in shared memory; the default when cfg[0] and
-   *            cfg[7] are 0 and the fields are 16-byte aligned)
+   *            cfg[7] are 0 and the fields are 16-byte aligned, but for
+   *            UPW1 on meshes where the per-edge kernel is faster)
    * cfg[10..11] unused, 0 */
   int cfg[12];
   /* w_split (dynamics%use_wsplit, lib/oce_adv_tra_driver.F90:221-231): NULL
