@@ -671,7 +671,7 @@ int tracer_set_values(int tracer_id, const double* values, int nl, int nod2D) {
   if (tracer_id == 1 && sync_values_to_host()) return -1;
   std::copy(values, values + n, t.values.begin());
   std::copy(values, values + n, t.valuesAB.begin());
-  g.inputs_dirty |= kDirtyT;
+  if (tracer_id == 1) g.inputs_dirty |= kDirtyT;  // the one that is stepped
   return 0;
 }
 
