@@ -448,6 +448,10 @@ __host__ __device__ constexpr int nofct_slices(int ver, int kc) {
   return ver_geo_slices(ver) + kc * (2 + ver_work_slices(ver));
 }
 constexpr int kClBytes = kMaxCl * 2 * (int)sizeof(int);
+// Blocks of kNodeWarps columns per SM that the node kernels' registers are held to (reasons at the kernels).
+constexpr int kNodeWarps = 4;
+__host__ __device__ constexpr int lo_blocks(int ver) { return ver == 1 ? 7 : 6; }
+constexpr int kRatioBlocks = 6, kUpdateBlocks = 7, kNofctBlocks = 6;
 
 // The column of one node: interfaces nzmin..nzmax (1-based), layers k0..k0+nlay-1 (0-based).
 struct Column {
@@ -681,7 +685,7 @@ __device__ __forceinline__ double ver_flux(const VerGeo<VER>& g, const Column& c
 // fast form, 4530 -> 4555 us), so the other schemes stay at six.
 // ---------------------------------------------------------------------------
 template <typename R, int VER>
-__global__ void __launch_bounds__(128, VER == 1 ? 7 : 6) k_fct_lo(DMesh m, StepPtrs<R> a, int kc_max) {
+__global__ void __launch_bounds__(kNodeWarps * kWarp, lo_blocks(VER)) k_fct_lo(DMesh m, StepPtrs<R> a, int kc_max) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kWarp - 1), wib = threadIdx.x / kWarp;
   const int vi = blockIdx.x * (blockDim.x / kWarp) + wib;
@@ -805,7 +809,7 @@ __device__ __forceinline__ void spread_nan(double& pos, double& neg) {
 // the distinct nodes with the deepest layer reaching them give the same value.
 // ---------------------------------------------------------------------------
 template <typename R>
-__global__ void __launch_bounds__(128, 6) k_fct_ratio(DMesh m, StepPtrs<R> a, int kc_max) {
+__global__ void __launch_bounds__(kNodeWarps * kWarp, kRatioBlocks) k_fct_ratio(DMesh m, StepPtrs<R> a, int kc_max) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kWarp - 1), wib = threadIdx.x / kWarp;
   const int vi = blockIdx.x * (blockDim.x / kWarp) + wib;
@@ -926,7 +930,7 @@ __device__ __forceinline__ void store_ab_below(const DMesh& m, const StepPtrs<R>
 // 512^2x48 step with 2 tracers 7785 -> 7694 us. Eight (64) would spill.
 // ---------------------------------------------------------------------------
 template <typename R>
-__global__ void __launch_bounds__(128, 7) k_fct_update(DMesh m, StepPtrs<R> a, int kc_max) {
+__global__ void __launch_bounds__(kNodeWarps * kWarp, kUpdateBlocks) k_fct_update(DMesh m, StepPtrs<R> a, int kc_max) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kWarp - 1), wib = threadIdx.x / kWarp;
   const int vi = blockIdx.x * (blockDim.x / kWarp) + wib;
@@ -996,7 +1000,7 @@ __global__ void __launch_bounds__(128, 7) k_fct_update(DMesh m, StepPtrs<R> a, i
 // (oce_tra_adv_flux2dtracer) and the tendency update in one pass.
 // ---------------------------------------------------------------------------
 template <typename R, int VER>
-__global__ void __launch_bounds__(128, 6) k_nofct_update(DMesh m, StepPtrs<R> a, int kc_max) {
+__global__ void __launch_bounds__(kNodeWarps * kWarp, kNofctBlocks) k_nofct_update(DMesh m, StepPtrs<R> a, int kc_max) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kWarp - 1), wib = threadIdx.x / kWarp;
   const int vi = blockIdx.x * (blockDim.x / kWarp) + wib;

@@ -18,9 +18,6 @@ inline namespace fast64 {
 inline namespace exact64 {
 #endif
 
-constexpr int kNodeWarps = 4;  // default node columns per block (the kernels' launch bound)
-
-
 template <typename R, int HOR, bool FCT>
 void launch_hflux_as(const DMesh& m, const StepPtrs<R>& a, bool vf, const double2* grad, cudaStream_t s) {
   const int grid = (m.E + kEdgeTile - 1) / kEdgeTile;
@@ -44,19 +41,31 @@ void allow_smem(F* kernel, size_t bytes) {
   if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-constexpr int kNodeBlocks = 6;  // the node kernels' launch bound: blocks of kNodeWarps warps
-
 // Launches a node kernel. Tracers per chunk: the requested 1, 2 or 4 if it
-// divides K, else the most (up to 4) whose shared memory leaves room for
-// kNodeBlocks blocks on an SM; the lanes share (tracer, layer) pairs, so that
-// chunk need not divide K. Columns too deep for nw of them in a block's shared
-// memory take fewer. bytes(kc): shared memory of one warp.
+// divides K, else at most 4 and as many as leave room for the kernel's blocks
+// in an SM's shared memory (with room for six where the registers allow seven,
+// the QR4C LO stage of 200^2x64 took 702 us against 668, four tracers, and 1533
+// against 1394 with 90 layers, six tracers and T_AB apart), fewer where that
+// takes a warp fewer rounds: the lanes share a chunk's (tracer, layer) pairs,
+// and chunks of three 48-layer tracers leave half a round idle (eight tracers,
+// T_AB apart, fast form: chunks of three 1097 us, of two 1017). Columns too
+// deep for nw of them in a block's shared memory take fewer. bytes(kc): shared
+// memory of one warp.
 template <typename F, typename R, typename B>
-void launch_nodes(F* kernel, const DMesh& m, const StepPtrs<R>& a, int nw, int want, B bytes, cudaStream_t s) {
+void launch_nodes(F* kernel, int blocks, const DMesh& m, const StepPtrs<R>& a, int nw, int want, B bytes,
+                  cudaStream_t s) {
   int kc = a.K < 4 ? a.K : 4;
-  if ((want == 1 || want == 2 || want == 4) && a.K % want == 0) kc = want;
-  else
-    while (kc > 1 && kNodeBlocks * kNodeWarps * bytes(kc) > (size_t)220 * 1024) --kc;
+  if ((want == 1 || want == 2 || want == 4) && a.K % want == 0) {
+    kc = want;
+  } else {
+    while (kc > 1 && blocks * kNodeWarps * bytes(kc) > (size_t)220 * 1024) --kc;
+    auto rounds = [&](int c) {  // of a warp over a full column's pairs
+      auto of = [&](int t) { return (t * m.nz + kWarp - 1) / kWarp; };
+      return a.K / c * of(c) + of(a.K % c);
+    };
+    for (int c = kc - 1; c >= 1; --c)
+      if (rounds(c) < rounds(kc)) kc = c;
+  }
   while (nw > 1 && nw * bytes(kc) > (size_t)227 * 1024) nw /= 2;
   const size_t sm = nw * bytes(kc);
   allow_smem(kernel, sm);
@@ -65,24 +74,25 @@ void launch_nodes(F* kernel, const DMesh& m, const StepPtrs<R>& a, int nw, int w
 
 template <typename R, int VER>
 void launch_lo(const DMesh& m, const StepPtrs<R>& a, int nw, int want, cudaStream_t s) {
-  launch_nodes(k_fct_lo<R, VER>, m, a, nw, want,
+  launch_nodes(k_fct_lo<R, VER>, lo_blocks(VER), m, a, nw, want,
                [&](int kc) { return warp_smem<R>(lo_slices(VER, kc, a.TA != a.T), m.LW, 0); }, s);
 }
 
 template <typename R>
 void launch_ratio(const DMesh& m, const StepPtrs<R>& a, int nw, int want, cudaStream_t s) {
-  launch_nodes(k_fct_ratio<R>, m, a, nw, want,
+  launch_nodes(k_fct_ratio<R>, kRatioBlocks, m, a, nw, want,
                [&](int kc) { return warp_smem<R>(ratio_slices(kc), m.LW, kClBytes); }, s);
 }
 
 template <typename R>
 void launch_update(const DMesh& m, const StepPtrs<R>& a, int nw, int want, cudaStream_t s) {
-  launch_nodes(k_fct_update<R>, m, a, nw, want, [&](int kc) { return warp_smem<R>(upd_slices(kc), m.LW, 0); }, s);
+  launch_nodes(k_fct_update<R>, kUpdateBlocks, m, a, nw, want,
+               [&](int kc) { return warp_smem<R>(upd_slices(kc), m.LW, 0); }, s);
 }
 
 template <typename R, int VER>
 void launch_nofct(const DMesh& m, const StepPtrs<R>& a, int nw, int want, cudaStream_t s) {
-  launch_nodes(k_nofct_update<R, VER>, m, a, nw, want,
+  launch_nodes(k_nofct_update<R, VER>, kNofctBlocks, m, a, nw, want,
                [&](int kc) { return warp_smem<R>(nofct_slices(VER, kc), m.LW, 0); }, s);
 }
 
