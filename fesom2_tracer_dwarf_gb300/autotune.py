@@ -1,22 +1,31 @@
 """Launch-configuration autotuner for the tracer-advection step.
 
-The step is five kernels (vertical fluxes, edge fluxes, FCT low-order
-solution, FCT ratios, update); four of them have launch knobs that do not
-change results (fgb_step_desc.cfg): edges per block of the edge-flux kernel
-(FP32: or the tiled edge kernel), node columns per block of the three node
-kernels, and tracers per chunk (FP64) or layers per lane per pass (FP32). The
-best choice depends on the mesh size, the number of layers, the tracer count
-and the precision, so this module times the candidates of each kernel on the
-caller's own engine (its mesh, fields and schemes) and keeps the fastest.
+The step has five stages (volume fluxes, edge fluxes, FCT low-order solution,
+FCT limiting factors, update); the last four have launch knobs that do not
+change results (fgb_step_desc.cfg): in the FP32 form the edge kernel (tiled, or
+per edge with its block size and layers per lane), the node kernels' columns per
+block and layers per lane per pass and, under w_split, the solver; in the FP64
+forms the node kernels' columns per block and tracers per chunk. Zeros leave a
+choice to the library's rules. The best choice depends on the mesh size, the
+number of layers, the tracer count and the precision, so this module times the
+candidates of each stage on the caller's own engine (its mesh, fields and
+schemes) and keeps the fastest.
 
-Each kernel is tuned on its own: a full step fills the workspace, then every
+The library's own choice is a candidate everywhere: by itself where the others
+cannot express it (FP64 chunks need not divide the tracers, the LO stage under
+w_split has a rule of its own), else as the values it stands for. In the FP64
+forms the edge stage has nothing to choose and is timed once.
+
+Each stage is tuned on its own: a full step fills the workspace, then every
 candidate of one stage is run ``reps`` times between CUDA events on the
 engine's stream and the median is kept. Re-running the flux, LO and ratio
 stages is idempotent; the update stage advances the tracers, so the tracer
 fields are saved before tuning and restored afterwards.
 
-Results are cached by (device, precision, K, schemes, mesh size) in memory,
-and in a JSON file when ``cache_path`` (or FGB_AUTOTUNE_CACHE) names one.
+Results are cached by (version of the kernels' choices, device, precision, K,
+schemes, mesh size) in memory, and in a JSON file when ``cache_path`` (or
+FGB_AUTOTUNE_CACHE) names one. Entries of another version stay in the file and
+are not used: they chose among other kernels.
 """
 from __future__ import annotations
 
@@ -30,12 +39,13 @@ EDGE_WARPS = (2, 4, 8)
 NODE_WARPS = (1, 2, 4)
 CHUNKS = (1, 2, 4)
 SLICES = (1, 2)
+CHOICES_VERSION = 2  # raise when kernels or defaults change under the knobs
 
 _MEMO: dict = {}
 
 
 def chunk_candidates(K: int):
-    """Tracers per chunk that divide K (the library falls back otherwise)."""
+    """Tracers per chunk that divide K (others are left to the library's rule)."""
     return [c for c in CHUNKS if K % c == 0]
 
 
@@ -52,8 +62,8 @@ def stage_candidates(stage: str, K: int, precision: str = "fp64", wsplit: bool =
     slot = {"lo": 0, "ratio": 1, "update": 2}[stage]
     if precision == "fp32":
         # the ratio kernel also has variants without shared memory (3; 4: fewer registers); the
-        # LO stage a whole-column kernel (3: columns of at most 64 layers, not under w_split;
-        # its block shape is fixed, so one candidate)
+        # LO stage a whole-column kernel (3: columns of at most 64 layers; its block shape is
+        # fixed, so one candidate; under w_split by the library's rule, see engine_candidates)
         slices = SLICES + ((3, 4) if stage == "ratio" else ())
         cands = [{1 + slot: w, 4 + slot: ns} for w, ns in product(NODE_WARPS, slices)]
         if stage == "lo" and not wsplit:
@@ -64,13 +74,22 @@ def stage_candidates(stage: str, K: int, precision: str = "fp64", wsplit: bool =
     return [{1 + slot: w, 4 + slot: c} for w, c in product(NODE_WARPS, chunk_candidates(K))]
 
 
+def engine_candidates(stage: str, engine):
+    """The candidates ``tune`` times for a stage of an engine: ``stage_candidates``, with the
+    library's own choice ({}, all zeros) first where they do not hold it."""
+    cands = stage_candidates(stage, engine.K, engine.precision, engine.wi is not None)
+    if engine.precision != "fp32":
+        return [{}] if stage == "hflux" else [{}, *cands]
+    return [{}, *cands] if stage == "lo" and engine.wi is not None else cands
+
+
 def cache_key(engine) -> str:
     import torch
 
     m = engine.mesh
     dev = torch.cuda.get_device_name(engine.device)
-    return "|".join(str(x) for x in (dev, engine.precision, engine.K, engine.V, engine.hor, engine.ver, engine.lim,
-                                     m.N, m.E, m.nz, "wsplit" if engine.wi is not None else "w"))
+    return "|".join(str(x) for x in (f"v{CHOICES_VERSION}", dev, engine.precision, engine.K, engine.V, engine.hor, engine.ver,
+                                     engine.lim, m.N, m.E, m.nz, "wsplit" if engine.wi is not None else "w"))
 
 
 def _load_file(path):
@@ -133,7 +152,7 @@ def tune(engine, dt: float = 1.0, reps: int = 5, cache_path: str | None = None, 
     best_ms = {}
     for name, mask in stages:
         best = None
-        for cand in stage_candidates(name, engine.K, engine.precision, engine.wi is not None):
+        for cand in engine_candidates(name, engine):
             trial = list(cfg)
             for i, v in cand.items():
                 trial[i] = v
