@@ -38,8 +38,8 @@ namespace intdiv {
 
 // The bits of a double, by a move that the compiler does not see through: it
 // turns integer tests of a double's bits (is it zero, is it finite) back into
-// floating-point ones, which occupy the FP64 pipe (two instructions each: with
-// them the step above took 8.88 ms).
+// floating-point ones, which occupy the FP64 pipe (the element-gradient kernel
+// issued 8.67 FP64 instructions per item with them, 6.0 without).
 FGB_HD uint64_t to_bits(double x) {
 #ifdef __CUDA_ARCH__
   uint64_t u;

@@ -681,8 +681,9 @@ __device__ __forceinline__ double ver_flux(const VerGeo<VER>& g, const Column& c
 // kc: tracers per chunk.
 // Blocks per SM: QR4C keeps its values in 72 registers without a spill and the
 // seventh block covers gather latency (512^2x48, 2 tracers, whole step 7694 ->
-// 7603 us); PPM loses more to the tighter allocation than it gains (321^2 basin,
-// fast form, 4530 -> 4555 us), so the other schemes stay at six.
+// 7603 us). The others' registers leave room for seven as they are (PPM 72,
+// UPW1 66, CDIFF 64); compiled for seven, PPM takes 68 and was slower all the
+// same (321^2 basin, fast form, step 4530 -> 4555 us), so their bound is six.
 // ---------------------------------------------------------------------------
 template <typename R, int VER>
 __global__ void __launch_bounds__(kNodeWarps * kWarp, lo_blocks(VER)) k_fct_lo(DMesh m, StepPtrs<R> a, int kc_max) {
