@@ -589,10 +589,7 @@ __global__ void __launch_bounds__(256, (NS == 1 ? 3 : 2)) kf_hflux(DMesh m, Fast
 
 // ---------------------------------------------------------------------------
 // Column staging and vertical fluxes (lib/oce_adv_tra_ver.F90:248-712).
-// Their subtractions are additions (see sub): as fma the LO stage that solves
-// the implicit step in the same pass took 149 us against 141 (220^2x64, four
-// tracers, QR4C), the update without a limiter 122 against 117 (two tracers,
-// PPM, two layers per lane).
+// F: the form of their subtractions (see sub and the kernels).
 // ---------------------------------------------------------------------------
 struct ColF {
   const float* W;
@@ -631,7 +628,7 @@ __device__ __forceinline__ V<KV> ppm_slope(const V<KV>* T, const float* hnn, int
 
 // PPM edge value at interface z (1-based), lib/oce_adv_tra_ver.F90:510-594;
 // the later assignment wins where the special cases coincide.
-template <int KV>
+template <int KV, bool F>
 __device__ __forceinline__ V<KV> ppm_edge(const V<KV>* T, const V<KV>* D, const ColF& c, int z, int nzmin,
                                           int nzmax) {
   if (z >= nzmin + 2 && z <= nzmax - 2) {
@@ -643,7 +640,7 @@ __device__ __forceinline__ V<KV> ppm_edge(const V<KV>* T, const V<KV>* D, const 
     const float P = c0 + ci * c1;
     const float Q2 = ci * fdv(dz * (dzm + dz), 2.f * dz + dzp);
     const float Q3 = ci * fdv(dzp * (dzp + dzpp), dz + 2.f * dzp);
-    const V<KV> d = sub<KV, false>(T[j0 + 1], T[j0]);
+    const V<KV> d = sub<KV, F>(T[j0 + 1], T[j0]);
     return fmas(D[j0], Q3, fmas(D[j0 + 1], -Q2, fmas(d, P, T[j0])));
   }
   if (z == nzmax) return T[nzmax - 2];
@@ -725,7 +722,7 @@ __device__ __forceinline__ V<KV> ppm_flux(const V<KV>& aL0, const V<KV>& aR0, co
 // column's layers; D and TV are scratch columns for PPM.
 // The bottom interface z = nl is never inside a column's stencil: its value
 // is set by one lane, so a 64-layer column needs two passes of 32 lanes.
-template <int VER, int KV>
+template <int VER, int KV, bool F>
 __device__ void vert_flux(const ColF& c, const V<KV>* T, V<KV>* D, V<KV>* TV, const V<KV>* fold, V<KV>* out, int nl,
                           int nzmin, int nzmax, float num_ord, float dt, int lane) {
   const int last = nl - 1;
@@ -735,7 +732,7 @@ __device__ void vert_flux(const ColF& c, const V<KV>* T, V<KV>* D, V<KV>* TV, co
     __syncwarp();
     for (int iz = lane; iz < last; iz += kW) {
       const int z = iz + 1;
-      if (z >= nzmin && z <= nzmax) TV[iz] = ppm_edge<KV>(T, D, c, z, nzmin, nzmax);
+      if (z >= nzmin && z <= nzmax) TV[iz] = ppm_edge<KV, F>(T, D, c, z, nzmin, nzmax);
     }
     if (lane == 0 && nzmax == nl) TV[last] = T[nzmax - 2];
     __syncwarp();
@@ -743,7 +740,7 @@ __device__ void vert_flux(const ColF& c, const V<KV>* T, V<KV>* D, V<KV>* TV, co
   if (lane == 0) {
     // z = nl: the column's last interface (zero flux, CDIFF leaves it) or below the column
     const V<KV> f0 = fold ? fold[last] : splat<KV>(0.f);
-    out[last] = (nzmax == nl && VER != 2) ? sub<KV, false>(splat<KV>(0.f), f0) : f0;
+    out[last] = (nzmax == nl && VER != 2) ? sub<KV, F>(splat<KV>(0.f), f0) : f0;
   }
   for (int iz = lane; iz < last; iz += kW) {
     const int z = iz + 1;
@@ -752,19 +749,19 @@ __device__ void vert_flux(const ColF& c, const V<KV>* T, V<KV>* D, V<KV>* TV, co
     if (z >= nzmin && z <= nzmax) {
       const float W = c.W[iz], ar = c.area[iz];
       if (VER == 0) {
-        if (z == nzmin) r = sub<KV, false>(muls(T[z - 1], -(W * ar)), f0);
-        else if (z == nzmax) r = sub<KV, false>(splat<KV>(0.f), f0);
+        if (z == nzmin) r = sub<KV, F>(muls(T[z - 1], -(W * ar)), f0);
+        else if (z == nzmax) r = sub<KV, F>(splat<KV>(0.f), f0);
         else
-          r = sub<KV, false>(fmas(T[z - 2], -0.5f * (W - fabsf(W)) * ar, muls(T[z - 1], -0.5f * (W + fabsf(W)) * ar)), f0);
+          r = sub<KV, F>(fmas(T[z - 2], -0.5f * (W - fabsf(W)) * ar, muls(T[z - 1], -0.5f * (W + fabsf(W)) * ar)), f0);
       } else if (VER == 1) {
         if (z == nzmin) {
-          r = sub<KV, false>(muls(T[z - 1], -(W * ar)), f0);
+          r = sub<KV, F>(muls(T[z - 1], -(W * ar)), f0);
         } else if (z == nzmax) {
-          r = sub<KV, false>(splat<KV>(0.f), f0);
+          r = sub<KV, F>(splat<KV>(0.f), f0);
         } else if (z == nzmin + 1 || z == nzmax - 1) {
           const V<KV> x = muls(add(T[z - 2], T[z - 1]), -0.5f * W * ar);
-          r = sub<KV, false>(x, f0);
-          if (nzmin + 1 == nzmax - 1) r = sub<KV, false>(x, r);  // written twice (lib/oce_adv_tra_ver.F90:405-411)
+          r = sub<KV, F>(x, f0);
+          if (nzmin + 1 == nzmax - 1) r = sub<KV, F>(x, r);  // written twice (lib/oce_adv_tra_ver.F90:405-411)
         } else {
           const float Z0 = c.Z[z - 1], Zm1 = c.Z[z - 2], Zm2 = c.Z[z - 3], Zp1 = c.Z[z];
           const float ic = fdv(1.f, Zm1 - Z0), iu = fdv(1.f, Z0 - Zp1), idn = fdv(1.f, Zm2 - Zm1);
@@ -773,16 +770,16 @@ __device__ void vert_flux(const ColF& c, const V<KV>* T, V<KV>* D, V<KV>* TV, co
           const float wp = W + fabsf(W), wm = W - fabsf(W);
           const float cA = -(0.5f * (1.f - num_ord)) * ar, cB = -(num_ord * 0.5f) * W * ar;
           const V<KV> T0 = T[z - 1], Tm1 = T[z - 2], Tm2 = T[z - 3], Tp1 = T[z];
-          const V<KV> qc = muls(sub<KV, false>(Tm1, T0), ic), qu = muls(sub<KV, false>(T0, Tp1), iu), qd = muls(sub<KV, false>(Tm2, Tm1), idn);
+          const V<KV> qc = muls(sub<KV, F>(Tm1, T0), ic), qu = muls(sub<KV, F>(T0, Tp1), iu), qd = muls(sub<KV, F>(Tm2, Tm1), idn);
           const V<KV> tm1 = fmas(fmas(qc, 2.f, qu), a1, T0);
           const V<KV> tm2 = fmas(fmas(qc, 2.f, qd), a2, Tm1);
           const V<KV> tm = fmas(tm2, wm, muls(tm1, wp));
-          r = sub<KV, false>(fmas(add(tm1, tm2), cB, muls(tm, cA)), f0);
+          r = sub<KV, F>(fmas(add(tm1, tm2), cB, muls(tm, cA)), f0);
         }
       } else if (VER == 2) {
         const int nzc = nzmax - 1;  // lib/oce_adv_tra_ver.F90:689
-        if (z == nzmin) r = sub<KV, false>(muls(T[z - 1], -(W * ar)), f0);
-        else if (z <= nzc) r = sub<KV, false>(muls(add(T[z - 2], T[z - 1]), -0.5f * W * ar), f0);
+        if (z == nzmin) r = sub<KV, F>(muls(T[z - 1], -(W * ar)), f0);
+        else if (z <= nzc) r = sub<KV, F>(muls(add(T[z - 2], T[z - 1]), -0.5f * W * ar), f0);
       } else {
         V<KV> tvert = splat<KV>(0.f);
         if (z == nzmin) {
@@ -794,7 +791,7 @@ __device__ void vert_flux(const ColF& c, const V<KV>* T, V<KV>* D, V<KV>* TV, co
           const float x = fminf(fdv(fabsf(W) * dt, c.hn[zl]), 1.f);
           tvert = ppm_flux<KV>(TV[zl], TV[zl + 1], T[zl], x, up, ar * W);
         }
-        r = sub<KV, false>(tvert, f0);
+        r = sub<KV, F>(tvert, f0);
       }
     }
     out[iz] = r;
@@ -958,10 +955,12 @@ __device__ __forceinline__ void vimpl_row(int k, int k0, int k1, float W0, float
 // ---------------------------------------------------------------------------
 template <int VER, int KV, int NS, bool WSPLIT, bool COMP>
 __global__ void __launch_bounds__(128, 7) kf_lo(DMesh m, FastPtrs a) {
-  // Two layers per lane fill the 72 registers: subtractions as additions (220^2, 4 tracers, 75
-  // layers, compensated: LO stage 11 to 15 % shorter than with fma; the w_split pass 3 to 6 % for
-  // QR4C), with one layer as fma (3 % shorter).
-  constexpr bool F = NS == 1;
+  // Forms of the subtractions (see sub), F, and of those in the compensated sums, FS. Two layers
+  // per lane fill the 72 registers: with the sums' as fma groups of four take 11 to 15 % longer,
+  // groups of two 2 to 3 % less but for QR4C (4 % more); QR4C's own as fma cost the w_split pass
+  // 3 to 6 %, the other schemes' save up to 4 %. With one layer both are fma (3 % shorter).
+  // LO stage, 220^2x64 and 160^2x75.
+  constexpr bool F = NS == 1 || VER != 1, FS = NS == 1 || (KV == 2 && VER != 1);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kW - 1), wib = threadIdx.x / kW;
   const int vi = blockIdx.x * (blockDim.x / kW) + wib;
@@ -1040,13 +1039,13 @@ __global__ void __launch_bounds__(128, 7) kf_lo(DMesh m, FastPtrs a) {
     // LO vertical flux: upwind on T with w_e; under w_split the antidiffusive
     // flux takes the upwind flux of the full w instead
     // (lib/oce_adv_tra_driver.F90:221-231).
-    vert_flux<0, KV>(WSPLIT ? cho : clo, sT, nullptr, nullptr, nullptr, sFlo, nl, nzmin, nzmax, 1.f, dt, lane);
+    vert_flux<0, KV, F>(WSPLIT ? cho : clo, sT, nullptr, nullptr, nullptr, sFlo, nl, nzmin, nzmax, 1.f, dt, lane);
     // HO vertical flux on T_AB with w; adf_v = HO - LO.
-    vert_flux<VER, KV>(cho, sTA, sD, sTV, sFlo, sFho, nl, nzmin, nzmax, a.pv, dt, lane);
+    vert_flux<VER, KV, F>(cho, sTA, sD, sTV, sFlo, sFho, nl, nzmin, nzmax, a.pv, dt, lane);
     float* __restrict__ adfv = a.adfv + gi * a.gW;
     for (int iz = lane; iz < nl - 1; iz += kW) st<KV>(adfv, n * LW + iz, sFho[iz]);
     if (lane == 0) st<KV>(adfv, n * LW + nl - 1, sFho[nl - 1]);
-    if (WSPLIT) vert_flux<0, KV>(clo, sT, nullptr, nullptr, nullptr, sFlo, nl, nzmin, nzmax, 1.f, dt, lane);
+    if (WSPLIT) vert_flux<0, KV, F>(clo, sT, nullptr, nullptr, nullptr, sFlo, nl, nzmin, nzmax, 1.f, dt, lane);
     float* __restrict__ lo = a.lo + gi * a.gN;
     for (unsigned base = 0; base < LZ; base += kW * NS) {
       unsigned kk[NS];
@@ -1085,7 +1084,7 @@ __global__ void __launch_bounds__(128, 7) kf_lo(DMesh m, FastPtrs a) {
           for (int c = 0; c < KV; ++c) tu.v[c] = own_up ? tnk[i].v[c] : to[i].v[c];
           const V<KV> p = muls(tu, v[i]);
           // with COMP the sum carries its rounding error (TwoSum)
-          if (COMP) two_sum<F>(acc[i], accc[i], role ? p : sub<KV, F>(splat<KV>(0.f), p));
+          if (COMP) two_sum<FS>(acc[i], accc[i], role ? p : sub<KV, F>(splat<KV>(0.f), p));
           else acc[i] = role ? add(acc[i], p) : sub<KV, F>(acc[i], p);
         }
       }
@@ -1546,8 +1545,9 @@ __device__ __forceinline__ void finish_node(const DMesh& m, const FastPtrs& a, i
 // flight per round, three for groups of one or two tracers (closed 513^2x64, 2
 // tracers: 470 against 489 us; four tracers, 1024^2x64: 2.68 against 2.63 ms,
 // and 2.81 or more with fewer warps of more registers), but two for one tracer
-// with a compensated divergence (220^2x64: 74 against 92 us) and where a lane
-// holds two layers (two tracers with the residual: 16 % shorter).
+// with a compensated divergence (220^2x64: 74 against 92 us), and with two
+// layers per lane for two tracers with plain sums (with the residual 16 %
+// shorter; compensated they are 8 % longer with two).
 // DEL: a persistent del_ttf is read and written (the reference C interface).
 // COMP: the limited edge fluxes are formed as one rounded product p = ae * f,
 // the same number at both ends of the edge (+p at the first node, -p at the
@@ -1653,7 +1653,7 @@ __global__ void __launch_bounds__(128, (NS == 1 ? (COMP || RES ? 8 : 9) : 4)) kf
           hn[i] = g.hnode[n * LZ + kk[i]];
         }
       }
-#pragma unroll(KV <= 2 && NS == 1 && !(KV == 1 && COMP) ? 3 : 2)
+#pragma unroll(KV <= 2 && (NS == 1 ? !(KV == 1 && COMP) : KV == 1 || COMP) ? 3 : 2)
       for (int j = 0; j < nb.deg; ++j) {
         const int2 q = nb.get(m, j);
         const unsigned ed = (unsigned)(q.x >> 1);
@@ -1739,6 +1739,8 @@ __global__ void __launch_bounds__(128, (NS == 1 ? (COMP || RES ? 8 : 9) : 4)) kf
 // ---------------------------------------------------------------------------
 template <int VER, int KV, int NS>
 __global__ void __launch_bounds__(128, 8) kf_nofct(DMesh m, FastPtrs a) {
+  // PPM with two layers per lane: subtractions as additions (two tracers, 220^2x64: 117 against 122 us)
+  constexpr bool F = !(VER == 3 && NS == 2);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kW - 1), wib = threadIdx.x / kW;
   const int vi = blockIdx.x * (blockDim.x / kW) + wib;
@@ -1777,7 +1779,7 @@ __global__ void __launch_bounds__(128, 8) kf_nofct(DMesh m, FastPtrs a) {
     const float* __restrict__ Fg = a.adfh + gi * a.gE;
     stage_v<KV>(sTA, TAg, n * LZ, nz, lane);
     __syncwarp();
-    vert_flux<VER, KV>(c, sTA, sD, sTV, nullptr, sF, nl, nzmin, nzmax, a.pv, a.dt, lane);
+    vert_flux<VER, KV, F>(c, sTA, sD, sTV, nullptr, sF, nl, nzmin, nzmax, a.pv, a.dt, lane);
     for (unsigned base = 0; base < LZ; base += kW * NS) {
       unsigned kk[NS];
       V<KV> dh[NS];
@@ -1795,14 +1797,14 @@ __global__ void __launch_bounds__(128, 8) kf_nofct(DMesh m, FastPtrs a) {
 #pragma unroll
         for (int i = 0; i < NS; ++i) {
           const V<KV> f = ld<KV>(Fg, ed * LZ + kk[i]);
-          dh[i] = role ? sub<KV, NS == 1>(dh[i], f) : add(dh[i], f);
+          dh[i] = role ? sub<KV, F>(dh[i], f) : add(dh[i], f);
         }
       }
 #pragma unroll
       for (int i = 0; i < NS; ++i) {
         const unsigned k = base + lane + kW * i;
         if (k >= LZ) continue;
-        finish_node<KV>(m, a, gi, n, k, nzmin, nzmax, dh[i], sub<KV, NS == 1>(sF[k], sF[k + 1]), nullptr, false);
+        finish_node<KV>(m, a, gi, n, k, nzmin, nzmax, dh[i], sub<KV, F>(sF[k], sF[k + 1]), nullptr, false);
       }
     }
     __syncwarp();

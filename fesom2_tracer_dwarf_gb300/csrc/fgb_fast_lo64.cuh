@@ -42,18 +42,18 @@ __host__ __device__ constexpr size_t lo64_warp_bytes(int KV, int ver, bool tasep
 // variants at 220^2x64 (periodic) and 220^2x47 (closed basin); LO stage with the
 // sign first against after: one tracer, plain sums, CDIFF 0.90, UPW1 0.99, PPM
 // 1.01 to 1.03, compensated sums 1.00 to 1.08; two tracers, plain sums, CDIFF
-// 0.80 to 0.86, QR4C 0.80 to 0.97, PPM 1.02 to 1.05, compensated 0.97 to 1.10;
-// four tracers 0.87 to 0.99 but for the two named variants (1.05, 1.02).
+// 0.80 to 0.86, QR4C 0.80 to 0.97, PPM 1.02 to 1.05, compensated UPW1 0.88 to
+// 0.95 (with fma subtractions, below), the others 0.97 to 1.10; four tracers 0.87 to 0.99 but for the two named variants (1.05, 1.02).
 __host__ __device__ constexpr bool lo64_sign_first(int VER, int KV, bool TASEP, bool WESEP, bool COMP) {
-  if (KV != 4) return !COMP && VER != 3;
+  if (KV != 4) return COMP ? KV == 2 && VER == 0 : VER != 3;
   return COMP || WESEP || (VER != 2 && VER != 1) || (VER == 2) == TASEP;
 }
 // Subtractions as fma (see sub): with four tracers and compensated sums, LO
 // stage against additions 0.98 for UPW1 and PPM (1.02 to 1.08 with a w_e of its
 // own), 1.04 to 1.06 for QR4C and CDIFF (0.94 with a w_e of its own), 0.96 under
-// w_split; with two tracers 1.0 to 1.25.
+// w_split; with two tracers 0.95 for UPW1, 1.0 to 1.25 for the others.
 __host__ __device__ constexpr bool lo64_fma_sub(int VER, int KV, bool WESEP, bool WS) {
-  return KV == 4 && (WS || ((VER == 0 || VER == 3) != WESEP));
+  return KV == 4 ? WS || (VER == 0 || VER == 3) != WESEP : KV == 2 && VER == 0;
 }
 
 // VERW: the vertical scheme, + 4 under w_split with a w_e of its own (the

@@ -20,8 +20,9 @@ WorkspaceLayout workspace_layout_f32(const DMesh& m, int K) { return workspace_l
 // 20 to 64 layers: with a T_AB of its own (two rows to stage per node), four
 // tracers 3.1 .. 1.0 up to 300,000 node-layers and 0.66 to 0.97 from 590,000 on,
 // eight 1.1 at 590,000 to 770,000, 0.66 to 1.06 from 1.0 million on, two 1.2 at
-// 590,000, 0.76 to 1.1 from 1.0 million on, six 1.1 to 1.3 at 1.0 to 1.3
-// million, 0.73 to 1.1 above 2 million; no limiter, T_AB shared, four and eight
+// 590,000, 0.76 to 0.95 from 1.0 million on (20 to 32 and 75 layers, which leave
+// more than a quarter of its lanes idle, 0.96 to 1.4), six 1.1 to 1.3 at 1.0 to
+// 1.3 million, 0.73 to 1.0 above 2 million; no limiter, T_AB shared, four and eight
 // tracers 1.0 to 1.2 up to 2 million, 0.80 to 1.09 above; with the limiter (and
 // for six tracers without) 0.88 to 0.96 at 16.8 million and 64 layers, 1.0 to 1.4
 // with fewer layers or columns; two tracers 0.97 to 2.8 with T_AB shared, one
@@ -29,10 +30,10 @@ WorkspaceLayout workspace_layout_f32(const DMesh& m, int K) { return workspace_l
 bool upw1_per_edge(const DMesh& m, int KV, int groups, bool fct, bool own_ta) {
   const long long cells = (long long)m.N * m.LZ;
   if (KV == 1) return false;
-  if (fct && own_ta) return cells > (1LL << 19) * (4 / KV) * std::min(groups, 2);
+  const int passes = (m.LZ + 63) / 64 * 64;  // layers its lanes could hold
+  if (fct && own_ta) return cells > (1LL << 19) * (4 / KV) * std::min(groups, 2) && (KV == 4 || 4 * m.LZ >= 3 * passes);
   if (!fct && KV == 4) return cells > 1LL << 21;
-  return (KV == 4 || groups > 1) && cells >= 1LL << 24 &&
-         4 * m.LZ > 3 * ((m.LZ + 63) / 64 * 64);  // most of its lanes at work
+  return (KV == 4 || groups > 1) && cells >= 1LL << 24 && 4 * m.LZ > 3 * passes;
 }
 
 int launch_stages_f32(const DMesh& m, const fgb_step_desc& d, int mask, cudaStream_t s, int* nlaunch,
@@ -134,12 +135,13 @@ int launch_stages_f32(const DMesh& m, const fgb_step_desc& d, int mask, cudaStre
   // groups of four tracers most. Two-layer kernel's time over the two kernels',
   // 48^2 to 400^2 columns of 20 to 64 layers: PPM 1.04 to 1.4; several groups of
   // one or two tracers 1.0 to 1.3; QR4C one tracer 1.0 to 1.1, eight 1.0 to 1.2,
-  // two 0.87 to 1.07, four 0.95 to 1.2 (0.95 to 0.99 at 220^2); UPW1 and CDIFF
-  // 0.85 to 1.07 for one and two tracers, 0.8 to 1.05 for four and eight. Below
+  // two 0.87 to 1.07, four 0.95 to 1.2 (0.95 to 0.99 at 220^2); UPW1 with one
+  // tracer and plain sums 1.0 to 1.13, otherwise UPW1 and CDIFF 0.85 to 1.07 for
+  // one and two tracers, 0.8 to 1.05 for four and eight. Below
   // a wave of columns the second launch costs more than either saves.
   const int groups = K / KV;
   const bool whole_pays = d.ver == FGB_VER_PPM || (d.ver == FGB_VER_QR4C && (KV == 1 || groups > 1)) ||
-                          (KV <= 2 && groups > 1);
+                          (KV <= 2 && groups > 1) || (d.ver == FGB_VER_UPW1 && KV == 1 && !(a.comp & 1));
   const bool whole = m.LZ <= 64 && (!wsplit || (m.N > kWaveColumns && whole_pays) || d.cfg[4] == 3);
   L.ns_lo = (d.cfg[4] == 1 || d.cfg[4] == 2) ? d.cfg[4] : (whole ? 3 : 2);
   // ratio: 1 or 2 layers per lane with shared-memory staging, or 3 (the default)
