@@ -36,24 +36,29 @@ __host__ __device__ constexpr size_t lo64_warp_bytes(int KV, int ver, bool tasep
 }
 
 // The gather adds v T_up or subtracts it. True: the sign goes onto the volume
-// flux before the product; false: the sum or the product takes it. Both give
-// the same bits, and at the 72 registers of seven blocks per SM the difference
-// is what ptxas makes of each variant, so the choice is from measurement, all
-// variants at 220^2x64 (periodic) and 220^2x47 (closed basin); LO stage with the
-// sign first against after: one tracer, plain sums, CDIFF 0.90, UPW1 0.99, PPM
-// 1.01 to 1.03, compensated sums 1.00 to 1.08; two tracers, plain sums, CDIFF
-// 0.80 to 0.86, QR4C 0.80 to 0.97, PPM 1.02 to 1.05, compensated UPW1 0.88 to
-// 0.95 (with fma subtractions, below), the others 0.97 to 1.10; four tracers 0.87 to 0.99 but for the two named variants (1.05, 1.02).
-__host__ __device__ constexpr bool lo64_sign_first(int VER, int KV, bool TASEP, bool WESEP, bool COMP) {
+// flux before the product; false: the sum or the product takes it. At the 72
+// registers of seven blocks per SM the difference is what ptxas makes of each
+// variant, so the choice is from measurement, all variants at 220^2x64
+// (periodic) and 220^2x47 (closed basin); LO stage with the sign first against
+// after: one tracer, plain sums, CDIFF 0.90, UPW1 0.99, PPM 1.01 to 1.03,
+// compensated sums 1.00 to 1.08; two tracers, plain sums, CDIFF 0.80 to 0.86,
+// QR4C 0.80 to 0.97, PPM 1.02 to 1.05, compensated UPW1 0.88 to 0.95 (with fma
+// subtractions, below), the others 0.97 to 1.10; four tracers 0.87 to 0.99 but
+// for UPW1 with a w_e of its own, compensated (1.01 to 1.04), and the two named
+// variants (1.05, 1.02). The products are the same; with plain sums and the
+// sign first ptxas fuses them into the packed additions, one rounding less.
+// Compensated sums are not to be fused (the error of a sum is that of adding the
+// rounded product): four tracers take the sign first only with fma subtractions,
+// which keep the product apart.
+__host__ __device__ constexpr bool lo64_sign_first(int VER, int KV, bool TASEP, bool WESEP, bool COMP, bool WS) {
   if (KV != 4) return COMP ? KV == 2 && VER == 0 : VER != 3;
-  return COMP || WESEP || (VER != 2 && VER != 1) || (VER == 2) == TASEP;
+  if (COMP) return WS || !(VER == 0 && WESEP);
+  return WESEP || (VER != 2 && VER != 1) || (VER == 2) == TASEP;
 }
-// Subtractions as fma (see sub): with four tracers and compensated sums, LO
-// stage against additions 0.98 for UPW1 and PPM (1.02 to 1.08 with a w_e of its
-// own), 1.04 to 1.06 for QR4C and CDIFF (0.94 with a w_e of its own), 0.96 under
-// w_split; with two tracers 0.95 for UPW1, 1.0 to 1.25 for the others.
-__host__ __device__ constexpr bool lo64_fma_sub(int VER, int KV, bool WESEP, bool WS) {
-  return KV == 4 ? WS || (VER == 0 || VER == 3) != WESEP : KV == 2 && VER == 0;
+// Subtractions as fma (see sub). Two tracers: LO stage against additions 0.95
+// for UPW1, 1.0 to 1.25 for the others.
+__host__ __device__ constexpr bool lo64_fma_sub(int VER, int KV, bool WESEP, bool COMP, bool WS) {
+  return KV == 4 ? WS || !(COMP && VER == 0 && WESEP) : KV == 2 && VER == 0;
 }
 
 // VERW: the vertical scheme, + 4 under w_split with a w_e of its own (the
@@ -62,7 +67,7 @@ __host__ __device__ constexpr bool lo64_fma_sub(int VER, int KV, bool WESEP, boo
 template <int VERW, int KV, bool TASEP, bool WESEP, bool COMP>
 __global__ void __launch_bounds__(kLo64Warps * kW, 7) kf_lo64(DMesh m, FastPtrs a) {
   constexpr int VER = VERW & 3;
-  constexpr bool WS = VERW >= 4, F = lo64_fma_sub(VER, KV, WESEP, WS);
+  constexpr bool WS = VERW >= 4, F = lo64_fma_sub(VER, KV, WESEP, COMP, WS);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & (kW - 1), wib = threadIdx.x / kW;
   const int vi = blockIdx.x * kLo64Warps + wib;
@@ -287,9 +292,9 @@ __global__ void __launch_bounds__(kLo64Warps * kW, 7) kf_lo64(DMesh m, FastPtrs 
     // over the incident edges in ascending edge order. The upwind flux
     // -(T1 (v + |v|) + T2 (v - |v|)) / 2 is exactly -v T_up, T_up the value at
     // the upwind node: each node adds -v T_up (first node) or +v T_up (second
-    // node), one rounded product that is the same number at both ends of the
-    // edge, so the low-order fluxes cancel between neighbours; with COMP the
-    // products are summed with compensation.
+    // node), one product that is the same number at both ends of the edge (rounded,
+    // or exact where it is fused into the addition), so the low-order fluxes cancel
+    // between neighbours; with COMP the rounded products are summed with compensation.
     V<KV> acc[2] = {splat<KV>(0.f), splat<KV>(0.f)}, accc[2] = {splat<KV>(0.f), splat<KV>(0.f)};
     const unsigned kc[2] = {(unsigned)min(k[0], LZ - 1), (unsigned)min(k[1], LZ - 1)};
 #pragma unroll 2
@@ -311,7 +316,7 @@ __global__ void __launch_bounds__(kLo64Warps * kW, 7) kf_lo64(DMesh m, FastPtrs 
         V<KV> tu;
 #pragma unroll
         for (int c = 0; c < KV; ++c) tu.v[c] = own_up ? t[s].v[c] : to[s].v[c];
-        if constexpr (lo64_sign_first(VER, KV, TASEP, WESEP, COMP)) {
+        if constexpr (lo64_sign_first(VER, KV, TASEP, WESEP, COMP, WS)) {
           const V<KV> p = muls(tu, role ? v[s] : -v[s]);
           if (COMP) two_sum<F>(acc[s], accc[s], p);
           else acc[s] = add(acc[s], p);

@@ -263,7 +263,7 @@ __device__ __forceinline__ void node_mean_grad(const DMesh& m, const double* __r
 // Bound by the FP64 pipe: 15 FP64 instructions per layer and tracer (MUSCL,
 // ph = 1; 87 in the form it replaced) and two divisions by six on the integer
 // pipe. 512^2 x 48, 2 tracers: volume fluxes, gradients and edge fluxes 4.4 ms
-// together against 10.9.
+// together against 10.9 (2.9 with the products that have moved since).
 // ---------------------------------------------------------------------------
 // The flux for any ph and for very large, infinite and NaN values.
 static __device__ __noinline__ double hor_flux_any(double v, double Tm1, double Tm2, double ph) {
@@ -398,10 +398,11 @@ __global__ void __launch_bounds__(kEdgeThreads, 4) k_hflux(DMesh m, StepPtrs<R> 
 // FP64 pipe, which a warp instruction with idle lanes occupies as long as a
 // full one), a lane holds one layer of one tracer (few registers, more warps),
 // and its chain of dependent operations is short. Per (tracer, layer) the
-// summation order is the reference's. 512^2 x 48, 2 tracers, against two layers
-// per lane and a compile-time tracer chunk: LO 1.95 / 3.34 ms, ratio 1.50 /
-// 2.07, update 1.62 / 2.64; closed 321^2 x 64, fast form: 2.17 / 2.43, 0.68 /
-// 0.76, 0.65 / 1.11; 361 columns of 9 layers, no limiter: 10 / 18 us.
+// summation order is the reference's. 512^2 x 48, 2 tracers, side by side with
+// two layers per lane and a compile-time tracer chunk: LO 1.95 / 3.34 ms, ratio
+// 1.50 / 2.07, update 1.62 / 2.64 (with what came after 1.63, 1.51, 1.55);
+// closed 321^2 x 64, fast form: 2.17 / 2.43, 0.68 / 0.76, 0.65 / 1.11 (1.76,
+// 0.69, 0.66); 361 columns of 9 layers, no limiter: 10 / 18 us.
 // ---------------------------------------------------------------------------
 struct Nbr {
   int e, role, other, lo, hi;
